@@ -911,6 +911,7 @@ extern "C" int wsb_matrix_kernel_times(wsb_context *ctx, wsb_matrix *m, const fl
     CHECK_CTX(ctx);
     if (!m || !d_b || !ms || iterations == 0) return fail(ctx, WSB_ERR_BAD_INPUT, "bad arguments");
     Engine E(ctx, ctx->stream);
+    E.use_loop_kernels();
     SolveCfg cfg;
     cfg.max_iter = iterations + 1;
     uint32_t slot;
@@ -983,11 +984,12 @@ extern "C" int wsb_batch_solve(wsb_batch *bt) {
     if (!bt) return fail(nullptr, WSB_ERR_BAD_INPUT, "batch is null");
     Context *ctx = bt->ctx;
     CHECK_CTX(ctx);
-    // Steps of 64 iterations: finished systems leave the work lists between steps.
+    // Steps of 64 iterations: finished systems leave the work lists between
+    // steps. Systems that k_team iterates run to their end in one.
     bool left = true;
     double ms = 0.0;
     while (left) {
-        int rc = bt->eng->step(64, &left);
+        int rc = bt->eng->step(64, &left, 0xffffffffu);
         if (rc) return rc;
         ms += bt->eng->last_device_ms();
     }

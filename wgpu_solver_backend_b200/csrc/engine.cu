@@ -160,7 +160,15 @@ struct Engine::Slot {
     bool stalled = false;
     uint64_t iters_total = 0;
     SolveOutcome out;
+    // k_team (team > 0): CTAs of the system's team, warp tiles a CTA holds and
+    // its shared memory, published partials, z packets.
+    uint32_t team = 0, team_warps = 0, team_smem = 0;
+    RedEntry *red = nullptr;
+    unsigned long long *zpk = nullptr;
+    bool red_dirty = false;  // a launch failed: the slots' tags are not the state's
 };
+
+static size_t team_red_bytes(uint32_t team) { return sizeof(RedEntry) * team_red_entries(team); }
 
 enum { AUX_REFINE = 0, AUX_RESID = 1, AUX_X32 = 2 };
 
@@ -182,6 +190,7 @@ Engine::Engine(Context *ctx, cudaStream_t stream) : ctx_(ctx), stream_(stream) {
     max_grid_a_ = std::max(1, occ_a) * std::max(1, ctx->sm_count);
     max_grid_b_ = std::max(1, occ_b) * std::max(1, ctx->sm_count);
     max_grid_c_ = std::max(1, occ_c) * std::max(1, ctx->sm_count);
+    cudaFuncSetAttribute(k_team, cudaFuncAttributeMaxDynamicSharedMemorySize, kTeamSmemMax);
     const char *loop_env = getenv("WSB_LOOP");
     use_graph_ = !(loop_env && std::strcmp(loop_env, "launch") == 0);
     cudaMallocHost(&h_sp_, sizeof(StepParams));
@@ -193,6 +202,7 @@ Engine::Engine(Context *ctx, cudaStream_t stream) : ctx_(ctx), stream_(stream) {
 }
 
 Engine::~Engine() {
+    if (team_stream_) cudaStreamSynchronize(team_stream_);
     cudaStreamSynchronize(stream_);
     if (exec_) cudaGraphExecDestroy(exec_);
     if (graph_) cudaGraphDestroy(graph_);
@@ -202,6 +212,8 @@ Engine::~Engine() {
     cudaFree(d_state_);
     cudaFree(d_sp_);
     cudaFree(d_work_);
+    cudaFree(d_team_);
+    cudaFreeHost(h_team_);
     cudaFreeHost(h_sys_);
     cudaFreeHost(h_state_);
     cudaFreeHost(h_sp_);
@@ -209,6 +221,9 @@ Engine::~Engine() {
     cudaFreeHost(h_work_);
     cudaEventDestroy(ev0_);
     cudaEventDestroy(ev1_);
+    if (team_stream_) cudaStreamDestroy(team_stream_);
+    if (fork_ev_) cudaEventDestroy(fork_ev_);
+    if (join_ev_) cudaEventDestroy(join_ev_);
 }
 
 int Engine::ensure_capacity(uint32_t need) {
@@ -252,14 +267,49 @@ int Engine::ensure_capacity(uint32_t need) {
     return WSB_OK;
 }
 
-int Engine::push_desc(uint32_t s) {
-    WSB_CUDA_TRY(ctx_, cudaMemcpyAsync(d_sys_ + s, h_sys_ + s, sizeof(SysDesc), cudaMemcpyHostToDevice, stream_));
+// Uploads the descriptors and states that changed on the host, one copy each
+// (between steps the pinned mirrors hold every system's, so a copy of the whole
+// array changes nothing else; one small copy per system cost a batch of 300
+// systems 2 ms).
+int Engine::push_changes() {
+    if (desc_dirty_)
+        WSB_CUDA_TRY(ctx_, cudaMemcpyAsync(d_sys_, h_sys_, sizeof(SysDesc) * cap_, cudaMemcpyHostToDevice, stream_));
+    if (state_dirty_)
+        WSB_CUDA_TRY(ctx_, cudaMemcpyAsync(d_state_, h_state_, sizeof(SysState) * cap_, cudaMemcpyHostToDevice, stream_));
+    desc_dirty_ = state_dirty_ = false;
     return WSB_OK;
 }
 
-int Engine::push_state(uint32_t s) {
-    WSB_CUDA_TRY(ctx_, cudaMemcpyAsync(d_state_ + s, h_state_ + s, sizeof(SysState), cudaMemcpyHostToDevice, stream_));
-    return WSB_OK;
+// Whether k_team iterates this system, and the team it needs: BSR6 (its
+// blocks are the preconditioner's blocks), the classic recurrence, and few
+// enough blocks for the shared memory of one CTA an SM in shared memory.
+void Engine::team_plan(Slot *sl) const {
+    const MatA &A = *sl->A;
+    if (!team_on_ || !use_graph_ || A.layout != LAYOUT_BSR6 || A.n == 0 || sl->M->nb != A.n / 6 ||
+        sl->cfg.algorithm != WSB_ALG_CLASSIC)
+        return;
+    const uint32_t nbr = A.n / 6, tiles = (nbr + kTeamWarpBrows - 1) / kTeamWarpBrows;
+    if (tiles > (uint32_t)ctx_->sm_count * kTeamWarps) return;
+    std::vector<uint32_t> cols(tiles, 0u);  // blocks of each warp tile's longest block row
+    for (uint32_t br = 0; br < nbr; ++br)
+        cols[br / kTeamWarpBrows] = std::max(cols[br / kTeamWarpBrows], A.h_rows[br + 1] - A.h_rows[br]);
+    // The most warp tiles a CTA that fit whichever CTA it is.
+    for (uint32_t w = kTeamWarps; w >= 1; --w) {
+        const uint32_t size = (tiles + w - 1) / w;
+        if (size > (uint32_t)ctx_->sm_count) return;
+        uint64_t most = 0;
+        for (uint32_t c = 0; c < size; ++c) {
+            uint64_t sum = 0;
+            for (uint32_t q = c * w; q < std::min((c + 1) * w, tiles); ++q) sum += team_tile_bytes(cols[q]);
+            most = std::max(most, sum);
+        }
+        const uint64_t smem = kTeamFixedSmem + (uint64_t)w * kTeamLuBytes + most;
+        if (smem > (uint64_t)kTeamSmemMax) continue;
+        sl->team = size;
+        sl->team_warps = w;
+        sl->team_smem = (uint32_t)smem;
+        return;
+    }
 }
 
 int Engine::add(const MatA *A, const Precond *M, const SolveCfg &cfg, uint32_t *slot_out) {
@@ -302,7 +352,8 @@ int Engine::add(const MatA *A, const Precond *M, const SolveCfg &cfg, uint32_t *
     const size_t n = A->n, vf = a256((n + kPadElems) * sizeof(float));
     const uint64_t max_hist = cfg.max_iter > 0 ? cfg.max_iter : 1;
     sl->hist_cap = std::min<uint64_t>(cfg.hist_cap, max_hist);
-    size_t off[12], tot = 0;
+    team_plan(sl.get());
+    size_t off[14], tot = 0;
     auto take = [&](int k, size_t bytes) {
         off[k] = tot;
         tot += a256(bytes);
@@ -319,6 +370,8 @@ int Engine::add(const MatA *A, const Precond *M, const SolveCfg &cfg, uint32_t *
     take(9, sizeof(double2) * (M->n_utiles + 1));
     take(10, sizeof(double) * (sl->hist_cap + 1));
     take(11, cfg.algorithm == WSB_ALG_SINGLE_REDUCTION ? vf : 0);  // s
+    take(12, sl->team ? sizeof(unsigned long long) * n : 0);  // z packets
+    take(13, team_red_bytes(sl->team));                       // published partials
     void *mem = nullptr;
     cudaError_t e = cudaMallocAsync(&mem, tot, stream_);
     if (e != cudaSuccess)
@@ -340,6 +393,8 @@ int Engine::add(const MatA *A, const Precond *M, const SolveCfg &cfg, uint32_t *
     sl->part_b = (double2 *)(base + off[9]);
     sl->hist = sl->hist_cap ? (double *)(base + off[10]) : nullptr;
     sl->s = cfg.algorithm == WSB_ALG_SINGLE_REDUCTION ? (float *)(base + off[11]) : nullptr;
+    sl->zpk = (unsigned long long *)(base + off[12]);
+    sl->red = (RedEntry *)(base + off[13]);
 
     SysDesc &d = h_sys_[s];
     std::memset(&d, 0, sizeof d);
@@ -381,9 +436,11 @@ int Engine::add(const MatA *A, const Precond *M, const SolveCfg &cfg, uint32_t *
     d.history = sl->hist;
     d.algo = (uint32_t)cfg.algorithm;
     d.s = sl->s;
+    d.team_warps = sl->team_warps;
+    d.zpk = sl->zpk;
+    d.red = sl->red;
     std::memset(h_state_ + s, 0, sizeof(SysState));
-    if ((rc = push_desc(s))) return rc;
-    if ((rc = push_state(s))) return rc;
+    desc_dirty_ = state_dirty_ = true;
     if (s == slots_.size())
         slots_.push_back(std::move(sl));
     else
@@ -418,7 +475,8 @@ int Engine::set_rhs(uint32_t s, const float *b, const float *x0, bool dev) {
     // Restore the history window (mixed solves move it per sweep).
     h_sys_[s].history = sl.hist;
     h_sys_[s].hist_cap = (uint32_t)std::min<uint64_t>(sl.hist_cap, 0xffffffffu);
-    return push_desc(s);
+    desc_dirty_ = true;
+    return WSB_OK;
 }
 
 bool Engine::done(uint32_t s) const { return slots_[s] && slots_[s]->phase == Slot::DONE; }
@@ -432,7 +490,7 @@ uint32_t Engine::active_count() const {
 
 void Engine::remove(uint32_t s) {
     if (s >= slots_.size() || !slots_[s]) return;
-    if (slots_[s]->phase == Slot::RUNNING) work_dirty_ = true;
+    if (slots_[s]->phase == Slot::RUNNING && !slots_[s]->team) work_dirty_ = true;
     cudaFreeAsync(slots_[s]->mem, stream_);
     slots_[s].reset();
     std::memset(h_sys_ + s, 0, sizeof(SysDesc));
@@ -546,7 +604,7 @@ int Engine::rebuild_work() {
     size_t per = 1;
     for (uint32_t s = 0; s < slots_.size(); ++s) {
         const Slot *sl = slots_[s].get();
-        if (!sl) continue;
+        if (!sl || sl->team) continue;
         per += std::max<size_t>(std::max(sl->A->n_stiles, sl->M->n_utiles), chunks_of(sl->A->n));
         if (sl->phase != Slot::RUNNING) continue;
         ga.push_back({s, sl->A->n_stiles, sl->sgroups});
@@ -565,7 +623,7 @@ int Engine::rebuild_work() {
     w_work_b_ = lb.w;
     for (uint32_t s = 0; s < slots_.size(); ++s) {
         const Slot *sl = slots_[s].get();
-        if (!sl || sl->phase != Slot::RUNNING) continue;
+        if (!sl || sl->team || sl->phase != Slot::RUNNING) continue;
         for (uint32_t t = 0; t < chunks_of(sl->A->n); ++t) wc[nch++] = {s, t};
     }
     n_work_a_ = na;
@@ -717,7 +775,70 @@ int Engine::finish_slot(uint32_t s, int status) {
     return WSB_OK;
 }
 
-int Engine::step(uint32_t loop_limit, bool *any_left) {
+// One cooperative launch of k_team over the given systems, one CTA per SM.
+// When the device holds all their teams at once, each CTA has one system.
+// Otherwise the systems, widest first, each take the CTAs that are free
+// soonest; a CTA works through its systems in that one order, which every CTA
+// shares, so no two systems wait for each other.
+int Engine::launch_team(const std::vector<uint32_t> &ids, uint32_t limit, cudaStream_t st) {
+    if (ids.empty()) return WSB_OK;
+    const uint32_t sms = (uint32_t)std::max(1, ctx_->sm_count);
+    uint64_t total = 0;
+    uint32_t smem = 0;
+    for (uint32_t s : ids) {
+        total += slots_[s]->team;
+        smem = std::max(smem, slots_[s]->team_smem);
+    }
+    std::vector<uint32_t> order(ids);
+    std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return slots_[a]->team > slots_[b]->team; });
+    const uint32_t grid = (uint32_t)std::min<uint64_t>(total, sms);
+    std::vector<std::vector<TeamItem>> lists(grid);
+    std::vector<std::pair<double, uint32_t>> free_at(grid);
+    for (uint32_t c = 0; c < grid; ++c) free_at[c] = {0.0, c};
+    for (uint32_t s : order) {
+        const Slot &sl = *slots_[s];
+        std::sort(free_at.begin(), free_at.end());
+        // A solve's iterations grow about as the fourth root of its rows.
+        const double end = free_at[sl.team - 1].first + std::pow((double)sl.A->n, 0.25);
+        for (uint32_t k = 0; k < sl.team; ++k) {
+            lists[free_at[k].second].push_back({s, k, sl.team, 0u});
+            free_at[k].first = end;
+        }
+    }
+    size_t items = 0;
+    for (const auto &l : lists) items += l.size();
+    const size_t head = ((size_t)grid + 1 + 3) & ~size_t(3), words = head + 4 * items;
+    if (words > team_cap_) {
+        WSB_CUDA_TRY(ctx_, cudaStreamSynchronize(stream_));
+        cudaFree(d_team_);
+        cudaFreeHost(h_team_);
+        d_team_ = h_team_ = nullptr;
+        team_cap_ = 0;
+        const size_t nc = std::max<size_t>(1024, 2 * words);
+        WSB_CUDA_TRY(ctx_, cudaMalloc(&d_team_, sizeof(uint32_t) * nc));
+        WSB_CUDA_TRY(ctx_, cudaMallocHost(&h_team_, sizeof(uint32_t) * nc));
+        team_cap_ = nc;
+    }
+    TeamItem *it = reinterpret_cast<TeamItem *>(h_team_ + head);
+    uint32_t at = 0;
+    for (uint32_t c = 0; c < grid; ++c) {
+        h_team_[c] = at;
+        for (const TeamItem &q : lists[c]) it[at++] = q;
+    }
+    h_team_[grid] = at;
+    WSB_CUDA_TRY(ctx_, cudaMemcpyAsync(d_team_, h_team_, sizeof(uint32_t) * words, cudaMemcpyHostToDevice, st));
+    const SysDesc *dsys = d_sys_;
+    StepParams *dsp = d_sp_;
+    const TeamItem *ditems = reinterpret_cast<const TeamItem *>(d_team_ + head);
+    const uint32_t *doff = d_team_;
+    void *args[] = {&dsys, &dsp, &ditems, &doff, &limit};
+    WSB_CUDA_TRY(ctx_, cudaLaunchCooperativeKernel((const void *)k_team, dim3(grid), dim3(kTeamThreads), args, smem,
+                                                   st));
+    launches_ += 1;
+    return WSB_OK;
+}
+
+int Engine::step(uint32_t loop_limit, bool *any_left, uint32_t team_limit) {
     int rc;
     // The lists change only when the active set does (work_dirty_); the
     // layout is not free (a linear pass over every tile of every active
@@ -725,6 +846,7 @@ int Engine::step(uint32_t loop_limit, bool *any_left) {
     if ((work_dirty_ || work_cap_ == 0) && (rc = rebuild_work())) return rc;
     const bool timing = true;
     if (timing) cudaEventRecord(ev0_, stream_);
+    if ((rc = push_changes())) return rc;
     // 1) Mixed precision: refinement sweeps (x64 += d; r64 = b - A x64).
     std::vector<uint32_t> refine;
     for (uint32_t s = 0; s < slots_.size(); ++s)
@@ -758,9 +880,9 @@ int Engine::step(uint32_t loop_limit, bool *any_left) {
     std::vector<uint32_t> init;
     for (uint32_t s = 0; s < slots_.size(); ++s)
         if (slots_[s] && slots_[s]->phase == Slot::NEED_INIT) init.push_back(s);
-    uint32_t running = 0;
+    uint32_t running = 0;  // systems of the loop kernels
     for (auto &sl : slots_)
-        if (sl && sl->phase == Slot::RUNNING) ++running;
+        if (sl && sl->phase == Slot::RUNNING && !sl->team) ++running;
     // Empty systems finish at once: b.b == 0 gives Ok(0) (compute.rs:252-254).
     for (auto it = init.begin(); it != init.end();) {
         Slot &sl = *slots_[*it];
@@ -775,7 +897,16 @@ int Engine::step(uint32_t loop_limit, bool *any_left) {
     for (uint32_t s : init) {
         Slot &sl = *slots_[s];
         SysState &st = h_state_[s];
+        uint32_t epoch = st.epoch;
+        if (sl.red_dirty) {
+            WSB_CUDA_TRY(ctx_, cudaMemsetAsync(sl.red, 0, team_red_bytes(sl.team), stream_));
+            WSB_CUDA_TRY(ctx_, cudaMemsetAsync(sl.zpk, 0, sizeof(unsigned long long) * sl.A->n, stream_));
+            epoch = 0;
+            sl.red_dirty = false;
+        }
         std::memset(&st, 0, sizeof st);
+        st.epoch = epoch;
+        st.fresh = 1;
         st.active = 1;
         st.status = ST_RUNNING;
         if (sl.mixed) {
@@ -787,15 +918,21 @@ int Engine::step(uint32_t loop_limit, bool *any_left) {
             const uint64_t hoff = std::min<uint64_t>(sl.iters_total, sl.hist_cap);
             h_sys_[s].history = sl.hist ? sl.hist + hoff : nullptr;
             h_sys_[s].hist_cap = (uint32_t)std::min<uint64_t>(sl.hist_cap - hoff, 0xffffffffu);
-            if ((rc = push_desc(s))) return rc;
+            desc_dirty_ = true;
         } else {
             st.max_iter = (uint32_t)std::min<uint64_t>(sl.cfg.max_iter, 0xffffffffu);
             st.rel2 = (double)sl.cfg.rel_tol * (double)sl.cfg.rel_tol;
             st.abs2 = (double)sl.cfg.abs_tol * (double)sl.cfg.abs_tol;
         }
-        if ((rc = push_state(s))) return rc;
+        state_dirty_ = true;
         sl.phase = Slot::RUNNING;
     }
+    if ((rc = push_changes())) return rc;
+    // k_team forms its systems' first residual itself.
+    init.erase(std::remove_if(init.begin(), init.end(), [&](uint32_t s) { return slots_[s]->team != 0; }), init.end());
+    std::vector<uint32_t> team;
+    for (uint32_t s = 0; s < slots_.size(); ++s)
+        if (slots_[s] && slots_[s]->phase == Slot::RUNNING && slots_[s]->team) team.push_back(s);
     if (!init.empty()) work_dirty_ = true;
     if (work_dirty_ && (rc = rebuild_work())) return rc;
     if ((rc = launch_init(init))) return rc;
@@ -812,17 +949,35 @@ int Engine::step(uint32_t loop_limit, bool *any_left) {
     // system stops by its own max_iter, so the loop ends even if one did not.
     uint64_t budget = 1;
     for (auto &sl : slots_)
-        if (sl && sl->phase == Slot::RUNNING) {
+        if (sl && sl->phase == Slot::RUNNING && !sl->team) {
             const uint64_t done = h_state_[&sl - &slots_[0]].iter;
             const uint64_t mx = sl->mixed ? (sl->cfg.max_iter > sl->iters_total ? sl->cfg.max_iter - sl->iters_total : 0)
                                           : sl->cfg.max_iter;
             budget = std::max<uint64_t>(budget, (mx > done ? mx - done : 0) + 1);
         }
+    // Beside a k_team launch that runs to its end, so do the loop kernels.
+    const bool fork = !team.empty() && num_active_ > 0;
+    if (fork) loop_limit = std::max(loop_limit, team_limit);
     const uint32_t limit = (uint32_t)std::min<uint64_t>(loop_limit, std::min<uint64_t>(budget, 0xffffffffu));
     h_sp_->num_active = num_active_;
     h_sp_->loop_count = 0;
     h_sp_->loop_limit = limit;
     WSB_CUDA_TRY(ctx_, cudaMemcpyAsync(d_sp_, h_sp_, sizeof(StepParams), cudaMemcpyHostToDevice, stream_));
+    // With systems of both paths, k_team runs beside the loop kernels on a
+    // stream of its own: it waits on latency most of the time and leaves half
+    // of every SM's shared memory, which one CTA of each loop kernel fits in
+    // (48 systems of side 4-24: 30.1 ms one after the other, 29.3 ms so).
+    if (fork) {
+        if (!team_stream_) {
+            WSB_CUDA_TRY(ctx_, cudaStreamCreateWithFlags(&team_stream_, cudaStreamNonBlocking));
+            WSB_CUDA_TRY(ctx_, cudaEventCreateWithFlags(&fork_ev_, cudaEventDisableTiming));
+            WSB_CUDA_TRY(ctx_, cudaEventCreateWithFlags(&join_ev_, cudaEventDisableTiming));
+        }
+        WSB_CUDA_TRY(ctx_, cudaEventRecord(fork_ev_, stream_));
+        WSB_CUDA_TRY(ctx_, cudaStreamWaitEvent(team_stream_, fork_ev_, 0));
+    }
+    if ((rc = launch_team(team, std::max<uint32_t>(1, team_limit), fork ? team_stream_ : stream_))) return rc;
+    if (fork) WSB_CUDA_TRY(ctx_, cudaEventRecord(join_ev_, team_stream_));
     if (!init.empty()) {
         const uint32_t ga = std::min<uint32_t>(h_sp_->w_init_a, (uint32_t)max_grid_a_);
         const uint32_t gb = std::min<uint32_t>(h_sp_->w_init_b, (uint32_t)max_grid_b_);
@@ -867,11 +1022,13 @@ int Engine::step(uint32_t loop_limit, bool *any_left) {
             h_sp_->loop_count = done_iters;
         }
     }
+    if (fork) WSB_CUDA_TRY(ctx_, cudaStreamWaitEvent(stream_, join_ev_, 0));
     if (timing) cudaEventRecord(ev1_, stream_);
     // 3) Read back states; retire or hand finished inner solves to refinement.
     std::vector<uint32_t> run_ids;
     for (uint32_t s = 0; s < slots_.size(); ++s)
         if (slots_[s] && slots_[s]->phase == Slot::RUNNING) run_ids.push_back(s);
+    WSB_CUDA_TRY(ctx_, cudaMemcpyAsync(h_sp_rb_, d_sp_, sizeof(StepParams), cudaMemcpyDeviceToHost, stream_));
     if ((rc = read_states(run_ids))) return rc;
     float ms = 0.f;
     if (timing && cudaEventElapsedTime(&ms, ev0_, ev1_) == cudaSuccess) last_device_ms_ = ms;
@@ -895,7 +1052,7 @@ int Engine::step(uint32_t loop_limit, bool *any_left) {
         // Its device state is inactive, so the kernels skip its tiles: the
         // lists are re-laid out only once a quarter of their tiles belong to
         // systems that stopped (or when one joins), not at every retirement.
-        retired_tiles_ += (uint64_t)sl.A->n_stiles + sl.M->n_utiles;
+        if (!sl.team) retired_tiles_ += (uint64_t)sl.A->n_stiles + sl.M->n_utiles;
         if (sl.mixed) {
             if (st.status == ST_BREAKDOWN) sl.stalled = true;
             if (st.status == ST_MAXITER && sl.iters_total >= sl.cfg.max_iter) sl.stalled = true;
@@ -908,8 +1065,6 @@ int Engine::step(uint32_t loop_limit, bool *any_left) {
     }
     (void)body_iters;
     if (retired_tiles_ * 4 > listed_tiles_) work_dirty_ = true;
-    WSB_CUDA_TRY(ctx_, cudaMemcpyAsync(h_sp_rb_, d_sp_, sizeof(StepParams), cudaMemcpyDeviceToHost, stream_));
-    WSB_CUDA_TRY(ctx_, cudaStreamSynchronize(stream_));
     // Graph: the gate kernel once, then three body kernels per loop pass.
     if (num_active_ > 0 && n_work_a_ > 0)
         launches_ += use_graph_ ? 1 + 3ull * h_sp_rb_->loop_count : 3ull * h_sp_->loop_count;
@@ -918,8 +1073,11 @@ int Engine::step(uint32_t loop_limit, bool *any_left) {
         const uint32_t code = h_sp_rb_->error;
         const int rc2 = (code & kErrWaitMask) ? fail(ctx_, WSB_ERR_TIMEOUT, "a device wait ran out (kernel code %u)", code)
                                     : fail(ctx_, WSB_ERR_CUDA, "a kernel met an invalid work item (code %u)", code);
-        for (uint32_t s2 = 0; s2 < slots_.size(); ++s2)
-            if (slots_[s2] && slots_[s2]->phase == Slot::RUNNING) finish_slot(s2, rc2);
+        for (uint32_t s2 = 0; s2 < slots_.size(); ++s2) {
+            if (!slots_[s2]) continue;
+            if (slots_[s2]->team) slots_[s2]->red_dirty = true;
+            if (slots_[s2]->phase == Slot::RUNNING) finish_slot(s2, rc2);
+        }
         h_sp_->error = 0;
         WSB_CUDA_TRY(ctx_, cudaMemcpyAsync(d_sp_, h_sp_, sizeof(StepParams), cudaMemcpyHostToDevice, stream_));
         work_dirty_ = true;
@@ -942,7 +1100,8 @@ int Engine::profile_kernels(uint32_t s, uint32_t iters, double ms[5]) {
     st.active = 1;
     st.status = ST_RUNNING;
     st.max_iter = iters + 1;  // tolerances 0: runs all iterations
-    if ((rc = push_state(s))) return rc;
+    state_dirty_ = true;
+    if ((rc = push_changes())) return rc;
     sl.phase = Slot::RUNNING;
     work_dirty_ = true;
     if ((rc = rebuild_work())) return rc;

@@ -4,6 +4,7 @@
 #include <memory>
 
 #include "kernels_fused.cuh"
+#include "kernels_team.cuh"
 
 namespace wsb {
 
@@ -104,8 +105,10 @@ struct SolveOutcome {
 
 
 // Multi-system PCG engine. Systems are slots; each owns its Krylov vectors,
-// partial buffers and state in HBM. run()/step() iterate all active slots
-// together with one captured graph: a gate kernel, then a while loop of
+// partial buffers and state in HBM. A slot is iterated by one of two paths,
+// chosen when it is added (team_plan): systems that fit in the shared memory
+// of a team of CTAs by one cooperative launch of k_team; the others together
+// by one captured graph: a gate kernel, then a while loop of
 // {k_spmv, k_update, k_pupdate} that ends when no slot is active or after
 // loop_limit iterations. Between steps the host retires finished slots,
 // restarts refinement sweeps and rebuilds the work lists.
@@ -117,7 +120,12 @@ class Engine {
     // b, x0: n floats each, host (pinned or pageable) or device memory.
     int set_rhs(uint32_t slot, const float *b, const float *x0, bool device_ptrs);
     int run();                                       // all slots to completion
-    int step(uint32_t loop_limit, bool *any_left);   // one scheduler step
+    // One scheduler step: at most loop_limit iterations of every system
+    // (team_limit for the systems k_team iterates).
+    int step(uint32_t loop_limit, bool *any_left, uint32_t team_limit);
+    int step(uint32_t loop_limit, bool *any_left) { return step(loop_limit, any_left, loop_limit); }
+    // All systems added from now on go through the loop kernels (kernel timing).
+    void use_loop_kernels() { team_on_ = false; }
     int fetch(uint32_t slot, float *x, bool device_ptr, bool always_x, SolveOutcome *out, double *hist,
               uint64_t hist_cap, uint64_t *hist_len, double *x64 = nullptr);
     int reset_slot(uint32_t slot, const SolveCfg &cfg);  // reuse for another solve
@@ -145,13 +153,14 @@ class Engine {
     static uint32_t chunks_of(uint32_t n) { return (n + kChunkRows - 1) / kChunkRows; }
     // Work-list regions in d_work_ / h_work_ (work_cap_ items each).
     enum { L_A = 0, L_B = 1, L_C = 2, L_IA = 3, L_IB = 4, L_X = 5, kLists = 6 };
-    int push_desc(uint32_t slot);
-    int push_state(uint32_t slot);
+    int push_changes();
     int launch_init(const std::vector<uint32_t> &slots);
     int launch_aux(const std::vector<uint32_t> &slots, int which);
     int rebuild_work();
     int read_states(const std::vector<uint32_t> &slots);
     int finish_slot(uint32_t slot, int status);
+    void team_plan(Slot *sl) const;
+    int launch_team(const std::vector<uint32_t> &slots, uint32_t limit, cudaStream_t st);
 
     Context *ctx_;
     cudaStream_t stream_;
@@ -168,7 +177,13 @@ class Engine {
     std::vector<uint32_t> layout_tmp_;  // scratch of the work-list layout (column lengths / cursors)
     uint64_t listed_tiles_ = 0, retired_tiles_ = 0;  // tiles in the lists; of systems stopped since
     bool work_dirty_ = true;
+    bool desc_dirty_ = false, state_dirty_ = false;  // host mirrors changed since the last upload
     bool use_graph_ = true;   // WSB_LOOP=launch: plain launches + host polling
+    bool team_on_ = true;     // small systems take k_team
+    uint32_t *d_team_ = nullptr, *h_team_ = nullptr;  // k_team lists: item offsets, then items
+    cudaStream_t team_stream_ = nullptr;              // k_team beside the loop kernels
+    cudaEvent_t fork_ev_ = nullptr, join_ev_ = nullptr;
+    size_t team_cap_ = 0;                             // words of d_team_ / h_team_
     cudaGraph_t graph_ = nullptr;
     cudaGraphExec_t exec_ = nullptr;
     uint32_t graph_grid_a_ = 0, graph_grid_b_ = 0, graph_grid_c_ = 0;

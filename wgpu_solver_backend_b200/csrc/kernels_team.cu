@@ -1,0 +1,625 @@
+// k_team: see kernels_team.cuh.
+//
+// What bounds it: below about 25,000 block rows an iteration of the loop
+// kernels (kernels_fused.cu) costs 22-28 us whatever the size: three
+// dependent launches, each with its ramp, its chain of work-item loads and its
+// last-CTA sum. Here an iteration is two exchanges between resident CTAs and
+// the latency of one row sum and one block solve:
+//   - a lane owns a row: x, r, z, p and its row of the block's LU factors stay
+//     in registers; the matrix (and p at every block's columns) stays in
+//     shared memory, so an iteration reads only other CTAs' z from the L2;
+//   - p.Ap and then r.r and r.z are all-reduced: every CTA stores its FP64
+//     partial as one 16-byte {value, tag} and reads the whole team's in the
+//     same fixed order, so all CTAs hold the same scalars and take the same
+//     decisions after one hop (r.r by one warp, r.z by another);
+//   - z travels as 8-byte {value, tag} packets: a reader waits for the packets
+//     it needs and no fence or flag stands between the block solve and the
+//     next product. Every CTA forms p = z + beta p for the block columns it
+//     multiplies (same operation, same bits as the owner's), so p is never
+//     exchanged.
+// Measured (B200, us an iteration, loop kernels -> here): 4^3 nodes 24.4 -> 3.1,
+// 9^3 23.5 -> 4.7, 12^3 24.8 -> 5.2, 17^3 25.7 -> 6.1, 20^3 27.2 -> 7.5.
+// What is left is latency (7 of 13 warps wait at a barrier at any time, issue
+// slots 28 % used): per iteration two hops through the L2 (800 cycles for
+// 8 CTAs, 1,400 for 31), the FP64 sums (nine cycles an add, 36 with the shuffle
+// between lanes), two FP64 divisions and the block solve. So products are
+// added through shared memory, 16 per lane as a tree, before the lanes; a block
+// is solved by one lane from shared memory (no shuffles between its steps); and
+// all waits are warp-uniform loops: lanes that leave such a loop one by one
+// stay apart and made the code after it up to ten times slower.
+// Arithmetic is that of kernels_fused.cu operation by operation; only the
+// grouping of the FP64 sums differs.
+//
+// All CTAs of a launch are resident (cooperative launch); a CTA takes its
+// items in list order, and the lists are cut from one global order of systems,
+// so the first unfinished system always has all its CTAs. Every wait is
+// bounded (StepParams::wait_cycles): one that runs out sets kErrTeamWait, and
+// every CTA leaves.
+#include "kernels_team.cuh"
+
+namespace wsb {
+namespace {
+
+constexpr uint32_t kFull = 0xffffffffu;
+constexpr long long kTeamWaitCycles = 4000000000ll;  // about 2 s
+
+__device__ __forceinline__ void st_entry(RedEntry *e, double v, uint32_t tag) {
+    asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(e),
+                 "l"(__double_as_longlong(v)), "l"((long long)tag)
+                 : "memory");
+}
+__device__ __forceinline__ bool ld_entry(const RedEntry *e, uint32_t tag, double *v) {
+    long long lo, hi;
+    asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+                 : "=l"(lo), "=l"(hi)
+                 : "l"(e)
+                 : "memory");
+    *v = __longlong_as_double(lo);
+    return (uint32_t)hi == tag;
+}
+__device__ __forceinline__ void st_packet(unsigned long long *p, float v, uint32_t tag) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p),
+                 "l"((unsigned long long)__float_as_uint(v) | ((unsigned long long)tag << 32))
+                 : "memory");
+}
+// The packet, or `other` when !want.
+__device__ __forceinline__ unsigned long long ld_packet_if(const unsigned long long *p, bool want,
+                                                           unsigned long long other) {
+    unsigned long long v = other;
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.relaxed.gpu.global.u64 %0, [%1];\n\t}"
+                 : "+l"(v)
+                 : "l"(p), "r"((uint32_t)want)
+                 : "memory");
+    return v;
+}
+__device__ __forceinline__ uint32_t ld_error(const StepParams *sp) {
+    uint32_t v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&sp->error) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cp_async8(void *dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async4(void *dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Two FP32 products in one packed instruction, each rounded to nearest.
+__device__ __forceinline__ float2 mul2_rn(float2 a, float2 b) {
+    float2 r;
+    asm("{\n\t.reg .b64 ra, rb, rc;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
+        "mul.rn.f32x2 rc, ra, rb;\n\tmov.b64 {%0, %1}, rc;\n}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+
+// The fixed part of a CTA's shared memory.
+struct TeamShared {
+    double v[2][kTeamThreads];  // the rows' products of a reduction (the reducing warps': zero)
+    float z[kTeamThreads];      // the CTA's rows of r, then of z
+    double rz, beta;            // the last r.z and beta
+    uint2 alpha;                // alpha; 0: the system stops here
+    float beta_f;
+    uint32_t go;                // 0: the system stops here
+    uint32_t err;               // a wait ran out
+    // Scalars of the recurrence, kept by one thread (the same in every CTA).
+    double bb, rz_old, pap, alpha_d, rr, rel2, abs2;
+    uint32_t iter, max_iter, status, breakdown;
+    uint32_t bytes[kTeamWarps];  // shared memory of each warp tile
+};
+static_assert(sizeof(TeamShared) <= kTeamFixedSmem && kTeamFixedSmem % 128 == 0, "fixed shared memory");
+
+struct WaitCtl {
+    StepParams *sp;
+    long long lim;
+};
+
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(kFull, v, o);
+    return v;
+}
+
+// Sum of one value per thread of the CTA, by one warp: lane l adds 16 of them
+// as a tree, then the lanes; valid in lane 0.
+__device__ __forceinline__ double cta_sum(const double *v, uint32_t lane) {
+    constexpr int kHalf = kTeamThreads / 64;
+    double s[kHalf];
+#pragma unroll
+    for (int k = 0; k < kHalf; ++k) {
+        const double2 a = reinterpret_cast<const double2 *>(v)[32 * k + lane];
+        s[k] = a.x + a.y;
+    }
+#pragma unroll
+    for (int h = kHalf / 2; h > 0; h >>= 1)
+#pragma unroll
+        for (int k = 0; k < h; ++k) s[k] += s[k + h];
+    return warp_sum(s[0]);
+}
+
+// Sum over the team of the partials in red[0 .. size), by one warp: lane l adds
+// entries l, l + 32, ... in order, then the lanes; valid in lane 0. Each round
+// keeps kPollBatch loads a lane in flight.
+constexpr int kPollBatch = 5;
+__device__ __noinline__ double team_gather(TeamShared &S, const RedEntry *red, uint32_t size, uint32_t tag,
+                                           StepParams *sp, long long lim) {
+    const uint32_t lane = threadIdx.x & 31u;
+    double sum = 0.0;
+    const long long t0 = clock64();
+#pragma unroll 1
+    for (uint32_t b = 0; b < size; b += 32u * kPollBatch) {
+        double v[kPollBatch];
+#pragma unroll 1
+        for (uint32_t k = 1;; ++k) {
+            bool ok = true;
+#pragma unroll
+            for (int j = 0; j < kPollBatch; ++j) {
+                if (b + 32u * j < size) ok = ld_entry(red + min(b + 32u * j + lane, size - 1u), tag, &v[j]) && ok;
+            }
+            if (__all_sync(kFull, ok)) break;
+            if (__any_sync(kFull, clock64() - t0 > lim) || ((k & 255u) == 0 && __any_sync(kFull, ld_error(sp) != 0))) {
+                S.err = 1;
+                return 0.0;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kPollBatch; ++j)
+            if (b + 32u * j + lane < size) sum += v[j];
+    }
+    return warp_sum(sum);
+}
+
+// a / b, or 0 when b is 0: an FP32 approximate reciprocal of b, two Newton steps, then
+// the product corrected once by its residual (Markstein, IBM J. Res. Dev. 34,
+// 1990); about 130 cycles against 420 for the division, which operands outside
+// [2^-100, 2^100] take.
+__device__ __noinline__ double quotient(double a, double b) {
+    if (b == 0.0) return 0.0;
+    const double aa = fabs(a), ab = fabs(b);
+    if (!(aa >= 7.888609052210118e-31 && aa <= 1.2676506002282294e30 && ab >= 7.888609052210118e-31 &&
+          ab <= 1.2676506002282294e30))
+        return a / b;
+    float seed;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(seed) : "f"((float)b));
+    double y = (double)seed;
+    y = __fma_rn(__fma_rn(-b, y, 1.0), y, y);
+    y = __fma_rn(__fma_rn(-b, y, 1.0), y, y);
+    const double q = __dmul_rn(a, y);
+    return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+
+// v / u correctly rounded, y = RN(1 / u) formed beforehand: q = v y, then
+// twice q += (v - u q) y in fused operations. By Markstein's theorem the last
+// step rounds correctly when q is within one ulp and nothing under- or
+// overflows, which lo <= |v| <= 2^60 ensures (lo = 2^-60 for |u| in
+// [2^-40, 2^40], else infinity); a zero v keeps the product's sign. *ok is
+// cleared for other operands, whose quotient is the division's.
+constexpr float kDivLo = 8.673617e-19f, kDivHi = 1.1529215e18f;  // 2^-60, 2^60
+__device__ __forceinline__ float div_by(float v, float u, float y, float lo, bool *ok) {
+    const float av = fabsf(v), q0 = __fmul_rn(v, y);
+    float q = __fmaf_rn(__fmaf_rn(-u, q0, v), y, q0);
+    q = __fmaf_rn(__fmaf_rn(-u, q, v), y, q);
+    *ok = *ok && ((av >= lo && av <= kDivHi) || (av == 0.0f && lo <= kDivHi));
+    return av == 0.0f ? q0 : q;
+}
+// Backward substitution with plain divisions.
+__device__ __noinline__ void back_general(const float *lu, const float *y, float *x) {
+#pragma unroll 1
+    for (int i = 5; i >= 0; --i) {
+        float v = y[i];
+#pragma unroll 1
+        for (int q = i + 1; q < 6; ++q) v = __fsub_rn(v, __fmul_rn(lu[6 * i + q], x[q]));
+        x[i] = __fdiv_rn(v, lu[7 * i]);
+    }
+}
+
+constexpr uint32_t kLocal = 0x80000000u;  // a block column inside the CTA's rows
+
+// One system, this CTA's rows, up to `limit` iterations.
+__device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamItem it, uint32_t limit, TeamShared &S,
+                                                 char *dyn, const WaitCtl &w) {
+    constexpr int kAhead = 8;  // block columns a lane handles at once
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    SysState *st = D.st;
+    if (!st->active) return;
+    const uint32_t nbr = D.n / 6u, tw = D.team_warps, cta_brows = tw * (uint32_t)kTeamWarpBrows;
+    const bool lead = it.rank == 0, alone = it.size == 1;
+    const uint32_t br0 = min(it.rank * cta_brows, nbr), br1 = min(br0 + cta_brows, nbr);
+    const bool fresh = st->fresh != 0;
+    // The lane's row.
+    const uint32_t bo = lane / 6u, a = lane % 6u;
+    const uint32_t br = br0 + warp * (uint32_t)kTeamWarpBrows + bo;
+    const bool on = lane < (uint32_t)kTeamWarpRows && warp < tw && br < br1;
+    const uint32_t row = on ? 6u * br + a : 0u;
+    uint32_t k0 = 0, nk = 0;
+    float x = 0.f, r = 0.f, z = 0.f, p = 0.f;
+    if (on) {
+        k0 = D.brow_ptr[br];
+        nk = D.brow_ptr[br + 1] - k0;
+        x = D.x[row];
+        if (!fresh) {
+            r = D.r[row];
+            z = D.z[row];
+            p = D.p[row];
+        }
+    }
+    const uint32_t cols = __reduce_max_sync(kFull, nk);  // of the warp tile
+    if (lane == 0 && warp < (uint32_t)kTeamWarps) S.bytes[warp] = team_tile_bytes(cols);
+    S.v[0][tid] = S.v[1][tid] = 0.0;
+    __syncthreads();
+    // Dynamic shared memory: LU factors of the CTA's block rows; then for each
+    // warp tile and block j of its block rows, lane by lane (no bank
+    // conflicts), the row's first four values, its last two, p at the block's
+    // columns, and the first row of the block's columns (in the system, or
+    // with kLocal in S.z).
+    float *lu = reinterpret_cast<float *>(dyn) + (size_t)warp * (kTeamLuBytes / 4);
+    uint32_t before = 0;
+    for (uint32_t q = 0; q < min(warp, tw); ++q) before += S.bytes[q];
+    char *mine = dyn + (size_t)tw * kTeamLuBytes + before;
+    // (cols == 0: a warp without rows; it touches none of this.)
+    const uint32_t colp = (cols + 7u) & ~7u;
+    float4 *b4 = reinterpret_cast<float4 *>(mine) + lane;
+    float2 *b2 = reinterpret_cast<float2 *>(mine + (size_t)cols * 16u * kTeamWarpRows) + lane;
+    float *xg = reinterpret_cast<float *>(mine + (size_t)cols * 24u * kTeamWarpRows) + 8u * bo;
+    uint32_t *bc = reinterpret_cast<uint32_t *>(mine + (size_t)cols * kTeamColBytes);
+    for (uint32_t j = lane; j < colp * (uint32_t)(kTeamWarpBrows + 1); j += 32u) bc[j] = kLocal;  // past a row's end
+    bc += colp * bo;
+    __syncwarp();
+    if (on) {
+        // p (or x0 for a fresh system) at the block columns, one component a lane.
+        const float *src = (fresh ? D.x : D.p) + a;
+#pragma unroll 1
+        for (uint32_t j = 0; j < nk; ++j) {
+            const float *v = D.bval + (size_t)(k0 + j) * 36u + 6u * a;
+            float4 *d4 = b4 + j * kTeamWarpRows;
+            cp_async8(d4, v);
+            cp_async8(reinterpret_cast<float2 *>(d4) + 1, v + 2);
+            cp_async8(b2 + j * kTeamWarpRows, v + 4);
+            const uint32_t c = D.bcol[k0 + j];
+            cp_async4(xg + 8u * kTeamWarpBrows * j + a, src + 6u * (size_t)c);
+            if (a == 0)
+                bc[j] =
+                    c >= br0 && c < br1 ? kLocal | (32u * ((c - br0) / kTeamWarpBrows) + 6u * ((c - br0) % kTeamWarpBrows))
+                                        : 6u * c;
+        }
+        // The lane's row of the LU factors; lane a == 0 solves the block.
+#pragma unroll
+        for (int q = 0; q < 3; ++q) cp_async8(lu + 36u * bo + 6u * a + 2 * q, D.lu + (size_t)br * 36u + 6u * a + 2 * q);
+    }
+    cp_async_wait_all();
+    __syncwarp();
+    const uint32_t sbo = min(lane, (uint32_t)kTeamWarpBrows - 1u);  // the block row that this lane solves
+    const bool solver = lane < (uint32_t)kTeamWarpBrows && warp < tw && br0 + warp * (uint32_t)kTeamWarpBrows + lane < br1;
+    const float *slu = lu + 36u * sbo;
+    float rdiag[6], dlo = kDivLo;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        const float u = solver ? slu[7 * i] : 1.0f, au = fabsf(u);
+        rdiag[i] = __frcp_rn(u);
+        if (!(au >= 9.094947e-13f && au <= 1.0995116e12f)) dlo = __int_as_float(0x7f800000);  // 2^-40, 2^40
+    }
+    __syncthreads();
+
+    // y = (row) . xg: products rounded, added in index order; the operands of
+    // the next block are loaded before this block's products are added.
+    auto row_sum = [&]() {
+        float acc = 0.0f;
+        const float4 *B4 = b4;
+        const float2 *B2 = b2;
+        const float4 *X = reinterpret_cast<const float4 *>(xg);
+        float4 v, x;
+        float2 v2, x2;
+        if (nk) v = B4[0], v2 = B2[0], x = X[0], x2 = *reinterpret_cast<const float2 *>(X + 1);
+#pragma unroll 2
+        for (uint32_t j = 0; j < nk; ++j) {
+            const float2 q0 = mul2_rn(make_float2(v.x, v.y), make_float2(x.x, x.y));
+            const float2 q1 = mul2_rn(make_float2(v.z, v.w), make_float2(x.z, x.w));
+            const float2 q2 = mul2_rn(v2, x2);
+            if (j + 1 < nk) {
+                B4 += kTeamWarpRows, B2 += kTeamWarpRows, X += 2 * kTeamWarpBrows;
+                v = *B4, v2 = *B2, x = X[0], x2 = *reinterpret_cast<const float2 *>(X + 1);
+            }
+            acc = __fadd_rn(acc, q0.x);
+            acc = __fadd_rn(acc, q0.y);
+            acc = __fadd_rn(acc, q1.x);
+            acc = __fadd_rn(acc, q1.y);
+            acc = __fadd_rn(acc, q2.x);
+            acc = __fadd_rn(acc, q2.y);
+        }
+        return acc;
+    };
+    // z = U^-1 L^-1 r of the warp tile's blocks, one lane a block, in the
+    // order of block_jacobi.wgsl:93-126; r comes and z goes through S.z.
+    float *const wz = S.z + 32u * warp;
+    auto block_solve = [&]() {
+        wz[lane] = r;
+        __syncwarp();
+        if (solver) {
+            float y[6], pr[6];
+            bool ok = true;
+            float *const rz = wz + 6u * sbo;
+            float l[36];
+#pragma unroll
+            for (int q = 0; q < 9; ++q) {
+                const float4 v = reinterpret_cast<const float4 *>(slu)[q];
+                l[4 * q] = v.x, l[4 * q + 1] = v.y, l[4 * q + 2] = v.z, l[4 * q + 3] = v.w;
+            }
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                const float2 v = reinterpret_cast<const float2 *>(rz)[i];
+                y[2 * i] = v.x, y[2 * i + 1] = v.y;
+            }
+#pragma unroll
+            for (int i = 1; i < 6; ++i)
+#pragma unroll
+                for (int q = 0; q < i; ++q) y[i] = __fsub_rn(y[i], __fmul_rn(l[6 * i + q], y[q]));
+#pragma unroll
+            for (int i = 5; i >= 0; --i) {
+                float v = y[i];
+#pragma unroll
+                for (int q = i + 1; q < 6; ++q) v = __fsub_rn(v, __fmul_rn(l[6 * i + q], pr[q]));
+                pr[i] = div_by(v, l[7 * i], rdiag[i], dlo, &ok);
+            }
+            if (ok) {
+#pragma unroll
+                for (int i = 0; i < 3; ++i) reinterpret_cast<float2 *>(rz)[i] = make_float2(pr[2 * i], pr[2 * i + 1]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 6; ++i) rz[i] = y[i];
+                back_general(slu, rz, rz);
+            }
+        }
+        __syncwarp();
+        return wz[lane];
+    };
+
+    uint32_t tag = st->epoch;
+    // This CTA's copy of the partials, and where lane l < copies stores copy l.
+    const uint32_t copies = team_copies(it.size);
+    const RedEntry *const red = D.red + (size_t)(it.rank % copies) * kRedEntries * it.size;
+    RedEntry *const out = D.red + (size_t)(lane % copies) * kRedEntries * it.size + it.rank;
+    unsigned long long *const zpk = D.zpk;
+    // The last two warps have no rows: they reduce. The first of them sums
+    // p.Ap and r.r and decides, the second sums r.z and forms beta.
+    const bool red_a = warp == (uint32_t)kTeamWarps, red_b = warp == (uint32_t)kTeamWarps + 1u;
+    if (red_a && lane == 0) {
+        S.bb = st->bb;
+        S.rr = S.pap = S.alpha_d = S.beta = 0.0;
+        S.beta_f = 0.0f;
+        S.rz = S.rz_old = st->rz_old;
+        S.rel2 = st->rel2;
+        S.abs2 = st->abs2;
+        S.iter = st->iter;
+        S.max_iter = st->max_iter;
+        S.status = ST_RUNNING;
+        S.breakdown = 0;
+    }
+
+    // The z packets of the row's block columns outside the CTA, one component
+    // a lane: requested, and waited for while the scalars are reduced.
+    auto block_cols = [&](uint32_t j0, uint32_t c[kAhead]) {
+#pragma unroll
+        for (int q = 0; q < kAhead / 4; ++q) {
+            const uint4 v = reinterpret_cast<const uint4 *>(bc + j0)[q];
+            c[4 * q] = v.x, c[4 * q + 1] = v.y, c[4 * q + 2] = v.z, c[4 * q + 3] = v.w;
+        }
+    };
+    unsigned long long zin[kAhead];
+    auto fetch_z = [&](uint32_t j0) {
+        const long long t0 = clock64();
+#pragma unroll 1
+        for (uint32_t k = 1;; ++k) {
+            uint32_t bad = 0;
+            uint32_t c[kAhead];
+            block_cols(j0, c);
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j)
+                zin[j] = ld_packet_if(zpk + c[j] + a, !(c[j] & kLocal), (unsigned long long)tag << 32);
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j) bad |= (uint32_t)(zin[j] >> 32) ^ tag;
+            if (__all_sync(kFull, bad == 0)) break;
+            if (__any_sync(kFull, clock64() - t0 > w.lim) || ((k & 255u) == 0 && __any_sync(kFull, ld_error(w.sp) != 0))) {
+                S.err = 1;
+                break;
+            }
+        }
+    };
+    // p = z + beta p of the lane's row and of its block columns (p = z when
+    // first); p at the first kAhead columns also stays in registers. All
+    // operands come before the first store, which the compiler could not move
+    // a load across.
+    float po[kAhead];
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) po[j] = (uint32_t)j < nk ? xg[8u * kTeamWarpBrows * j + a] : 0.0f;
+    auto advance = [&](bool first, float bf) {
+        p = first ? z : __fadd_rn(__fmul_rn(p, bf), z);
+#pragma unroll 1
+        for (uint32_t j0 = 0; j0 < cols; j0 += kAhead) {
+            if (j0) fetch_z(j0);
+            float *dst = xg + 8u * kTeamWarpBrows * j0 + a;
+            uint32_t c[kAhead];
+            float pn[kAhead];
+            block_cols(j0, c);
+            if (j0) {
+#pragma unroll
+                for (int j = 0; j < kAhead; ++j) pn[j] = j0 + j < nk ? dst[8u * kTeamWarpBrows * j] : 0.0f;
+            } else {
+#pragma unroll
+                for (int j = 0; j < kAhead; ++j) pn[j] = po[j];
+            }
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j) {
+                const bool local = (c[j] & kLocal) != 0;
+                const float zl = S.z[local ? (c[j] & ~kLocal) + a : 0u];
+                const float zj = local ? zl : __uint_as_float((uint32_t)zin[j]);
+                pn[j] = first ? zj : __fadd_rn(__fmul_rn(pn[j], bf), zj);
+            }
+            if (j0 == 0) {
+#pragma unroll
+                for (int j = 0; j < kAhead; ++j) po[j] = pn[j];
+            }
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j)
+                if (j0 + j < nk) dst[8u * kTeamWarpBrows * j] = pn[j];
+        }
+        __syncwarp();
+    };
+
+    // Results of a reduction are written between its two barriers and read by
+    // all after the second; S.err may change at any time. The first pass of a
+    // fresh system has xg = x0 and stands for k_init: r = b - A x0, z = M r,
+    // b.b and r.z, p = z.
+    bool init = fresh;
+    uint32_t done = 0;
+    for (;;) {
+        ++tag;
+        float ap = 0.0f;
+        if (!red_a && !red_b) {
+            ap = row_sum();
+            __syncwarp();
+        }
+        if (init) {
+            const float bi = on ? __ldg(D.b + row) : 0.0f;
+            r = __fsub_rn(bi, ap);
+            S.v[0][tid] = (double)bi * (double)bi;
+        } else {
+            S.v[0][tid] = (double)p * (double)ap;
+            __syncthreads();
+            if (red_a) {
+                const double rz_old = S.rz;
+                double pap = cta_sum(S.v[0], lane);
+                if (!alone) {
+                    pap = __shfl_sync(kFull, pap, 0);
+                    if (lane < copies) st_entry(out, pap, tag);
+                    __syncwarp();
+                    pap = team_gather(S, red, it.size, tag, w.sp, w.lim);
+                }
+                if (lane == 0) {
+                    const double alpha = quotient(rz_old, pap);
+                    S.rz_old = rz_old;
+                    S.pap = pap;
+                    S.alpha_d = alpha;
+                    S.alpha = make_uint2(__float_as_uint((float)alpha), S.err ? 0u : 1u);
+                }
+            }
+            __syncthreads();
+            const uint2 al2 = S.alpha;
+            if (!al2.y) break;
+            const float al = __uint_as_float(al2.x), ma = -al;
+            x = __fadd_rn(x, __fmul_rn(al, p));
+            r = __fadd_rn(r, __fmul_rn(ma, ap));
+            if (!on) r = 0.0f;
+        }
+        if (!red_a && !red_b) {
+            z = block_solve();
+            if (on && !alone) st_packet(zpk + row, z, tag);
+            if (!init) S.v[0][tid] = (double)r * (double)r;
+            S.v[1][tid] = (double)r * (double)z;
+        }
+        __syncthreads();
+        if (red_a || red_b) {
+            const double *v = red_a ? S.v[0] : S.v[1];
+            const uint32_t slot = (red_a ? 1u : 2u) * it.size;
+            double sum = cta_sum(v, lane);
+            if (!alone) {
+                sum = __shfl_sync(kFull, sum, 0);
+                if (lane < copies) st_entry(out + slot, sum, tag);
+                __syncwarp();
+                sum = team_gather(S, red + slot, it.size, tag, w.sp, w.lim);
+            }
+            if (lane == 0 && red_b) {
+                const double beta = quotient(sum, S.rz);
+                S.beta = beta;
+                S.beta_f = (float)beta;
+                S.rz = sum;
+            } else if (lane == 0) {
+                uint32_t status = ST_RUNNING;
+                if (init) {
+                    S.bb = sum;
+                    if (sum == 0.0) status = ST_CONVERGED;
+                    else if (S.max_iter == 0) status = ST_MAXITER;
+                } else {
+                    const uint32_t iter = S.iter;
+                    S.rr = sum;
+                    if (lead && D.history && iter < D.hist_cap) D.history[iter] = sum;
+                    if (S.pap == 0.0) {
+                        status = ST_BREAKDOWN;
+                        S.breakdown = 1;
+                    } else if (S.rz_old == 0.0) {
+                        status = ST_BREAKDOWN;
+                        S.breakdown = 2;
+                    } else if (sum <= S.abs2 || sum <= S.rel2 * S.bb) {
+                        status = ST_CONVERGED;
+                    } else if (iter + 1 >= S.max_iter) {
+                        status = ST_MAXITER;
+                    }
+                    S.iter = iter + 1;
+                }
+                S.status = status;
+                S.go = status == ST_RUNNING && !S.err;
+            }
+        } else if (!alone && cols) {
+            fetch_z(0);
+        }
+        __syncthreads();
+        if (!S.go) break;
+        if (!red_a && !red_b) advance(init, S.beta_f);
+        if (!init && ++done >= limit) break;
+        init = false;
+    }
+    __syncthreads();
+    if (S.err) {
+        if (tid == 0) atomicOr(&w.sp->error, kErrTeamWait);
+        return;
+    }
+    if (on) {
+        D.x[row] = x;
+        D.r[row] = r;
+        D.z[row] = z;
+        D.p[row] = p;
+    }
+    if (lead && red_a && lane == 0) {
+        const bool running = S.status == ST_RUNNING, none = S.iter == 0;  // none: stopped before the first iteration
+        st->bb = S.bb;
+        st->rz_old = running || none ? S.rz : S.rz_old;
+        st->pap = S.pap;
+        st->rr = S.rr;
+        st->rz_new = none ? 0.0 : S.rz;
+        st->alpha = S.alpha_d;
+        st->beta = none ? 0.0 : S.beta;
+        st->alpha_f = (float)S.alpha_d;
+        st->beta_f = none ? 0.0f : S.beta_f;
+        st->iter = S.iter;
+        st->status = S.status;
+        st->breakdown = S.breakdown;
+        st->epoch = tag;
+        st->fresh = 0;
+        st->active = running ? 1u : 0u;
+    }
+}
+
+}  // namespace
+
+__global__ void __launch_bounds__(kTeamThreads, 1)
+    k_team(const SysDesc *__restrict__ sys, StepParams *sp, const TeamItem *__restrict__ items,
+           const uint32_t *__restrict__ item_off, uint32_t limit) {
+    extern __shared__ __align__(128) char smem[];
+    TeamShared &S = *reinterpret_cast<TeamShared *>(smem);
+    const unsigned long long wl = sp->wait_cycles;
+    const WaitCtl w{sp, wl == 0 || wl > (unsigned long long)kTeamWaitCycles ? kTeamWaitCycles : (long long)wl};
+    if (threadIdx.x == 0) S.err = 0;
+    __syncthreads();
+    const uint32_t i1 = item_off[blockIdx.x + 1];
+    for (uint32_t i = item_off[blockIdx.x]; i < i1; ++i) {
+        const TeamItem it = items[i];
+        team_system_bsr6(sys[it.sys], it, limit, S, smem + kTeamFixedSmem, w);
+        __syncthreads();
+        if (S.err) return;  // every CTA's later waits would run out as well
+    }
+}
+
+}  // namespace wsb

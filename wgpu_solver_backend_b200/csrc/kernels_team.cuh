@@ -1,0 +1,51 @@
+// Persistent PCG kernels: whole solves (or steps of a solve) in one launch.
+//
+// k_team iterates systems whose matrix fits in the shared memory of the CTAs
+// that share it (a "team"): the matrix is read once per launch, the vectors
+// live in registers, and the CTAs of a team meet in two all-reduces per
+// iteration over global memory.
+#pragma once
+#include "wsb_internal.h"
+
+namespace wsb {
+
+// A system's rows are cut into warp tiles (one row a lane, no block cut;
+// kTeamWarpBrows block rows for BSR6); a CTA of its team holds a fixed number
+// of consecutive warp tiles, at most kTeamWarps. The cut depends on the matrix
+// alone, so a system's arithmetic does not depend on what else runs.
+constexpr int kTeamWarps = 14;
+constexpr int kTeamThreads = 32 * (kTeamWarps + 2);  // two more warps reduce
+constexpr int kTeamWarpBrows = 5;
+constexpr int kTeamWarpRows = 6 * kTeamWarpBrows;
+// Shared memory of a CTA: a fixed part, kTeamLuBytes of LU factors per warp
+// tile, then per warp tile kTeamColBytes for each block of its longest block
+// row (values, p at the block columns) and kTeamIdxBytes for each eight of
+// them begun (block columns).
+constexpr int kTeamFixedSmem = 10624;
+constexpr int kTeamLuBytes = 144 * kTeamWarpBrows;
+constexpr int kTeamColBytes = 24 * kTeamWarpRows + 32 * kTeamWarpBrows;
+constexpr int kTeamIdxBytes = 32 * (kTeamWarpBrows + 1);
+constexpr int kTeamSmemMax = 227 * 1024;
+__host__ __device__ constexpr uint32_t team_tile_bytes(uint32_t cols) {
+    return kTeamColBytes * cols + kTeamIdxBytes * ((cols + 7u) / 8u);
+}
+static_assert(kTeamLuBytes % 16 == 0 && kTeamColBytes % 16 == 0 && kTeamIdxBytes % 16 == 0, "16-byte operands");
+
+// Copies of the published partials of a team, each read by every copies-th
+// CTA: with one copy, the polls of a hundred CTAs on the same few cache lines
+// hold up the stores (106 CTAs: 8.6 us an iteration against 7.5 with four);
+// fewer CTAs are faster with one store (71 CTAs: 6.1 against 6.8 with three).
+__host__ __device__ constexpr uint32_t team_copies(uint32_t size) { return size <= 96u ? 1u : 4u; }
+__host__ __device__ constexpr uint64_t team_red_entries(uint32_t size) {
+    return (uint64_t)kRedEntries * size * team_copies(size);
+}
+
+// Launched cooperatively, one CTA per SM, with kTeamThreads threads: CTA c
+// works through items [item_off[c], item_off[c + 1]), each for up to `limit`
+// iterations. (Two CTAs an SM, at 64 registers a thread, spilled, and the
+// spills did not fit in what L1 the shared memory leaves: 26 systems of 9^3
+// nodes 13.5 us an iteration against 10.7.)
+__global__ void k_team(const SysDesc *__restrict__ sys, StepParams *sp, const TeamItem *__restrict__ items,
+                       const uint32_t *__restrict__ item_off, uint32_t limit);
+
+}  // namespace wsb

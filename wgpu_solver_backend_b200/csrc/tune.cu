@@ -113,6 +113,7 @@ using namespace wsb;
 static int time_tiling(Context *ctx, MatA *A, Precond *M, const float *d_b, uint32_t iters, double *spmv_ms,
                        double *upd_ms) {
     Engine E(ctx, ctx->stream);
+    E.use_loop_kernels();
     SolveCfg cfg;
     cfg.max_iter = iters + 1;
     uint32_t slot;

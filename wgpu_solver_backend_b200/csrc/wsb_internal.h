@@ -101,11 +101,20 @@ struct alignas(64) SysState {
     uint32_t iter, max_iter, status, active;
     uint32_t cnt_a, cnt_b;      // last-CTA tickets of the two reductions
     uint32_t breakdown;         // 1: pAp == 0, 2: rz_old == 0
-    uint32_t pad0;
+    uint32_t epoch;             // persistent kernels: tag of the last all-reduce
     double rr64, bb64;          // FP64 true residual and ||b||^2 (mixed precision)
-    uint32_t cnt_c, pad1;
+    uint32_t cnt_c;
+    uint32_t fresh;             // persistent kernels: r, z, p and the first scalars are still to be formed
     double gamma_prev;          // single reduction: (r, u) of the previous iteration
 };
+
+// A published partial sum: written and read as one 16-byte access, valid once
+// its tag is the expected one.
+struct alignas(16) RedEntry {
+    double v;
+    unsigned long long tag;
+};
+constexpr uint32_t kRedEntries = 3;  // p.Ap, r.r, r.z
 
 // Read-mostly description of one system in device memory.
 struct SysDesc {
@@ -128,8 +137,17 @@ struct SysDesc {
     double2 *part_b;                   // (r.r, r.z) partials of each update tile group (refinement: of each tile)
     SysState *st;
     double *history;                   // hist_cap entries or null
-    uint32_t algo, pad_algo;           // Algo
+    uint32_t algo;                     // Algo
+    uint32_t team_warps;               // k_team: warp tiles a CTA holds (0: iterated by other kernels)
     float *s;                          // single reduction: s = A p (by recurrence)
+    unsigned long long *zpk;           // k_team: z of each row with the tag of its all-reduce (value low, tag high)
+    RedEntry *red;                     // k_team: published partials (team_red_entries)
+};
+
+// One CTA's part of one system in a k_team launch: member `rank` of the `size`
+// CTAs that share system `sys`.
+struct TeamItem {
+    uint32_t sys, rank, size, pad;
 };
 
 // Bits of StepParams::error. The wait bits mean a bounded mbarrier wait ran
@@ -143,8 +161,9 @@ constexpr uint32_t kErrBadItem = 8u;            // invalid work item
 constexpr uint32_t kErrSpmvProducerWait = 16u;  // SpMV producer: a free stage
 constexpr uint32_t kErrUpdProducerWait = 32u;   // update producer: a free stage
 constexpr uint32_t kErrGatherWait = 64u;        // SpMV gather warp: a tile descriptor
+constexpr uint32_t kErrTeamWait = 128u;         // persistent kernels: another CTA's partial sum or vector entry
 constexpr uint32_t kErrWaitMask = kErrSpmvConsumerWait | kErrUpdConsumerWait | kErrInitConsumerWait |
-                                  kErrSpmvProducerWait | kErrUpdProducerWait | kErrGatherWait;
+                                  kErrSpmvProducerWait | kErrUpdProducerWait | kErrGatherWait | kErrTeamWait;
 
 // Kernel parameters of one loop step that the host may change between graph
 // launches (work lists, counts); lives in device memory so a captured graph
