@@ -163,12 +163,21 @@ struct Engine::Slot {
     // k_team (team > 0): CTAs of the system's team, warp tiles a CTA holds and
     // its shared memory, published partials, z packets.
     uint32_t team = 0, team_warps = 0, team_smem = 0;
+    // k_stream (stream > 0): CTAs; its second buffer of p and partials.
+    uint32_t stream = 0;
+    float *p2 = nullptr;
+    bool looped() const { return team == 0 && stream == 0; }
+    uint32_t red_ctas() const { return team ? team : stream; }
     RedEntry *red = nullptr;
     unsigned long long *zpk = nullptr;
     bool red_dirty = false;  // a launch failed: the slots' tags are not the state's
 };
 
 static size_t team_red_bytes(uint32_t team) { return sizeof(RedEntry) * team_red_entries(team); }
+
+// Matrix and factors up to this size are left to stay in the L2 (126 MB) beside
+// the vectors; k_stream reads larger ones past it.
+constexpr uint64_t kL2Keep = 80ull << 20;
 
 enum { AUX_REFINE = 0, AUX_RESID = 1, AUX_X32 = 2 };
 
@@ -191,6 +200,8 @@ Engine::Engine(Context *ctx, cudaStream_t stream) : ctx_(ctx), stream_(stream) {
     max_grid_b_ = std::max(1, occ_b) * std::max(1, ctx->sm_count);
     max_grid_c_ = std::max(1, occ_c) * std::max(1, ctx->sm_count);
     cudaFuncSetAttribute(k_team, cudaFuncAttributeMaxDynamicSharedMemorySize, kTeamSmemMax);
+    for (bool sr : {false, true})
+        cudaFuncSetAttribute(stream_kernel(sr), cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmem);
     const char *loop_env = getenv("WSB_LOOP");
     use_graph_ = !(loop_env && std::strcmp(loop_env, "launch") == 0);
     cudaMallocHost(&h_sp_, sizeof(StepParams));
@@ -202,7 +213,6 @@ Engine::Engine(Context *ctx, cudaStream_t stream) : ctx_(ctx), stream_(stream) {
 }
 
 Engine::~Engine() {
-    if (team_stream_) cudaStreamSynchronize(team_stream_);
     cudaStreamSynchronize(stream_);
     if (exec_) cudaGraphExecDestroy(exec_);
     if (graph_) cudaGraphDestroy(graph_);
@@ -221,9 +231,6 @@ Engine::~Engine() {
     cudaFreeHost(h_work_);
     cudaEventDestroy(ev0_);
     cudaEventDestroy(ev1_);
-    if (team_stream_) cudaStreamDestroy(team_stream_);
-    if (fork_ev_) cudaEventDestroy(fork_ev_);
-    if (join_ev_) cudaEventDestroy(join_ev_);
 }
 
 int Engine::ensure_capacity(uint32_t need) {
@@ -312,6 +319,26 @@ void Engine::team_plan(Slot *sl) const {
     }
 }
 
+// Whether k_stream iterates a system that k_team does not: BSR6, more block
+// rows than k_team's CTAs hold, every five consecutive ones within a product
+// stage. (It takes the device for one system at a time, which pays where one
+// system fills it: 22^3 nodes 11.5 us an iteration alone, 25 us in the loop
+// kernels, which need 9 us a system-iteration at 20^3 when eight share them.)
+// The loop kernels keep what is left: CSR, longer block rows, and small
+// systems of the single-reduction recurrence.
+void Engine::stream_plan(Slot *sl) const {
+    const MatA &A = *sl->A;
+    if (!team_on_ || !use_graph_ || sl->team || A.layout != LAYOUT_BSR6 || A.n == 0 || sl->M->nb != A.n / 6) return;
+    const uint32_t nbr = A.n / 6;
+    if (nbr <= (uint32_t)(ctx_->sm_count * kTeamWarps * kTeamWarpBrows)) return;
+    for (uint32_t br = 0; br < nbr; ++br) {
+        const uint32_t end = std::min(br + (uint32_t)kStreamBrows, nbr);
+        if (A.h_rows[br + 1] - A.h_rows[br] > (uint32_t)kStreamMaxCols || A.h_rows[end] - A.h_rows[br] > (uint32_t)kStreamMaxBlocks)
+            return;
+    }
+    sl->stream = stream_grid(nbr, (uint32_t)std::max(1, ctx_->sm_count));
+}
+
 int Engine::add(const MatA *A, const Precond *M, const SolveCfg &cfg, uint32_t *slot_out) {
     if (A->n != M->n) return fail(ctx_, WSB_ERR_BAD_INPUT, "matrix and preconditioner sizes differ (%u vs %u)", A->n, M->n);
     if (cfg.algorithm != WSB_ALG_CLASSIC && cfg.algorithm != WSB_ALG_SINGLE_REDUCTION)
@@ -353,7 +380,8 @@ int Engine::add(const MatA *A, const Precond *M, const SolveCfg &cfg, uint32_t *
     const uint64_t max_hist = cfg.max_iter > 0 ? cfg.max_iter : 1;
     sl->hist_cap = std::min<uint64_t>(cfg.hist_cap, max_hist);
     team_plan(sl.get());
-    size_t off[14], tot = 0;
+    stream_plan(sl.get());
+    size_t off[15], tot = 0;
     auto take = [&](int k, size_t bytes) {
         off[k] = tot;
         tot += a256(bytes);
@@ -371,7 +399,8 @@ int Engine::add(const MatA *A, const Precond *M, const SolveCfg &cfg, uint32_t *
     take(10, sizeof(double) * (sl->hist_cap + 1));
     take(11, cfg.algorithm == WSB_ALG_SINGLE_REDUCTION ? vf : 0);  // s
     take(12, sl->team ? sizeof(unsigned long long) * n : 0);  // z packets
-    take(13, team_red_bytes(sl->team));                       // published partials
+    take(13, team_red_bytes(sl->red_ctas()));                 // published partials
+    take(14, sl->stream && cfg.algorithm == WSB_ALG_CLASSIC ? vf : 0);  // the other buffer of p
     void *mem = nullptr;
     cudaError_t e = cudaMallocAsync(&mem, tot, stream_);
     if (e != cudaSuccess)
@@ -395,6 +424,7 @@ int Engine::add(const MatA *A, const Precond *M, const SolveCfg &cfg, uint32_t *
     sl->s = cfg.algorithm == WSB_ALG_SINGLE_REDUCTION ? (float *)(base + off[11]) : nullptr;
     sl->zpk = (unsigned long long *)(base + off[12]);
     sl->red = (RedEntry *)(base + off[13]);
+    sl->p2 = (float *)(base + off[14]);
 
     SysDesc &d = h_sys_[s];
     std::memset(&d, 0, sizeof d);
@@ -437,6 +467,9 @@ int Engine::add(const MatA *A, const Precond *M, const SolveCfg &cfg, uint32_t *
     d.algo = (uint32_t)cfg.algorithm;
     d.s = sl->s;
     d.team_warps = sl->team_warps;
+    d.path = sl->team ? PATH_TEAM : sl->stream ? PATH_STREAM : PATH_LOOP;
+    d.p2 = sl->p2;
+    d.stream_past_l2 = 148ull * A->nbsr + 144ull * M->nb > kL2Keep;
     d.zpk = sl->zpk;
     d.red = sl->red;
     std::memset(h_state_ + s, 0, sizeof(SysState));
@@ -490,7 +523,7 @@ uint32_t Engine::active_count() const {
 
 void Engine::remove(uint32_t s) {
     if (s >= slots_.size() || !slots_[s]) return;
-    if (slots_[s]->phase == Slot::RUNNING && !slots_[s]->team) work_dirty_ = true;
+    if (slots_[s]->phase == Slot::RUNNING && slots_[s]->looped()) work_dirty_ = true;
     cudaFreeAsync(slots_[s]->mem, stream_);
     slots_[s].reset();
     std::memset(h_sys_ + s, 0, sizeof(SysDesc));
@@ -604,7 +637,7 @@ int Engine::rebuild_work() {
     size_t per = 1;
     for (uint32_t s = 0; s < slots_.size(); ++s) {
         const Slot *sl = slots_[s].get();
-        if (!sl || sl->team) continue;
+        if (!sl || !sl->looped()) continue;
         per += std::max<size_t>(std::max(sl->A->n_stiles, sl->M->n_utiles), chunks_of(sl->A->n));
         if (sl->phase != Slot::RUNNING) continue;
         ga.push_back({s, sl->A->n_stiles, sl->sgroups});
@@ -623,7 +656,7 @@ int Engine::rebuild_work() {
     w_work_b_ = lb.w;
     for (uint32_t s = 0; s < slots_.size(); ++s) {
         const Slot *sl = slots_[s].get();
-        if (!sl || sl->team || sl->phase != Slot::RUNNING) continue;
+        if (!sl || !sl->looped() || sl->phase != Slot::RUNNING) continue;
         for (uint32_t t = 0; t < chunks_of(sl->A->n); ++t) wc[nch++] = {s, t};
     }
     n_work_a_ = na;
@@ -780,7 +813,7 @@ int Engine::finish_slot(uint32_t s, int status) {
 // Otherwise the systems, widest first, each take the CTAs that are free
 // soonest; a CTA works through its systems in that one order, which every CTA
 // shares, so no two systems wait for each other.
-int Engine::launch_team(const std::vector<uint32_t> &ids, uint32_t limit, cudaStream_t st) {
+int Engine::launch_team(const std::vector<uint32_t> &ids, uint32_t limit) {
     if (ids.empty()) return WSB_OK;
     const uint32_t sms = (uint32_t)std::max(1, ctx_->sm_count);
     uint64_t total = 0;
@@ -826,15 +859,30 @@ int Engine::launch_team(const std::vector<uint32_t> &ids, uint32_t limit, cudaSt
         for (const TeamItem &q : lists[c]) it[at++] = q;
     }
     h_team_[grid] = at;
-    WSB_CUDA_TRY(ctx_, cudaMemcpyAsync(d_team_, h_team_, sizeof(uint32_t) * words, cudaMemcpyHostToDevice, st));
+    WSB_CUDA_TRY(ctx_, cudaMemcpyAsync(d_team_, h_team_, sizeof(uint32_t) * words, cudaMemcpyHostToDevice, stream_));
     const SysDesc *dsys = d_sys_;
     StepParams *dsp = d_sp_;
     const TeamItem *ditems = reinterpret_cast<const TeamItem *>(d_team_ + head);
     const uint32_t *doff = d_team_;
     void *args[] = {&dsys, &dsp, &ditems, &doff, &limit};
     WSB_CUDA_TRY(ctx_, cudaLaunchCooperativeKernel((const void *)k_team, dim3(grid), dim3(kTeamThreads), args, smem,
-                                                   st));
+                                                   stream_));
     launches_ += 1;
+    return WSB_OK;
+}
+
+// k_stream takes the whole device for one system: one launch each.
+int Engine::launch_stream(const std::vector<uint32_t> &ids, uint32_t limit) {
+    for (uint32_t s : ids) {
+        const SysDesc *dsys = d_sys_;
+        StepParams *dsp = d_sp_;
+        uint32_t system = s;
+        void *args[] = {&dsys, &dsp, &system, &limit};
+        WSB_CUDA_TRY(ctx_, cudaLaunchCooperativeKernel(stream_kernel(slots_[s]->cfg.algorithm == WSB_ALG_SINGLE_REDUCTION),
+                                                       dim3(slots_[s]->stream), dim3(kStreamThreads), args,
+                                                       (size_t)kStreamSmem, stream_));
+        launches_ += 1;
+    }
     return WSB_OK;
 }
 
@@ -882,7 +930,7 @@ int Engine::step(uint32_t loop_limit, bool *any_left, uint32_t team_limit) {
         if (slots_[s] && slots_[s]->phase == Slot::NEED_INIT) init.push_back(s);
     uint32_t running = 0;  // systems of the loop kernels
     for (auto &sl : slots_)
-        if (sl && sl->phase == Slot::RUNNING && !sl->team) ++running;
+        if (sl && sl->phase == Slot::RUNNING && sl->looped()) ++running;
     // Empty systems finish at once: b.b == 0 gives Ok(0) (compute.rs:252-254).
     for (auto it = init.begin(); it != init.end();) {
         Slot &sl = *slots_[*it];
@@ -899,8 +947,8 @@ int Engine::step(uint32_t loop_limit, bool *any_left, uint32_t team_limit) {
         SysState &st = h_state_[s];
         uint32_t epoch = st.epoch;
         if (sl.red_dirty) {
-            WSB_CUDA_TRY(ctx_, cudaMemsetAsync(sl.red, 0, team_red_bytes(sl.team), stream_));
-            WSB_CUDA_TRY(ctx_, cudaMemsetAsync(sl.zpk, 0, sizeof(unsigned long long) * sl.A->n, stream_));
+            WSB_CUDA_TRY(ctx_, cudaMemsetAsync(sl.red, 0, team_red_bytes(sl.red_ctas()), stream_));
+            if (sl.team) WSB_CUDA_TRY(ctx_, cudaMemsetAsync(sl.zpk, 0, sizeof(unsigned long long) * sl.A->n, stream_));
             epoch = 0;
             sl.red_dirty = false;
         }
@@ -930,13 +978,18 @@ int Engine::step(uint32_t loop_limit, bool *any_left, uint32_t team_limit) {
     if ((rc = push_changes())) return rc;
     // k_team forms its systems' first residual itself.
     init.erase(std::remove_if(init.begin(), init.end(), [&](uint32_t s) { return slots_[s]->team != 0; }), init.end());
-    std::vector<uint32_t> team;
-    for (uint32_t s = 0; s < slots_.size(); ++s)
-        if (slots_[s] && slots_[s]->phase == Slot::RUNNING && slots_[s]->team) team.push_back(s);
-    if (!init.empty()) work_dirty_ = true;
+    std::vector<uint32_t> team, streamed;
+    for (uint32_t s = 0; s < slots_.size(); ++s) {
+        if (!slots_[s] || slots_[s]->phase != Slot::RUNNING) continue;
+        if (slots_[s]->team) team.push_back(s);
+        if (slots_[s]->stream) streamed.push_back(s);
+    }
+    uint32_t starting = 0;  // systems of the loop kernels that start
+    for (uint32_t s : init) starting += slots_[s]->looped();
+    if (starting) work_dirty_ = true;
     if (work_dirty_ && (rc = rebuild_work())) return rc;
     if ((rc = launch_init(init))) return rc;
-    num_active_ = running + (uint32_t)init.size();
+    num_active_ = running + starting;
     fill_list_ptrs();
     h_sp_->n_work_a = n_work_a_;
     h_sp_->n_work_b = n_work_b_;
@@ -949,35 +1002,18 @@ int Engine::step(uint32_t loop_limit, bool *any_left, uint32_t team_limit) {
     // system stops by its own max_iter, so the loop ends even if one did not.
     uint64_t budget = 1;
     for (auto &sl : slots_)
-        if (sl && sl->phase == Slot::RUNNING && !sl->team) {
+        if (sl && sl->phase == Slot::RUNNING && sl->looped()) {
             const uint64_t done = h_state_[&sl - &slots_[0]].iter;
             const uint64_t mx = sl->mixed ? (sl->cfg.max_iter > sl->iters_total ? sl->cfg.max_iter - sl->iters_total : 0)
                                           : sl->cfg.max_iter;
             budget = std::max<uint64_t>(budget, (mx > done ? mx - done : 0) + 1);
         }
-    // Beside a k_team launch that runs to its end, so do the loop kernels.
-    const bool fork = !team.empty() && num_active_ > 0;
-    if (fork) loop_limit = std::max(loop_limit, team_limit);
     const uint32_t limit = (uint32_t)std::min<uint64_t>(loop_limit, std::min<uint64_t>(budget, 0xffffffffu));
     h_sp_->num_active = num_active_;
     h_sp_->loop_count = 0;
     h_sp_->loop_limit = limit;
     WSB_CUDA_TRY(ctx_, cudaMemcpyAsync(d_sp_, h_sp_, sizeof(StepParams), cudaMemcpyHostToDevice, stream_));
-    // With systems of both paths, k_team runs beside the loop kernels on a
-    // stream of its own: it waits on latency most of the time and leaves half
-    // of every SM's shared memory, which one CTA of each loop kernel fits in
-    // (48 systems of side 4-24: 30.1 ms one after the other, 29.3 ms so).
-    if (fork) {
-        if (!team_stream_) {
-            WSB_CUDA_TRY(ctx_, cudaStreamCreateWithFlags(&team_stream_, cudaStreamNonBlocking));
-            WSB_CUDA_TRY(ctx_, cudaEventCreateWithFlags(&fork_ev_, cudaEventDisableTiming));
-            WSB_CUDA_TRY(ctx_, cudaEventCreateWithFlags(&join_ev_, cudaEventDisableTiming));
-        }
-        WSB_CUDA_TRY(ctx_, cudaEventRecord(fork_ev_, stream_));
-        WSB_CUDA_TRY(ctx_, cudaStreamWaitEvent(team_stream_, fork_ev_, 0));
-    }
-    if ((rc = launch_team(team, std::max<uint32_t>(1, team_limit), fork ? team_stream_ : stream_))) return rc;
-    if (fork) WSB_CUDA_TRY(ctx_, cudaEventRecord(join_ev_, team_stream_));
+    if ((rc = launch_team(team, std::max<uint32_t>(1, team_limit)))) return rc;
     if (!init.empty()) {
         const uint32_t ga = std::min<uint32_t>(h_sp_->w_init_a, (uint32_t)max_grid_a_);
         const uint32_t gb = std::min<uint32_t>(h_sp_->w_init_b, (uint32_t)max_grid_b_);
@@ -987,6 +1023,7 @@ int Engine::step(uint32_t loop_limit, bool *any_left, uint32_t team_limit) {
         if (gb) WSB_CUDA_TRY(ctx_, launch_pdl(k_init, gb, kUpdThreads, kUpdSmem, stream_, dsys, dsp));
         launches_ += (ga ? 1 : 0) + (gb ? 1 : 0);
     }
+    if ((rc = launch_stream(streamed, std::max<uint32_t>(1, team_limit)))) return rc;
     if (num_active_ > 0 && n_work_a_ > 0) {
         const uint32_t ga = std::max<uint32_t>(1, std::min<uint32_t>(w_work_a_, (uint32_t)max_grid_a_));
         const uint32_t gb = std::max<uint32_t>(1, std::min<uint32_t>(w_work_b_, (uint32_t)update_grid_max()));
@@ -1022,7 +1059,6 @@ int Engine::step(uint32_t loop_limit, bool *any_left, uint32_t team_limit) {
             h_sp_->loop_count = done_iters;
         }
     }
-    if (fork) WSB_CUDA_TRY(ctx_, cudaStreamWaitEvent(stream_, join_ev_, 0));
     if (timing) cudaEventRecord(ev1_, stream_);
     // 3) Read back states; retire or hand finished inner solves to refinement.
     std::vector<uint32_t> run_ids;
@@ -1052,7 +1088,7 @@ int Engine::step(uint32_t loop_limit, bool *any_left, uint32_t team_limit) {
         // Its device state is inactive, so the kernels skip its tiles: the
         // lists are re-laid out only once a quarter of their tiles belong to
         // systems that stopped (or when one joins), not at every retirement.
-        if (!sl.team) retired_tiles_ += (uint64_t)sl.A->n_stiles + sl.M->n_utiles;
+        if (sl.looped()) retired_tiles_ += (uint64_t)sl.A->n_stiles + sl.M->n_utiles;
         if (sl.mixed) {
             if (st.status == ST_BREAKDOWN) sl.stalled = true;
             if (st.status == ST_MAXITER && sl.iters_total >= sl.cfg.max_iter) sl.stalled = true;
@@ -1075,7 +1111,7 @@ int Engine::step(uint32_t loop_limit, bool *any_left, uint32_t team_limit) {
                                     : fail(ctx_, WSB_ERR_CUDA, "a kernel met an invalid work item (code %u)", code);
         for (uint32_t s2 = 0; s2 < slots_.size(); ++s2) {
             if (!slots_[s2]) continue;
-            if (slots_[s2]->team) slots_[s2]->red_dirty = true;
+            if (!slots_[s2]->looped()) slots_[s2]->red_dirty = true;
             if (slots_[s2]->phase == Slot::RUNNING) finish_slot(s2, rc2);
         }
         h_sp_->error = 0;

@@ -4,6 +4,7 @@
 #include <memory>
 
 #include "kernels_fused.cuh"
+#include "kernels_stream.cuh"
 #include "kernels_team.cuh"
 
 namespace wsb {
@@ -105,10 +106,11 @@ struct SolveOutcome {
 
 
 // Multi-system PCG engine. Systems are slots; each owns its Krylov vectors,
-// partial buffers and state in HBM. A slot is iterated by one of two paths,
-// chosen when it is added (team_plan): systems that fit in the shared memory
-// of a team of CTAs by one cooperative launch of k_team; the others together
-// by one captured graph: a gate kernel, then a while loop of
+// partial buffers and state in HBM. A slot is iterated by one of three paths,
+// chosen when it is added: systems that fit in the shared memory of a team of
+// CTAs by one cooperative launch of k_team (team_plan); larger BSR6 systems
+// one after the other by k_stream (stream_plan); the rest (CSR, long block
+// rows) together by one captured graph: a gate kernel, then a while loop of
 // {k_spmv, k_update, k_pupdate} that ends when no slot is active or after
 // loop_limit iterations. Between steps the host retires finished slots,
 // restarts refinement sweeps and rebuilds the work lists.
@@ -121,7 +123,7 @@ class Engine {
     int set_rhs(uint32_t slot, const float *b, const float *x0, bool device_ptrs);
     int run();                                       // all slots to completion
     // One scheduler step: at most loop_limit iterations of every system
-    // (team_limit for the systems k_team iterates).
+    // (team_limit for those that k_team and k_stream iterate).
     int step(uint32_t loop_limit, bool *any_left, uint32_t team_limit);
     int step(uint32_t loop_limit, bool *any_left) { return step(loop_limit, any_left, loop_limit); }
     // All systems added from now on go through the loop kernels (kernel timing).
@@ -160,7 +162,9 @@ class Engine {
     int read_states(const std::vector<uint32_t> &slots);
     int finish_slot(uint32_t slot, int status);
     void team_plan(Slot *sl) const;
-    int launch_team(const std::vector<uint32_t> &slots, uint32_t limit, cudaStream_t st);
+    void stream_plan(Slot *sl) const;
+    int launch_stream(const std::vector<uint32_t> &slots, uint32_t limit);
+    int launch_team(const std::vector<uint32_t> &slots, uint32_t limit);
 
     Context *ctx_;
     cudaStream_t stream_;
@@ -181,8 +185,6 @@ class Engine {
     bool use_graph_ = true;   // WSB_LOOP=launch: plain launches + host polling
     bool team_on_ = true;     // small systems take k_team
     uint32_t *d_team_ = nullptr, *h_team_ = nullptr;  // k_team lists: item offsets, then items
-    cudaStream_t team_stream_ = nullptr;              // k_team beside the loop kernels
-    cudaEvent_t fork_ev_ = nullptr, join_ev_ = nullptr;
     size_t team_cap_ = 0;                             // words of d_team_ / h_team_
     cudaGraph_t graph_ = nullptr;
     cudaGraphExec_t exec_ = nullptr;

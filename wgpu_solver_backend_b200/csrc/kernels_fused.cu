@@ -1245,7 +1245,7 @@ __device__ __forceinline__ void flush_upd(const SysDesc *__restrict__ sys, StepP
         if (status != ST_RUNNING) {
             st->status = status;
             st->active = 0;
-            atomicSub(&sp->num_active, 1u);
+            if (S.path == PATH_LOOP) atomicSub(&sp->num_active, 1u);  // the loop kernels' count
         }
     } else {
         const double rr_t = sum.x, rz_new = sum.y;

@@ -65,8 +65,9 @@ uint64_t estimate_bytes(const Request &r) {
     uint64_t v = 6 * 4 * (n + kPadElems) + 8 * (n / 16 + 64) + 16 * (n / 16 + 64) + 8 * 4096;
     if (r.cfg.precision == WSB_PREC_MIXED_F64_IR) v += 12 * (n + kPadElems);
     if (r.cfg.algorithm == WSB_ALG_SINGLE_REDUCTION) v += 4 * (n + kPadElems);
-    // k_team: z packets, published partials (for teams of one warp tile a CTA at most).
-    v += 8 * n + sizeof(RedEntry) * team_red_entries((uint32_t)std::min<uint64_t>(n / (6 * kTeamWarpBrows) + 1, 512));
+    // k_team: z packets; k_stream: the other buffer of p; published partials
+    // (for teams of one warp tile a CTA at most).
+    v += 8 * (n + kPadElems) + sizeof(RedEntry) * team_red_entries((uint32_t)std::min<uint64_t>(n / (6 * kTeamWarpBrows) + 1, 512));
     v += 8 * std::min<uint64_t>(r.cfg.hist_cap, r.cfg.max_iter + 1);
     return a + m + v;
 }

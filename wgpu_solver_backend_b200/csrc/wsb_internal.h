@@ -70,6 +70,9 @@ enum Layout : uint32_t { LAYOUT_CSR = 1, LAYOUT_BSR6 = 2 };
 // direction update p = u + beta p moves into the update kernel.
 enum Algo : uint32_t { ALGO_CLASSIC = 0, ALGO_SINGLE_REDUCTION = 1 };
 
+// Which kernels iterate a system.
+enum SysPath : uint32_t { PATH_LOOP = 0, PATH_TEAM = 1, PATH_STREAM = 2 };
+
 // Row tile of the SpMV: rows [row0, row1) (CSR) or block rows (BSR6), and
 // their nonzero (or 6x6 block) range [k0, k1). A tile holds at most
 // kCsrCap nonzeros (kBsrCapBlocks blocks) unless it is a single longer row.
@@ -138,10 +141,13 @@ struct SysDesc {
     SysState *st;
     double *history;                   // hist_cap entries or null
     uint32_t algo;                     // Algo
-    uint32_t team_warps;               // k_team: warp tiles a CTA holds (0: iterated by other kernels)
+    uint32_t team_warps;               // k_team: warp tiles a CTA holds
     float *s;                          // single reduction: s = A p (by recurrence)
     unsigned long long *zpk;           // k_team: z of each row with the tag of its all-reduce (value low, tag high)
-    RedEntry *red;                     // k_team: published partials (team_red_entries)
+    float *p2;                         // k_stream: the other buffer of p
+    uint32_t path;                     // SysPath
+    uint32_t stream_past_l2;           // k_stream: matrix and factors do not stay in the L2
+    RedEntry *red;                     // k_team, k_stream: published partials (team_red_entries)
 };
 
 // One CTA's part of one system in a k_team launch: member `rank` of the `size`
