@@ -47,8 +47,9 @@ def ring_system(nbr, offsets, seed):
 
 
 # Block rows: the fewest; 80 a CTA less one, exactly (16 warps with one product
-# tile each), plus one; several update tiles a warp, an odd count.
-@pytest.mark.parametrize("nbr", [10361, 11839, 11840, 11841, 75777])
+# tile each), plus one; the same with 100; several update tiles a warp, an odd
+# count.
+@pytest.mark.parametrize("nbr", [10361, 11839, 11840, 11841, 13321, 14799, 14800, 14801, 75777])
 def test_single_reduction(ctx, nbr):
     rp, ci, v, bs, b = ring_system(nbr, (1, 3, 170), nbr)
     n = len(rp) - 1
@@ -62,7 +63,7 @@ def test_single_reduction(ctx, nbr):
 
 # More block rows than k_team's CTAs hold (148 x 70): odd and even counts, with
 # rows that end in the middle of tiles.
-@pytest.mark.parametrize("nbr", [10361, 12346, 75777])
+@pytest.mark.parametrize("nbr", [10361, 12346, 13321, 75777])
 def test_classic_beyond_shared_memory(ctx, nbr):
     rp, ci, v, bs, b = ring_system(nbr, (1, 7, 101), nbr)
     n = len(rp) - 1
@@ -81,8 +82,9 @@ def test_paths_together_and_cut_into_steps(ctx):
     loop kernels): the bits of each solved alone."""
     small = wsb.lattice_generate(6, seed=1)
     large = ring_system(10500, (1, 7, 101), 3)
+    larger = ring_system(13500, (1, 7, 101), 3)
     long_rows = ring_system(12000, (1, 2, 3, 4, 5, 6), 4)  # 13 blocks a row: too long for k_stream
-    systems = [(small["row_ptr"], small["col_idx"], small["values"], small["block_starts"], small["b"]), large, long_rows]
+    systems = [(small["row_ptr"], small["col_idx"], small["values"], small["block_starts"], small["b"]), large, larger, long_rows]
     kw = dict(max_iter=3000, rel_tol=1e-6)
     mats = [wsb.Matrix.create(ctx, *s[:4]) for s in systems]
     alone = [m.solve(s[4], **kw) for m, s in zip(mats, systems)]
@@ -101,10 +103,11 @@ def test_paths_together_and_cut_into_steps(ctx):
             assert np.array_equal(x.view(np.uint32), alone[i][0].view(np.uint32)), i
 
 
-def test_wait_limit_and_recovery():
+@pytest.mark.parametrize("nbr", [10400, 13400])
+def test_wait_limit_and_recovery(nbr):
     c = wsb.GpuContext.create("auto", 0)
     try:
-        rp, ci, v, bs, b = ring_system(10400, (1, 7, 101), 5)
+        rp, ci, v, bs, b = ring_system(nbr, (1, 7, 101), 5)
         m = wsb.Matrix.create(c, rp, ci, v, bs)
         x_ok, r_ok = m.solve(b, max_iter=2000, rel_tol=1e-6)
         c.set_wait_limit(1)
@@ -118,8 +121,9 @@ def test_wait_limit_and_recovery():
         c.set_wait_limit(0)
 
 
-def test_zero_rhs_and_iteration_limit(ctx):
-    rp, ci, v, bs, b = ring_system(10400, (1, 7, 101), 6)
+@pytest.mark.parametrize("nbr", [10400, 13400])
+def test_zero_rhs_and_iteration_limit(ctx, nbr):
+    rp, ci, v, bs, b = ring_system(nbr, (1, 7, 101), 6)
     m = wsb.Matrix.create(ctx, rp, ci, v, bs)
     x0 = np.full(len(b), 2.0, np.float32)
     x, r = m.solve(np.zeros_like(b), x0=x0, max_iter=10, rel_tol=1e-6)

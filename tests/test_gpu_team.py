@@ -106,3 +106,25 @@ def test_zero_entries_of_the_residual(ctx):
     rp, ci, v, bs, b = block_system(200, 1, 4)
     b[12:] = 0.0
     check(ctx, rp, ci, v, bs, b)
+
+
+# Block rows: the most of a narrow cut of up to 120 CTAs; one more (the wide
+# cut, 94 CTAs); a wide cut on all 148 SMs with a ragged last warp tile.
+@pytest.mark.parametrize("nbr", [8400, 8401, 13318])
+def test_narrow_and_wide_cuts(ctx, nbr):
+    check(ctx, *block_system(nbr, 0, nbr))
+
+
+def test_wide_and_narrow_teams_in_one_launch(ctx):
+    # Narrow teams run in the wide variant here, and more teams than the device
+    # holds wait for idle CTAs: the same bits as alone.
+    systems = [block_system(nbr, 1, nbr) for nbr in (8401, 3000, 1, 71, 6000, 8500, 500, 69, 2000, 281)]
+    mats = [wsb.Matrix.create(ctx, rp, ci, v, bs, layout=wsb.LAYOUT_BSR6) for rp, ci, v, bs, _ in systems]
+    batch = wsb.Batch(ctx)
+    ids = [batch.add(m, s[4], max_iter=4000, rel_tol=1e-6) for m, s in zip(mats, systems)]
+    batch.solve()
+    for i, m, s in zip(ids, mats, systems):
+        x, r = m.solve(s[4], max_iter=4000, rel_tol=1e-6)
+        xb, rb = batch.result(i, m.n)
+        assert rb["iterations"] == r["iterations"]
+        assert np.array_equal(xb.view(np.uint32), x.view(np.uint32))

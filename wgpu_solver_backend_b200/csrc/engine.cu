@@ -1,6 +1,7 @@
 // Multi-system PCG engine: device-resident systems iterated together by the
 // fused kernels inside one CUDA graph whose while loop runs on the device.
 #include <algorithm>
+#include <map>
 #include <chrono>
 #include <cmath>
 #include <cstdlib>
@@ -160,9 +161,9 @@ struct Engine::Slot {
     bool stalled = false;
     uint64_t iters_total = 0;
     SolveOutcome out;
-    // k_team (team > 0): CTAs of the system's team, warp tiles a CTA holds and
-    // its shared memory, published partials, z packets.
-    uint32_t team = 0, team_warps = 0, team_smem = 0;
+    // k_team (team > 0): CTAs of the system's team, warp tiles and most blocks a
+    // CTA holds, most bytes of its tiles, published partials, z packets.
+    uint32_t team = 0, team_warps = 0, team_ext = 0, team_tiles = 0;
     // k_stream (stream > 0): CTAs; its second buffer of p and partials.
     uint32_t stream = 0;
     float *p2 = nullptr;
@@ -199,7 +200,8 @@ Engine::Engine(Context *ctx, cudaStream_t stream) : ctx_(ctx), stream_(stream) {
     max_grid_a_ = std::max(1, occ_a) * std::max(1, ctx->sm_count);
     max_grid_b_ = std::max(1, occ_b) * std::max(1, ctx->sm_count);
     max_grid_c_ = std::max(1, occ_c) * std::max(1, ctx->sm_count);
-    cudaFuncSetAttribute(k_team, cudaFuncAttributeMaxDynamicSharedMemorySize, kTeamSmemMax);
+    for (int w : {kTeamWarps, kTeamWarpsWide})
+        cudaFuncSetAttribute(team_kernel(w), cudaFuncAttributeMaxDynamicSharedMemorySize, kTeamSmemMax);
     for (bool sr : {false, true})
         cudaFuncSetAttribute(stream_kernel(sr), cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmem);
     const char *loop_env = getenv("WSB_LOOP");
@@ -295,42 +297,49 @@ void Engine::team_plan(Slot *sl) const {
     if (!team_on_ || !use_graph_ || A.layout != LAYOUT_BSR6 || A.n == 0 || sl->M->nb != A.n / 6 ||
         sl->cfg.algorithm != WSB_ALG_CLASSIC)
         return;
-    const uint32_t nbr = A.n / 6, tiles = (nbr + kTeamWarpBrows - 1) / kTeamWarpBrows;
-    if (tiles > (uint32_t)ctx_->sm_count * kTeamWarps) return;
+    const uint32_t nbr = A.n / 6, tiles = (nbr + kTeamWarpBrows - 1) / kTeamWarpBrows, sms = (uint32_t)ctx_->sm_count;
+    if (tiles > sms * kTeamWarpsWide) return;
     std::vector<uint32_t> cols(tiles, 0u);  // blocks of each warp tile's longest block row
     for (uint32_t br = 0; br < nbr; ++br)
         cols[br / kTeamWarpBrows] = std::max(cols[br / kTeamWarpBrows], A.h_rows[br + 1] - A.h_rows[br]);
     // The most warp tiles a CTA that fit whichever CTA it is.
-    for (uint32_t w = kTeamWarps; w >= 1; --w) {
+    for (uint32_t w = tiles <= kTeamNarrowCtas * kTeamWarps ? kTeamWarps : kTeamWarpsWide; w >= 1; --w) {
         const uint32_t size = (tiles + w - 1) / w;
-        if (size > (uint32_t)ctx_->sm_count) return;
+        if (size > sms) return;
         uint64_t most = 0;
+        uint32_t blocks = 0;
         for (uint32_t c = 0; c < size; ++c) {
             uint64_t sum = 0;
-            for (uint32_t q = c * w; q < std::min((c + 1) * w, tiles); ++q) sum += team_tile_bytes(cols[q]);
+            const uint32_t end = std::min((c + 1) * w, tiles);
+            for (uint32_t q = c * w; q < end; ++q) sum += team_tile_bytes(cols[q]);
             most = std::max(most, sum);
+            blocks = std::max(blocks, A.h_rows[std::min(end * kTeamWarpBrows, nbr)] - A.h_rows[c * w * kTeamWarpBrows]);
         }
-        const uint64_t smem = kTeamFixedSmem + (uint64_t)w * kTeamLuBytes + most;
+        const uint32_t ext = size > 1 ? blocks : 0u;
+        // A narrow team may run in the wide variant, beside wide ones.
+        const uint64_t smem = team_fixed_bytes(kTeamWarpsWide) + team_z_bytes(kTeamWarpsWide, ext) + most;
         if (smem > (uint64_t)kTeamSmemMax) continue;
         sl->team = size;
         sl->team_warps = w;
-        sl->team_smem = (uint32_t)smem;
+        sl->team_ext = ext;
+        sl->team_tiles = (uint32_t)most;
         return;
     }
 }
 
 // Whether k_stream iterates a system that k_team does not: BSR6, more block
-// rows than k_team's CTAs hold, every five consecutive ones within a product
-// stage. (It takes the device for one system at a time, which pays where one
-// system fills it: 22^3 nodes 11.5 us an iteration alone, 25 us in the loop
-// kernels, which need 9 us a system-iteration at 20^3 when eight share them.)
+// rows than k_team's narrow CTAs hold, every five consecutive ones within a
+// product stage. (It takes the device for one system at a time, which pays
+// where one system fills it: 22^3 nodes 11.5 us an iteration alone, 25 us in
+// the loop kernels, which need 9 us a system-iteration at 20^3 when eight share
+// them.)
 // The loop kernels keep what is left: CSR, longer block rows, and small
 // systems of the single-reduction recurrence.
 void Engine::stream_plan(Slot *sl) const {
     const MatA &A = *sl->A;
     if (!team_on_ || !use_graph_ || sl->team || A.layout != LAYOUT_BSR6 || A.n == 0 || sl->M->nb != A.n / 6) return;
     const uint32_t nbr = A.n / 6;
-    if (nbr <= (uint32_t)(ctx_->sm_count * kTeamWarps * kTeamWarpBrows)) return;
+    if (nbr <= (uint32_t)ctx_->sm_count * kTeamWarps * kTeamWarpBrows) return;
     for (uint32_t br = 0; br < nbr; ++br) {
         const uint32_t end = std::min(br + (uint32_t)kStreamBrows, nbr);
         if (A.h_rows[br + 1] - A.h_rows[br] > (uint32_t)kStreamMaxCols || A.h_rows[end] - A.h_rows[br] > (uint32_t)kStreamMaxBlocks)
@@ -467,6 +476,7 @@ int Engine::add(const MatA *A, const Precond *M, const SolveCfg &cfg, uint32_t *
     d.algo = (uint32_t)cfg.algorithm;
     d.s = sl->s;
     d.team_warps = sl->team_warps;
+    d.team_ext = sl->team_ext;
     d.path = sl->team ? PATH_TEAM : sl->stream ? PATH_STREAM : PATH_LOOP;
     d.p2 = sl->p2;
     d.stream_past_l2 = 148ull * A->nbsr + 144ull * M->nb > kL2Keep;
@@ -810,33 +820,49 @@ int Engine::finish_slot(uint32_t s, int status) {
 
 // One cooperative launch of k_team over the given systems, one CTA per SM.
 // When the device holds all their teams at once, each CTA has one system.
-// Otherwise the systems, widest first, each take the CTAs that are free
-// soonest; a CTA works through its systems in that one order, which every CTA
-// shares, so no two systems wait for each other.
+// Otherwise the lists follow a simulated run in which, whenever CTAs fall idle,
+// the widest system that fits starts (a system that ends leaves room for any
+// that could not start before it, so wide ones do not starve). A solve takes
+// about the fourth root of its rows in iterations, each of about 4.2 us plus
+// 26 ns a CTA. Every CTA's list is in the order in which systems start, so no
+// two systems wait for each other whatever the times turn out to be.
 int Engine::launch_team(const std::vector<uint32_t> &ids, uint32_t limit) {
     if (ids.empty()) return WSB_OK;
     const uint32_t sms = (uint32_t)std::max(1, ctx_->sm_count);
     uint64_t total = 0;
-    uint32_t smem = 0;
+    int warps = kTeamWarps;
     for (uint32_t s : ids) {
         total += slots_[s]->team;
-        smem = std::max(smem, slots_[s]->team_smem);
+        if (slots_[s]->team_warps > (uint32_t)kTeamWarps) warps = kTeamWarpsWide;
     }
-    std::vector<uint32_t> order(ids);
-    std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return slots_[a]->team > slots_[b]->team; });
+    uint32_t smem = 0;
+    for (uint32_t s : ids)
+        smem = std::max(smem, (uint32_t)team_fixed_bytes(warps) + team_z_bytes(warps, slots_[s]->team_ext) + slots_[s]->team_tiles);
+    std::map<uint32_t, std::vector<uint32_t>> waiting;  // by team size, the first to start last
+    for (auto it = ids.rbegin(); it != ids.rend(); ++it) waiting[slots_[*it]->team].push_back(*it);
     const uint32_t grid = (uint32_t)std::min<uint64_t>(total, sms);
     std::vector<std::vector<TeamItem>> lists(grid);
-    std::vector<std::pair<double, uint32_t>> free_at(grid);
-    for (uint32_t c = 0; c < grid; ++c) free_at[c] = {0.0, c};
-    for (uint32_t s : order) {
-        const Slot &sl = *slots_[s];
-        std::sort(free_at.begin(), free_at.end());
-        // A solve's iterations grow about as the fourth root of its rows.
-        const double end = free_at[sl.team - 1].first + std::pow((double)sl.A->n, 0.25);
-        for (uint32_t k = 0; k < sl.team; ++k) {
-            lists[free_at[k].second].push_back({s, k, sl.team, 0u});
-            free_at[k].first = end;
+    std::vector<uint32_t> idle(grid);
+    for (uint32_t c = 0; c < grid; ++c) idle[c] = grid - 1 - c;
+    std::multimap<double, std::vector<uint32_t>> running;  // CTAs of a system by when it ends
+    double now = 0.0;
+    while (!waiting.empty()) {
+        auto fits = waiting.upper_bound((uint32_t)idle.size());
+        if (fits == waiting.begin()) {
+            now = running.begin()->first;
+            idle.insert(idle.end(), running.begin()->second.rbegin(), running.begin()->second.rend());
+            running.erase(running.begin());
+            continue;
         }
+        --fits;
+        const uint32_t s = fits->second.back(), team = fits->first;
+        fits->second.pop_back();
+        if (fits->second.empty()) waiting.erase(fits);
+        const Slot &sl = *slots_[s];
+        std::vector<uint32_t> ctas(idle.rbegin(), idle.rbegin() + team);
+        idle.resize(idle.size() - team);
+        for (uint32_t k = 0; k < team; ++k) lists[ctas[k]].push_back({s, k, team, 0u});
+        running.emplace(now + std::pow((double)sl.A->n, 0.25) * (160.0 + team), std::move(ctas));
     }
     size_t items = 0;
     for (const auto &l : lists) items += l.size();
@@ -865,8 +891,8 @@ int Engine::launch_team(const std::vector<uint32_t> &ids, uint32_t limit) {
     const TeamItem *ditems = reinterpret_cast<const TeamItem *>(d_team_ + head);
     const uint32_t *doff = d_team_;
     void *args[] = {&dsys, &dsp, &ditems, &doff, &limit};
-    WSB_CUDA_TRY(ctx_, cudaLaunchCooperativeKernel((const void *)k_team, dim3(grid), dim3(kTeamThreads), args, smem,
-                                                   stream_));
+    WSB_CUDA_TRY(ctx_, cudaLaunchCooperativeKernel(team_kernel(warps), dim3(grid), dim3(team_threads(warps)), args,
+                                                   (size_t)smem, stream_));
     launches_ += 1;
     return WSB_OK;
 }

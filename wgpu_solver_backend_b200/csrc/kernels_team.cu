@@ -5,9 +5,10 @@
 // dependent launches, each with its ramp, its chain of work-item loads and its
 // last-CTA sum. Here an iteration is two exchanges between resident CTAs and
 // the latency of one row sum and one block solve:
-//   - a lane owns a row: x, r, z, p and its row of the block's LU factors stay
-//     in registers; the matrix (and p at every block's columns) stays in
-//     shared memory, so an iteration reads only other CTAs' z from the L2;
+//   - a lane owns a row: x, r, z and p stay in registers; the matrix, p at
+//     every block's columns and the blocks' LU factors stay in shared memory,
+//     so an iteration reads only other CTAs' z from the L2, each block of it
+//     once a CTA (all row warps fetch, then all read it from shared memory);
 //   - p.Ap and then r.r and r.z are all-reduced: every CTA stores its FP64
 //     partial as one 16-byte {value, tag} and reads the whole team's in the
 //     same fixed order, so all CTAs hold the same scalars and take the same
@@ -17,13 +18,14 @@
 //     next product. Every CTA forms p = z + beta p for the block columns it
 //     multiplies (same operation, same bits as the owner's), so p is never
 //     exchanged.
-// Measured (B200, us an iteration, loop kernels -> here): 4^3 nodes 24.4 -> 3.1,
-// 9^3 23.5 -> 4.7, 12^3 24.8 -> 5.2, 17^3 25.7 -> 6.1, 20^3 27.2 -> 7.5.
+// Measured (B200, us an iteration, loop kernels -> here): 4^3 nodes 24.4 -> 2.9,
+// 9^3 23.5 -> 4.5, 12^3 24.8 -> 5.0, 17^3 25.7 -> 5.9, 20^3 27.2 -> 7.2,
+// 23^3 28 -> 8.7. 48 systems of 4^3 to 24^3 nodes at once: 27.6 ms -> 22.0.
 // What is left is latency (7 of 13 warps wait at a barrier at any time, issue
 // slots 28 % used): per iteration two hops through the L2 (800 cycles for
 // 8 CTAs, 1,400 for 31), the FP64 sums (nine cycles an add, 36 with the shuffle
 // between lanes), two FP64 divisions and the block solve. So products are
-// added through shared memory, 16 per lane as a tree, before the lanes; a block
+// added through shared memory, 14 or 18 per lane, before the lanes; a block
 // is solved by one lane from shared memory (no shuffles between its steps); and
 // all waits are warp-uniform loops: lanes that leave such a loop one by one
 // stay apart and made the code after it up to ten times slower.
@@ -43,45 +45,57 @@ namespace {
 
 // The fixed part of a CTA's shared memory.
 struct TeamShared {
-    double v[2][kTeamThreads];  // the rows' products of a reduction (the reducing warps': zero)
-    float z[kTeamThreads];      // the CTA's rows of r, then of z
     double rz, beta;            // the last r.z and beta
     uint2 alpha;                // alpha; 0: the system stops here
     float beta_f;
     uint32_t go;                // 0: the system stops here
     uint32_t err;               // a wait ran out
+    uint32_t ext;               // blocks outside the CTA's rows
     // Scalars of the recurrence, kept by one thread (the same in every CTA).
     double bb, rz_old, pap, alpha_d, rr, rel2, abs2;
     uint32_t iter, max_iter, status, breakdown;
-    uint32_t bytes[kTeamWarps];  // shared memory of each warp tile
+    uint32_t bytes[kTeamWarpsWide];  // shared memory of each warp tile
+    alignas(16) double v[1];     // the rows' products of a reduction, twice 32 a warp tile
 };
-static_assert(sizeof(TeamShared) <= kTeamFixedSmem && kTeamFixedSmem % 128 == 0, "fixed shared memory");
 
 struct WaitCtl {
     StepParams *sp;
     long long lim;
 };
 
-// Sum of one value per thread of the CTA, by one warp: lane l adds 16 of them
-// as a tree, then the lanes; valid in lane 0.
+// Sum of one value per row of the CTA, by one warp: lane l adds a pair per two
+// warp tiles, those of the first kTeamWarps as a tree, then (wide) the others,
+// then the lanes; valid in lane 0. Warp tiles that a narrow CTA does not have
+// are zeros in a wide one: the same sum.
+template <int kWarps>
 __device__ __forceinline__ double cta_sum(const double *v, uint32_t lane) {
-    constexpr int kHalf = kTeamThreads / 64;
-    double s[kHalf];
+    constexpr int kPairs = kTeamWarps / 2;
+    const double2 *v2 = reinterpret_cast<const double2 *>(v) + lane;
+    double s[kPairs];
 #pragma unroll
-    for (int k = 0; k < kHalf; ++k) {
-        const double2 a = reinterpret_cast<const double2 *>(v)[32 * k + lane];
+    for (int k = 0; k < kPairs; ++k) {
+        const double2 a = v2[32 * k];
         s[k] = a.x + a.y;
     }
 #pragma unroll
-    for (int h = kHalf / 2; h > 0; h >>= 1)
+    for (int n = kPairs; n > 1; n = (n + 1) / 2)
 #pragma unroll
-        for (int k = 0; k < h; ++k) s[k] += s[k + h];
+        for (int k = 0; k < n / 2; ++k) s[k] += s[k + (n + 1) / 2];
+    if (kWarps > kTeamWarps) {
+        double t = 0.0;
+#pragma unroll
+        for (int k = kPairs; k < kWarps / 2; ++k) {
+            const double2 a = v2[32 * k];
+            t += a.x + a.y;
+        }
+        s[0] += t;
+    }
     return warp_sum(s[0]);
 }
-
-constexpr uint32_t kLocal = 0x80000000u;  // a block column inside the CTA's rows
+static_assert(kTeamWarps % 2 == 0 && kTeamWarpsWide % 2 == 0, "cta_sum");
 
 // One system, this CTA's rows, up to `limit` iterations.
+template <int kWarps>
 __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamItem it, uint32_t limit, TeamShared &S,
                                                  char *dyn, const WaitCtl &w) {
     constexpr int kAhead = 8;  // block columns a lane handles at once
@@ -110,25 +124,32 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
         }
     }
     const uint32_t cols = __reduce_max_sync(kFull, nk);  // of the warp tile
-    if (lane == 0 && warp < (uint32_t)kTeamWarps) S.bytes[warp] = team_tile_bytes(cols);
-    S.v[0][tid] = S.v[1][tid] = 0.0;
+    if (lane == 0 && warp < (uint32_t)kWarps) S.bytes[warp] = team_tile_bytes(cols);
+    double *const v0 = S.v, *const v1 = S.v + 32 * kWarps;
+    if (warp < (uint32_t)kWarps) v0[tid] = v1[tid] = 0.0;
+    if (tid == 0) S.ext = 0;
     __syncthreads();
-    // Dynamic shared memory: LU factors of the CTA's block rows; then for each
-    // warp tile and block j of its block rows, lane by lane (no bank
+    // Dynamic shared memory: z of the CTA's rows (first r, then z, 32 a warp
+    // tile) and of the blocks outside, and those blocks' first rows; then for
+    // each warp tile its LU factors, 1 / diagonal and the range test of the
+    // short division, and for block j of its block rows, lane by lane (no bank
     // conflicts), the row's first four values, its last two, p at the block's
-    // columns, and the first row of the block's columns (in the system, or
-    // with kLocal in S.z).
-    float *lu = reinterpret_cast<float *>(dyn) + (size_t)warp * (kTeamLuBytes / 4);
+    // columns, and where z of the block's columns is.
+    float *const zx = reinterpret_cast<float *>(dyn);
+    uint32_t *const ext = reinterpret_cast<uint32_t *>(zx + 32 * kWarps + 6u * D.team_ext);
     uint32_t before = 0;
     for (uint32_t q = 0; q < min(warp, tw); ++q) before += S.bytes[q];
-    char *mine = dyn + (size_t)tw * kTeamLuBytes + before;
+    char *mine = dyn + team_z_bytes(kWarps, D.team_ext) + before;
     // (cols == 0: a warp without rows; it touches none of this.)
+    float *const lu = reinterpret_cast<float *>(mine);
+    float *const rd = lu + 36 * kTeamWarpBrows;
+    mine += kTeamLuBytes;
     const uint32_t colp = (cols + 7u) & ~7u;
     float4 *b4 = reinterpret_cast<float4 *>(mine) + lane;
     float2 *b2 = reinterpret_cast<float2 *>(mine + (size_t)cols * 16u * kTeamWarpRows) + lane;
     float *xg = reinterpret_cast<float *>(mine + (size_t)cols * 24u * kTeamWarpRows) + 8u * bo;
     uint32_t *bc = reinterpret_cast<uint32_t *>(mine + (size_t)cols * kTeamColBytes);
-    for (uint32_t j = lane; j < colp * (uint32_t)(kTeamWarpBrows + 1); j += 32u) bc[j] = kLocal;  // past a row's end
+    for (uint32_t j = lane; j < colp * (uint32_t)(kTeamWarpBrows + 1); j += 32u) bc[j] = 0;  // past a row's end
     bc += colp * bo;
     __syncwarp();
     if (on) {
@@ -143,10 +164,15 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
             cp_async8(b2 + j * kTeamWarpRows, v + 4);
             const uint32_t c = D.bcol[k0 + j];
             cp_async4(xg + 8u * kTeamWarpBrows * j + a, src + 6u * (size_t)c);
-            if (a == 0)
-                bc[j] =
-                    c >= br0 && c < br1 ? kLocal | (32u * ((c - br0) / kTeamWarpBrows) + 6u * ((c - br0) % kTeamWarpBrows))
-                                        : 6u * c;
+            if (a == 0) {
+                if (c >= br0 && c < br1) {
+                    bc[j] = 32u * ((c - br0) / kTeamWarpBrows) + 6u * ((c - br0) % kTeamWarpBrows);
+                } else {
+                    const uint32_t e = atomicAdd(&S.ext, 1u);  // (the order changes no value)
+                    bc[j] = 32u * kWarps + 6u * e;
+                    ext[e] = 6u * c;
+                }
+            }
         }
         // The lane's row of the LU factors; lane a == 0 solves the block.
 #pragma unroll
@@ -156,15 +182,20 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
     __syncwarp();
     const uint32_t sbo = min(lane, (uint32_t)kTeamWarpBrows - 1u);  // the block row that this lane solves
     const bool solver = lane < (uint32_t)kTeamWarpBrows && warp < tw && br0 + warp * (uint32_t)kTeamWarpBrows + lane < br1;
-    const float *slu = lu + 36u * sbo;
-    float rdiag[6], dlo = kDivLo;
+    const float *const slu = lu + 36u * sbo;
+    float *const srd = rd + 8u * sbo;
+    if (solver) {
+        float dlo = kDivLo;
 #pragma unroll
-    for (int i = 0; i < 6; ++i) {
-        const float u = solver ? slu[7 * i] : 1.0f, au = fabsf(u);
-        rdiag[i] = __frcp_rn(u);
-        if (!(au >= kDivULo && au <= kDivUHi)) dlo = __int_as_float(0x7f800000);
+        for (int i = 0; i < 6; ++i) {
+            const float u = slu[7 * i], au = fabsf(u);
+            srd[i] = __frcp_rn(u);
+            if (!(au >= kDivULo && au <= kDivUHi)) dlo = __int_as_float(0x7f800000);
+        }
+        srd[6] = dlo;
     }
     __syncthreads();
+    const uint32_t n_ext = 6u * S.ext;
 
     // y = (row) . xg: products rounded, added in index order; the operands of
     // the next block are loaded before this block's products are added.
@@ -196,7 +227,7 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
     };
     // z = U^-1 L^-1 r of the warp tile's blocks, one lane a block, in the
     // order of block_jacobi.wgsl:93-126; r comes and z goes through S.z.
-    float *const wz = S.z + 32u * warp;
+    float *const wz = zx + 32u * min(warp, (uint32_t)kWarps - 1u);
     auto block_solve = [&]() {
         wz[lane] = r;
         __syncwarp();
@@ -215,6 +246,8 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
                 const float2 v = reinterpret_cast<const float2 *>(rz)[i];
                 y[2 * i] = v.x, y[2 * i + 1] = v.y;
             }
+            const float4 d0 = reinterpret_cast<const float4 *>(srd)[0], d1 = reinterpret_cast<const float4 *>(srd)[1];
+            const float rdiag[6] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y}, dlo = d1.z;
 #pragma unroll
             for (int i = 1; i < 6; ++i)
 #pragma unroll
@@ -247,7 +280,7 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
     unsigned long long *const zpk = D.zpk;
     // The last two warps have no rows: they reduce. The first of them sums
     // p.Ap and r.r and decides, the second sums r.z and forms beta.
-    const bool red_a = warp == (uint32_t)kTeamWarps, red_b = warp == (uint32_t)kTeamWarps + 1u;
+    const bool red_a = warp == (uint32_t)kWarps, red_b = warp == (uint32_t)kWarps + 1u;
     if (red_a && lane == 0) {
         S.bb = st->bb;
         S.rr = S.pap = S.alpha_d = S.beta = 0.0;
@@ -261,72 +294,59 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
         S.breakdown = 0;
     }
 
-    // The z packets of the row's block columns outside the CTA, one component
-    // a lane: requested, and waited for while the scalars are reduced.
-    auto block_cols = [&](uint32_t j0, uint32_t c[kAhead]) {
-#pragma unroll
-        for (int q = 0; q < kAhead / 4; ++q) {
-            const uint4 v = reinterpret_cast<const uint4 *>(bc + j0)[q];
-            c[4 * q] = v.x, c[4 * q + 1] = v.y, c[4 * q + 2] = v.z, c[4 * q + 3] = v.w;
-        }
-    };
-    unsigned long long zin[kAhead];
-    auto fetch_z = [&](uint32_t j0) {
-        const long long t0 = clock64();
+    // The z packets of the blocks outside the CTA, by its warps with rows, into
+    // shared memory, while the scalars are reduced.
+    auto fetch_z = [&]() {
+        constexpr uint32_t kBatch = 4;
+        const uint32_t step = 32u * tw;
 #pragma unroll 1
-        for (uint32_t k = 1;; ++k) {
-            uint32_t bad = 0;
-            uint32_t c[kAhead];
-            block_cols(j0, c);
+        for (uint32_t b = 0; b < n_ext; b += kBatch * step) {
+            unsigned long long zin[kBatch];
+            const long long t0 = clock64();
+#pragma unroll 1
+            for (uint32_t k = 1;; ++k) {
+                uint32_t bad = 0;
 #pragma unroll
-            for (int j = 0; j < kAhead; ++j)
-                zin[j] = ld_packet_if(zpk + c[j] + a, !(c[j] & kLocal), (unsigned long long)tag << 32);
+                for (uint32_t q = 0; q < kBatch; ++q) {
+                    const uint32_t i = b + q * step + tid, e = i / 6u;
+                    const bool want = i < n_ext;
+                    zin[q] = ld_packet_if(zpk + (want ? ext[e] + (i - 6u * e) : 0u), want, (unsigned long long)tag << 32);
+                }
 #pragma unroll
-            for (int j = 0; j < kAhead; ++j) bad |= (uint32_t)(zin[j] >> 32) ^ tag;
-            if (__all_sync(kFull, bad == 0)) break;
-            if (__any_sync(kFull, clock64() - t0 > w.lim) || ((k & 255u) == 0 && __any_sync(kFull, ld_error(w.sp) != 0))) {
-                S.err = 1;
-                break;
+                for (uint32_t q = 0; q < kBatch; ++q) bad |= (uint32_t)(zin[q] >> 32) ^ tag;
+                if (__all_sync(kFull, bad == 0)) break;
+                if (__any_sync(kFull, clock64() - t0 > w.lim) ||
+                    ((k & 255u) == 0 && __any_sync(kFull, ld_error(w.sp) != 0))) {
+                    S.err = 1;
+                    break;
+                }
+            }
+#pragma unroll
+            for (uint32_t q = 0; q < kBatch; ++q) {
+                const uint32_t i = b + q * step + tid;
+                if (i < n_ext) zx[32 * kWarps + i] = __uint_as_float((uint32_t)zin[q]);
             }
         }
     };
     // p = z + beta p of the lane's row and of its block columns (p = z when
-    // first); p at the first kAhead columns also stays in registers. All
-    // operands come before the first store, which the compiler could not move
-    // a load across.
-    float po[kAhead];
-#pragma unroll
-    for (int j = 0; j < kAhead; ++j) po[j] = (uint32_t)j < nk ? xg[8u * kTeamWarpBrows * j + a] : 0.0f;
+    // first). All operands come before the first store, which the compiler
+    // could not move a load across.
     auto advance = [&](bool first, float bf) {
         p = first ? z : __fadd_rn(__fmul_rn(p, bf), z);
 #pragma unroll 1
         for (uint32_t j0 = 0; j0 < cols; j0 += kAhead) {
-            if (j0) fetch_z(j0);
             float *dst = xg + 8u * kTeamWarpBrows * j0 + a;
-            uint32_t c[kAhead];
-            float pn[kAhead];
-            block_cols(j0, c);
-            if (j0) {
+            float pn[kAhead], zn[kAhead];
 #pragma unroll
-                for (int j = 0; j < kAhead; ++j) pn[j] = j0 + j < nk ? dst[8u * kTeamWarpBrows * j] : 0.0f;
-            } else {
-#pragma unroll
-                for (int j = 0; j < kAhead; ++j) pn[j] = po[j];
+            for (int q = 0; q < kAhead / 4; ++q) {
+                const uint4 c = reinterpret_cast<const uint4 *>(bc + j0)[q];
+                zn[4 * q] = zx[c.x + a], zn[4 * q + 1] = zx[c.y + a], zn[4 * q + 2] = zx[c.z + a], zn[4 * q + 3] = zx[c.w + a];
             }
 #pragma unroll
-            for (int j = 0; j < kAhead; ++j) {
-                const bool local = (c[j] & kLocal) != 0;
-                const float zl = S.z[local ? (c[j] & ~kLocal) + a : 0u];
-                const float zj = local ? zl : __uint_as_float((uint32_t)zin[j]);
-                pn[j] = first ? zj : __fadd_rn(__fmul_rn(pn[j], bf), zj);
-            }
-            if (j0 == 0) {
-#pragma unroll
-                for (int j = 0; j < kAhead; ++j) po[j] = pn[j];
-            }
+            for (int j = 0; j < kAhead; ++j) pn[j] = j0 + j < nk ? dst[8u * kTeamWarpBrows * j] : 0.0f;
 #pragma unroll
             for (int j = 0; j < kAhead; ++j)
-                if (j0 + j < nk) dst[8u * kTeamWarpBrows * j] = pn[j];
+                if (j0 + j < nk) dst[8u * kTeamWarpBrows * j] = first ? zn[j] : __fadd_rn(__fmul_rn(pn[j], bf), zn[j]);
         }
         __syncwarp();
     };
@@ -347,13 +367,13 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
         if (init) {
             const float bi = on ? __ldg(D.b + row) : 0.0f;
             r = __fsub_rn(bi, ap);
-            S.v[0][tid] = (double)bi * (double)bi;
+            if (!red_a && !red_b) v0[tid] = (double)bi * (double)bi;
         } else {
-            S.v[0][tid] = (double)p * (double)ap;
+            if (!red_a && !red_b) v0[tid] = (double)p * (double)ap;
             __syncthreads();
             if (red_a) {
                 const double rz_old = S.rz;
-                double pap = cta_sum(S.v[0], lane);
+                double pap = cta_sum<kWarps>(v0, lane);
                 if (!alone) {
                     pap = __shfl_sync(kFull, pap, 0);
                     if (lane < copies) st_entry(out, pap, tag);
@@ -379,14 +399,14 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
         if (!red_a && !red_b) {
             z = block_solve();
             if (on && !alone) st_packet(zpk + row, z, tag);
-            if (!init) S.v[0][tid] = (double)r * (double)r;
-            S.v[1][tid] = (double)r * (double)z;
+            if (!init) v0[tid] = (double)r * (double)r;
+            v1[tid] = (double)r * (double)z;
         }
         __syncthreads();
         if (red_a || red_b) {
-            const double *v = red_a ? S.v[0] : S.v[1];
+            const double *v = red_a ? v0 : v1;
             const uint32_t slot = (red_a ? 1u : 2u) * it.size;
-            double sum = cta_sum(v, lane);
+            double sum = cta_sum<kWarps>(v, lane);
             if (!alone) {
                 sum = __shfl_sync(kFull, sum, 0);
                 if (lane < copies) st_entry(out + slot, sum, tag);
@@ -424,8 +444,8 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
                 S.status = status;
                 S.go = status == ST_RUNNING && !S.err;
             }
-        } else if (!alone && cols) {
-            fetch_z(0);
+        } else if (warp < tw) {
+            fetch_z();
         }
         __syncthreads();
         if (!S.go) break;
@@ -464,11 +484,11 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
     }
 }
 
-}  // namespace
-
-__global__ void __launch_bounds__(kTeamThreads, 1)
+template <int kWarps>
+__global__ void __launch_bounds__(team_threads(kWarps), 1)
     k_team(const SysDesc *__restrict__ sys, StepParams *sp, const TeamItem *__restrict__ items,
            const uint32_t *__restrict__ item_off, uint32_t limit) {
+    static_assert(offsetof(TeamShared, v) <= 512, "fixed shared memory");
     extern __shared__ __align__(128) char smem[];
     TeamShared &S = *reinterpret_cast<TeamShared *>(smem);
     const unsigned long long wl = sp->wait_cycles;
@@ -478,10 +498,16 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
     const uint32_t i1 = item_off[blockIdx.x + 1];
     for (uint32_t i = item_off[blockIdx.x]; i < i1; ++i) {
         const TeamItem it = items[i];
-        team_system_bsr6(sys[it.sys], it, limit, S, smem + kTeamFixedSmem, w);
+        team_system_bsr6<kWarps>(sys[it.sys], it, limit, S, smem + team_fixed_bytes(kWarps), w);
         __syncthreads();
         if (S.err) return;  // every CTA's later waits would run out as well
     }
+}
+
+}  // namespace
+
+const void *team_kernel(int warps) {
+    return warps <= kTeamWarps ? (const void *)k_team<kTeamWarps> : (const void *)k_team<kTeamWarpsWide>;
 }
 
 }  // namespace wsb

@@ -142,6 +142,7 @@ struct SysDesc {
     double *history;                   // hist_cap entries or null
     uint32_t algo;                     // Algo
     uint32_t team_warps;               // k_team: warp tiles a CTA holds
+    uint32_t team_ext;                 // k_team: most blocks a CTA holds
     float *s;                          // single reduction: s = A p (by recurrence)
     unsigned long long *zpk;           // k_team: z of each row with the tag of its all-reduce (value low, tag high)
     float *p2;                         // k_stream: the other buffer of p
