@@ -21,12 +21,14 @@
 // Arithmetic is that of kernels_fused.cu operation by operation; only the
 // grouping of the FP64 sums differs (per lane over its tiles, warp, CTA, device).
 //
-// Measured (B200, us an iteration, loop kernels -> here): 22^3 nodes 25.4 ->
-// 11.6, 32^3 31.8 -> 15.4, 40^3 41.5 -> 21.9 (single reduction 39.2 -> 22.7),
-// 64^3 87.0 -> 65.4, 80^3 145.9 -> 123.0. At 80^3 the product moves 6.1 TB/s
-// of matrix (93 % of the copy rate) and takes 88 of the 123 us; below 40^3 the
-// two all-reduces (1.7 us each over 148 CTAs, as long alone) and the latencies
-// around them are half of the time.
+// Measured (B200, us an iteration, loop kernels -> here): 24^3 nodes 27.5 ->
+// 12.2, 32^3 31.8 -> 15.0, 40^3 41.5 -> 20.8 (single reduction 39.2 -> 20.8),
+// 64^3 87.0 -> 61.5, 80^3 145.9 -> 115.5 (and 13.0, 15.8, 21.8, 65, 123 with
+// the gathers behind the wait for the tile's values). At 80^3 the product runs
+// at the copy rate of HBM; up to 40^3 the two all-reduces (1.7 us each over 148
+// CTAs, as long alone) and the latencies around them are half of the time, and
+// the product (200 cycles a tile and SM; its bytes need 70 from the L2) waits
+// for shared-memory and gather wavefronts, 60 % of what the SM can issue.
 //
 // Single reduction (kSr): the update phase comes first with alpha and beta of
 // the last iteration; the product multiplies u = M r (in z).
@@ -145,7 +147,8 @@ __device__ __forceinline__ void stream_system(const SysDesc &D, uint32_t limit, 
     const uint32_t tiles_u = (rows + tu - 1) / tu;
     uint64_t *const bar = S.bar[warp];
     char *const stage = dyn + (size_t)warp * kStreamWarpBytes;
-    float *const xg = reinterpret_cast<float *>(stage + 2 * kStreamSpmvStage);
+    uint32_t *const cols = reinterpret_cast<uint32_t *>(stage + 2 * kStreamSpmvStage);
+    float *const xg = reinterpret_cast<float *>(stage + 2 * kStreamSpmvStage + kStreamColBytes);
     // The lane's row in a product tile: block row bo, row a of it. The third
     // block row's lanes are turned by two: with seven blocks a block row the
     // 16 lanes of a half-warp then read 16 different bank pairs.
@@ -183,17 +186,25 @@ __device__ __forceinline__ void stream_system(const SysDesc &D, uint32_t limit, 
     // Row pointers of tile t: a lane has that of its block row, lanes 30 and 31
     // the tile's end.
     auto row_ptrs = [&](uint32_t t) { return __ldg(D.brow_ptr + min(b0 + t * kStreamBrows + bo, b1)); };
-    // Two bulk copies, one a lane.
     auto issue_a = [&](uint32_t rp, uint32_t s) {
         const uint32_t k0 = __shfl_sync(kFull, rp, 0), k1 = __shfl_sync(kFull, rp, 30);
-        const uint32_t ka = k0 & ~3u, idx = k1 > k0 ? 4u * ((k1 - ka + 3u) & ~3u) : 0u, val = 144u * (k1 - k0);
-        char *dst = stage + s * kStreamSpmvStage;
-        if (lane == 0) mbar_expect(bar + s, val + idx);
+        if (lane == 0) {
+            mbar_expect(bar + s, 144u * (k1 - k0));
+            bulk_load_hint(stage + s * kStreamSpmvStage, D.bval + (size_t)k0 * 36u, 144u * (k1 - k0), bar + s, pol);
+        }
         __syncwarp();
-        if (lane < 2u)
-            bulk_load_hint(dst + (lane ? kStreamIdxOff : 0),
-                           lane ? (const void *)(D.bcol + ka) : (const void *)(D.bval + (size_t)k0 * 36u), lane ? idx : val,
-                           bar + s, pol);
+    };
+    // The block columns of a tile, two a lane.
+    uint32_t col0 = 0, col1 = 0;
+    auto load_cols = [&](uint32_t rp) {
+        const uint32_t k = __shfl_sync(kFull, rp, 0) + lane, k1 = __shfl_sync(kFull, rp, 30);
+        col0 = k < k1 ? __ldg(D.bcol + k) : 0u;
+        col1 = k + 32u < k1 ? __ldg(D.bcol + k + 32u) : 0u;
+    };
+    auto stage_cols = [&]() {
+        cols[lane] = col0;
+        if (lane + 32u < kStreamColBytes / 4u) cols[lane + 32u] = col1;
+        __syncwarp();
     };
     auto wait_stage = [&](uint32_t s) {
         if (!mbar_wait(bar + s, (phases >> s) & 1u, lim)) {
@@ -203,23 +214,25 @@ __device__ __forceinline__ void stream_system(const SysDesc &D, uint32_t limit, 
         }
         phases ^= 1u << s;
     };
-    // Row pointers of the first two tiles, and of the tiles in flight.
-    const uint32_t rpa = row_ptrs(warp), rpb = row_ptrs(warp + kStreamWarps);
-    uint32_t rp0 = 0, rp1 = 0;
+    // Row pointers of the first three tiles, and of this tile and the next two.
+    const uint32_t rpa = row_ptrs(warp), rpb = row_ptrs(warp + kStreamWarps), rpc = row_ptrs(warp + 2 * kStreamWarps);
+    uint32_t rp0 = 0, rp1 = 0, rp2 = 0;
     auto start_a = [&]() {
         rp0 = rpa;
         rp1 = rpb;
+        rp2 = rpc;
         if (warp < tiles_a) issue_a(rp0, 0);
         if (warp + kStreamWarps < tiles_a) issue_a(rp1, 1);
+        load_cols(rp0);
     };
     float zq[kStreamMaxCols], pq[kStreamMaxCols], z_own = 0.0f, p_own = 0.0f;
-    // Requests the gathered vectors of a tile whose stage has arrived. Plain
+    // Requests the gathered vectors of a tile whose columns are in `cols`. Plain
     // loads: the reduction's acquire has dropped the L1's older lines, and a
     // value is gathered by several rows of this SM.
-    auto gather = [&](uint32_t t, uint32_t rp, uint32_t s, const float *pv) {
+    auto gather = [&](uint32_t t, uint32_t rp, const float *pv) {
         const uint32_t k0 = __shfl_sync(kFull, rp, 0), end = __shfl_sync(kFull, rp, after);
         const uint32_t nk = lane < 30u ? end - rp : 0u;
-        const uint32_t *c = reinterpret_cast<const uint32_t *>(stage + s * kStreamSpmvStage + kStreamIdxOff) + (rp - (k0 & ~3u));
+        const uint32_t *c = cols + (rp - k0);
 #pragma unroll
         for (int j = 0; j < kStreamMaxCols; ++j) {
             zq[j] = pq[j] = 0.0f;
@@ -241,12 +254,13 @@ __device__ __forceinline__ void stream_system(const SysDesc &D, uint32_t limit, 
     auto product = [&](bool first, float bf, const float *pv, float *pw) {
         double sum = 0.0;
         if (warp < tiles_a) {
-            wait_stage(0);
-            gather(warp, rp0, 0, pv);
+            stage_cols();
+            gather(warp, rp0, pv);
+            load_cols(rp1);
         }
         uint32_t s = 0;
         for (uint32_t t = warp; t < tiles_a; t += kStreamWarps, s ^= 1u) {
-            const uint32_t rp = s ? rp1 : rp0;
+            const uint32_t rp = rp0;
             const uint32_t next = __shfl_sync(kFull, rp, after), k0 = __shfl_sync(kFull, rp, 0);
             const uint32_t nk = lane < 30u ? next - rp : 0u;
             float *const xl = xg + 8u * bo;
@@ -255,14 +269,16 @@ __device__ __forceinline__ void stream_system(const SysDesc &D, uint32_t limit, 
                 if ((uint32_t)j < nk)
                     xl[8u * (kStreamBrows + 1) * j + a] = kSr || first ? zq[j] : __fadd_rn(__fmul_rn(pq[j], bf), zq[j]);
             const float own = kSr || first ? z_own : __fadd_rn(__fmul_rn(p_own, bf), z_own);
-            __syncwarp();
-            // The next tile's gathers run behind this tile's sums.
-            if (t + kStreamWarps < tiles_a) {
-                wait_stage(s ^ 1u);
-                gather(t + kStreamWarps, s ? rp0 : rp1, s ^ 1u, pv);
-            }
-            uint32_t rp2 = 0;
-            if (t + 2 * kStreamWarps < tiles_a) rp2 = row_ptrs(t + 2 * kStreamWarps);
+            // The next tile's gathers, the columns of the one after it and the
+            // row pointers of a third run behind this tile's sums; they do not
+            // wait for the matrix values (that wait for each tile's bulk copy
+            // took half of the product phase).
+            stage_cols();
+            if (t + kStreamWarps < tiles_a) gather(t + kStreamWarps, rp1, pv);
+            if (t + 2 * kStreamWarps < tiles_a) load_cols(rp2);
+            uint32_t rp3 = 0;
+            if (t + 3 * kStreamWarps < tiles_a) rp3 = row_ptrs(t + 3 * kStreamWarps);
+            wait_stage(s);
             float acc = 0.0f;
             const float2 *B = reinterpret_cast<const float2 *>(stage + s * kStreamSpmvStage) + (size_t)(rp - k0) * 18u + 3u * a;
             const float4 *X = reinterpret_cast<const float4 *>(xl);
@@ -283,11 +299,10 @@ __device__ __forceinline__ void stream_system(const SysDesc &D, uint32_t limit, 
                 }
             }
             __syncwarp();  // the stage and xg are read
-            if (t + 2 * kStreamWarps < tiles_a) {
-                if (s) rp1 = rp2;
-                else rp0 = rp2;
-                issue_a(rp2, s);
-            }
+            if (t + 2 * kStreamWarps < tiles_a) issue_a(rp2, s);
+            rp0 = rp1;
+            rp1 = rp2;
+            rp2 = rp3;
             if (lane < 30u && b0 + t * kStreamBrows + bo < b1) {
                 const size_t i = 6u * (size_t)(b0 + t * kStreamBrows) + trow;
                 D.ap[i] = acc;
@@ -443,14 +458,13 @@ __device__ __forceinline__ void stream_system(const SysDesc &D, uint32_t limit, 
         float *const p_old = kSr ? D.p : (iter & 1u ? D.p2 : D.p), *const p_new = kSr ? D.p : (iter & 1u ? D.p : D.p2);
         const double pw = warp_sum(product(first, S.beta_f, p_old, p_new));
         ++tag;
-        // The update's stages reuse the product's.
-        fence_proxy_smem();
-        __syncwarp();
-        start_u();
         if (lane == 0) S.w[0][warp] = pw;
+        fence_proxy_smem();
         __syncthreads();
         double pap = 0.0;
         if (warp == 0) pap = publish(S, 0, out, copies, tag, false);
+        // The update's stages reuse the product's.
+        start_u();
         if (warp < tiles_u) fetch_u(warp, p_new);
         if (warp == 0) {
             if (gridDim.x > 1) pap = team_gather(&S.err, red, gridDim.x, tag, sp, lim);

@@ -13,8 +13,8 @@ constexpr int kStreamThreads = 32 * kStreamWarps;
 constexpr int kStreamBrows = 5;
 constexpr int kStreamMaxBlocks = 36;
 constexpr int kStreamMaxCols = 8;
-constexpr int kStreamIdxOff = 144 * kStreamMaxBlocks;                     // block columns in a product stage
-constexpr int kStreamSpmvStage = kStreamIdxOff + 4 * (kStreamMaxBlocks + 12);
+constexpr int kStreamSpmvStage = 144 * kStreamMaxBlocks;
+constexpr int kStreamColBytes = 4 * ((kStreamMaxBlocks + 3) / 4 * 4);     // a tile's block columns
 constexpr int kStreamXgBytes = 32 * (kStreamBrows + 1) * kStreamMaxCols;  // p at a tile's block columns
 // Update tiles: up to kStreamUpd(Sr)Brows block rows, one a lane: the factors,
 // the slices of x and r (kSr: p and s too) and the new z.
@@ -25,8 +25,9 @@ static_assert(kStreamUpdBrowsSr * (144 + 5 * 24) <= kStreamUpdStage, "update sta
 static_assert(kStreamUpdBrows % 2 == 0 && kStreamUpdBrowsSr % 2 == 0, "16-byte slices");
 // Each warp has two stages, used by both phases.
 constexpr int kStreamWarpBytes = 2 * kStreamUpdStage;
-static_assert(2 * kStreamSpmvStage + kStreamXgBytes <= kStreamWarpBytes, "product stages");
-static_assert(kStreamUpdStage % 16 == 0 && kStreamSpmvStage % 16 == 0 && kStreamIdxOff % 16 == 0, "TMA alignment");
+static_assert(2 * kStreamSpmvStage + kStreamColBytes + kStreamXgBytes <= kStreamWarpBytes, "product stages");
+static_assert(kStreamMaxBlocks <= 64, "two columns a lane");
+static_assert(kStreamUpdStage % 16 == 0 && kStreamSpmvStage % 16 == 0 && kStreamColBytes % 16 == 0, "TMA alignment");
 constexpr int kStreamFixedSmem = 2048;
 constexpr int kStreamSmem = kStreamFixedSmem + kStreamWarps * kStreamWarpBytes;
 static_assert(kStreamSmem <= 227 * 1024, "shared memory");
