@@ -63,7 +63,7 @@ def test_single_reduction(ctx, nbr):
 
 # More block rows than k_team's CTAs hold (148 x 70): odd and even counts, with
 # rows that end in the middle of tiles.
-@pytest.mark.parametrize("nbr", [10361, 12346, 13321, 75777])
+@pytest.mark.parametrize("nbr", [10361, 12346, 13321, 19241, 19999, 75777])
 def test_classic_beyond_shared_memory(ctx, nbr):
     rp, ci, v, bs, b = ring_system(nbr, (1, 7, 101), nbr)
     n = len(rp) - 1
@@ -82,7 +82,7 @@ def test_paths_together_and_cut_into_steps(ctx):
     loop kernels): the bits of each solved alone."""
     small = wsb.lattice_generate(6, seed=1)
     large = ring_system(10500, (1, 7, 101), 3)
-    larger = ring_system(13500, (1, 7, 101), 3)
+    larger = ring_system(19500, (1, 7, 101), 3)
     long_rows = ring_system(12000, (1, 2, 3, 4, 5, 6), 4)  # 13 blocks a row: too long for k_stream
     systems = [(small["row_ptr"], small["col_idx"], small["values"], small["block_starts"], small["b"]), large, larger, long_rows]
     kw = dict(max_iter=3000, rel_tol=1e-6)
@@ -103,7 +103,7 @@ def test_paths_together_and_cut_into_steps(ctx):
             assert np.array_equal(x.view(np.uint32), alone[i][0].view(np.uint32)), i
 
 
-@pytest.mark.parametrize("nbr", [10400, 13400])
+@pytest.mark.parametrize("nbr", [10400, 19400])
 def test_wait_limit_and_recovery(nbr):
     c = wsb.GpuContext.create("auto", 0)
     try:
@@ -121,7 +121,7 @@ def test_wait_limit_and_recovery(nbr):
         c.set_wait_limit(0)
 
 
-@pytest.mark.parametrize("nbr", [10400, 13400])
+@pytest.mark.parametrize("nbr", [10400, 19400])
 def test_zero_rhs_and_iteration_limit(ctx, nbr):
     rp, ci, v, bs, b = ring_system(nbr, (1, 7, 101), 6)
     m = wsb.Matrix.create(ctx, rp, ci, v, bs)

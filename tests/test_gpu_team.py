@@ -108,17 +108,18 @@ def test_zero_entries_of_the_residual(ctx):
     check(ctx, rp, ci, v, bs, b)
 
 
-# Block rows: the most of a narrow cut of up to 120 CTAs; one more (the wide
-# cut, 94 CTAs); a wide cut on all 148 SMs with a ragged last warp tile.
-@pytest.mark.parametrize("nbr", [8400, 8401, 13318])
-def test_narrow_and_wide_cuts(ctx, nbr):
+# Block rows (70 a part): 120 parts exactly, plus one row; the most with one
+# part a CTA (148 SMs); one more (two parts a CTA, an odd count: 149); a ragged
+# last warp tile; two parts on all SMs.
+@pytest.mark.parametrize("nbr", [8400, 8401, 10360, 10361, 13318, 20720])
+def test_one_and_two_parts_a_cta(ctx, nbr):
     check(ctx, *block_system(nbr, 0, nbr))
 
 
-def test_wide_and_narrow_teams_in_one_launch(ctx):
-    # Narrow teams run in the wide variant here, and more teams than the device
-    # holds wait for idle CTAs: the same bits as alone.
-    systems = [block_system(nbr, 1, nbr) for nbr in (8401, 3000, 1, 71, 6000, 8500, 500, 69, 2000, 281)]
+def test_more_teams_than_the_device_holds(ctx):
+    # Two parts a CTA, and systems that wait for idle CTAs: the same bits as
+    # alone (one part a CTA, but for the first).
+    systems = [block_system(nbr, 1, nbr) for nbr in (10500, 8401, 3000, 1, 71, 140, 141, 6000, 8500, 500, 69, 2000, 281)]
     mats = [wsb.Matrix.create(ctx, rp, ci, v, bs, layout=wsb.LAYOUT_BSR6) for rp, ci, v, bs, _ in systems]
     batch = wsb.Batch(ctx)
     ids = [batch.add(m, s[4], max_iter=4000, rel_tol=1e-6) for m, s in zip(mats, systems)]

@@ -161,9 +161,13 @@ struct Engine::Slot {
     bool stalled = false;
     uint64_t iters_total = 0;
     SolveOutcome out;
-    // k_team (team > 0): CTAs of the system's team, warp tiles and most blocks a
-    // CTA holds, most bytes of its tiles, published partials, z packets.
-    uint32_t team = 0, team_warps = 0, team_ext = 0, team_tiles = 0;
+    // k_team (team > 0): parts of the system, warp tiles of a part; for CTAs of
+    // one and of two parts, the most blocks a CTA multiplies and the most bytes
+    // of its warp tiles (0: two parts do not fit).
+    uint32_t team = 0, team_warps = 0, team_ext[2] = {0, 0}, team_tiles[2] = {0, 0};
+    uint32_t team_smem(uint32_t launch_parts, uint32_t parts) const {
+        return (uint32_t)team_fixed_bytes(launch_parts) + team_z_bytes(launch_parts, team_ext[parts - 1]) + team_tiles[parts - 1];
+    }
     // k_stream (stream > 0): CTAs; its second buffer of p and partials.
     uint32_t stream = 0;
     float *p2 = nullptr;
@@ -200,8 +204,8 @@ Engine::Engine(Context *ctx, cudaStream_t stream) : ctx_(ctx), stream_(stream) {
     max_grid_a_ = std::max(1, occ_a) * std::max(1, ctx->sm_count);
     max_grid_b_ = std::max(1, occ_b) * std::max(1, ctx->sm_count);
     max_grid_c_ = std::max(1, occ_c) * std::max(1, ctx->sm_count);
-    for (int w : {kTeamWarps, kTeamWarpsWide})
-        cudaFuncSetAttribute(team_kernel(w), cudaFuncAttributeMaxDynamicSharedMemorySize, kTeamSmemMax);
+    for (int parts : {1, 2})
+        cudaFuncSetAttribute(team_kernel(parts), cudaFuncAttributeMaxDynamicSharedMemorySize, kTeamSmemMax);
     for (bool sr : {false, true})
         cudaFuncSetAttribute(stream_kernel(sr), cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmem);
     const char *loop_env = getenv("WSB_LOOP");
@@ -298,33 +302,36 @@ void Engine::team_plan(Slot *sl) const {
         sl->cfg.algorithm != WSB_ALG_CLASSIC)
         return;
     const uint32_t nbr = A.n / 6, tiles = (nbr + kTeamWarpBrows - 1) / kTeamWarpBrows, sms = (uint32_t)ctx_->sm_count;
-    if (tiles > sms * kTeamWarpsWide) return;
+    if (tiles > 2 * sms * kTeamWarps) return;
     std::vector<uint32_t> cols(tiles, 0u);  // blocks of each warp tile's longest block row
     for (uint32_t br = 0; br < nbr; ++br)
         cols[br / kTeamWarpBrows] = std::max(cols[br / kTeamWarpBrows], A.h_rows[br + 1] - A.h_rows[br]);
-    // The most warp tiles a CTA that fit whichever CTA it is.
-    for (uint32_t w = tiles <= kTeamNarrowCtas * kTeamWarps ? kTeamWarps : kTeamWarpsWide; w >= 1; --w) {
-        const uint32_t size = (tiles + w - 1) / w;
-        if (size > sms) return;
-        uint64_t most = 0;
-        uint32_t blocks = 0;
-        for (uint32_t c = 0; c < size; ++c) {
-            uint64_t sum = 0;
-            const uint32_t end = std::min((c + 1) * w, tiles);
-            for (uint32_t q = c * w; q < end; ++q) sum += team_tile_bytes(cols[q]);
-            most = std::max(most, sum);
-            blocks = std::max(blocks, A.h_rows[std::min(end * kTeamWarpBrows, nbr)] - A.h_rows[c * w * kTeamWarpBrows]);
+    // The most warp tiles a part with which two parts fit in a CTA, whichever
+    // CTA it is; when none does, one part.
+    for (uint32_t parts = 2; parts >= 1 && !sl->team; --parts)
+        for (uint32_t w = kTeamWarps; w >= 1; --w) {
+            const uint32_t size = (tiles + w - 1) / w;
+            if ((size + parts - 1) / parts > sms) break;
+            sl->team_warps = w;
+            for (uint32_t k = 1; k <= 2; ++k) {
+                uint64_t most = 0;
+                uint32_t blocks = 0;
+                for (uint32_t c = 0; c < size; c += k) {
+                    uint64_t sum = 0;
+                    const uint32_t end = std::min((c + k) * w, tiles);
+                    for (uint32_t q = c * w; q < end; ++q) sum += team_tile_bytes(cols[q]);
+                    most = std::max(most, sum);
+                    blocks = std::max(blocks, A.h_rows[std::min(end * kTeamWarpBrows, nbr)] - A.h_rows[c * w * kTeamWarpBrows]);
+                }
+                sl->team_ext[k - 1] = size > k ? blocks : 0u;
+                sl->team_tiles[k - 1] = (uint32_t)std::min<uint64_t>(most, kTeamSmemMax);
+                // One part a CTA may run beside pairs, in their kernel.
+                if (sl->team_smem(2, k) > (uint32_t)kTeamSmemMax) sl->team_tiles[k - 1] = 0;
+            }
+            if (!sl->team_tiles[parts - 1]) continue;
+            sl->team = size;
+            return;
         }
-        const uint32_t ext = size > 1 ? blocks : 0u;
-        // A narrow team may run in the wide variant, beside wide ones.
-        const uint64_t smem = team_fixed_bytes(kTeamWarpsWide) + team_z_bytes(kTeamWarpsWide, ext) + most;
-        if (smem > (uint64_t)kTeamSmemMax) continue;
-        sl->team = size;
-        sl->team_warps = w;
-        sl->team_ext = ext;
-        sl->team_tiles = (uint32_t)most;
-        return;
-    }
 }
 
 // Whether k_stream iterates a system that k_team does not: BSR6, more block
@@ -476,7 +483,9 @@ int Engine::add(const MatA *A, const Precond *M, const SolveCfg &cfg, uint32_t *
     d.algo = (uint32_t)cfg.algorithm;
     d.s = sl->s;
     d.team_warps = sl->team_warps;
-    d.team_ext = sl->team_ext;
+    d.team_ext[0] = sl->team_ext[0];
+    d.team_ext[1] = sl->team_ext[1];
+    d.team_pairs = sl->team > (uint32_t)ctx_->sm_count;
     d.path = sl->team ? PATH_TEAM : sl->stream ? PATH_STREAM : PATH_LOOP;
     d.p2 = sl->p2;
     d.stream_past_l2 = 148ull * A->nbsr + 144ull * M->nb > kL2Keep;
@@ -818,52 +827,80 @@ int Engine::finish_slot(uint32_t s, int status) {
     return WSB_OK;
 }
 
-// One cooperative launch of k_team over the given systems, one CTA per SM.
-// When the device holds all their teams at once, each CTA has one system.
-// Otherwise the lists follow a simulated run in which, whenever CTAs fall idle,
-// the widest system that fits starts (a system that ends leaves room for any
-// that could not start before it, so wide ones do not starve). A solve takes
-// about the fourth root of its rows in iterations, each of about 4.2 us plus
-// 26 ns a CTA. Every CTA's list is in the order in which systems start, so no
-// two systems wait for each other whatever the times turn out to be.
+// One cooperative launch of k_team over the given systems, one CTA per SM. A
+// CTA holds one part of a system, or two of a system with more parts than SMs.
+// When the device holds all teams at once, each CTA has one system. Otherwise
+// the lists follow a simulated run in which, whenever CTAs fall idle, the
+// widest system that fits starts (a system that ends leaves room for any that
+// could not start before it, so wide ones do not starve), with one or with two
+// parts a CTA, whichever run ends first: a pair takes about 1.4 times as long
+// on half the CTAs, which pays once systems wait for CTAs (B200, us a
+// system-iteration, one part against two: 24 systems of 14^3 nodes 1.74 and
+// 1.14, 13 of 9^3 0.38 and 0.49). A solve takes about twenty times the fourth
+// root of its rows in iterations; the time of one is fitted to measured ones.
+// Every CTA's list is in the order in which systems start, so no two systems
+// wait for each other whatever the times turn out to be.
 int Engine::launch_team(const std::vector<uint32_t> &ids, uint32_t limit) {
     if (ids.empty()) return WSB_OK;
     const uint32_t sms = (uint32_t)std::max(1, ctx_->sm_count);
-    uint64_t total = 0;
-    int warps = kTeamWarps;
-    for (uint32_t s : ids) {
-        total += slots_[s]->team;
-        if (slots_[s]->team_warps > (uint32_t)kTeamWarps) warps = kTeamWarpsWide;
-    }
-    uint32_t smem = 0;
-    for (uint32_t s : ids)
-        smem = std::max(smem, (uint32_t)team_fixed_bytes(warps) + team_z_bytes(warps, slots_[s]->team_ext) + slots_[s]->team_tiles);
-    std::map<uint32_t, std::vector<uint32_t>> waiting;  // by team size, the first to start last
-    for (auto it = ids.rbegin(); it != ids.rend(); ++it) waiting[slots_[*it]->team].push_back(*it);
-    const uint32_t grid = (uint32_t)std::min<uint64_t>(total, sms);
-    std::vector<std::vector<TeamItem>> lists(grid);
-    std::vector<uint32_t> idle(grid);
-    for (uint32_t c = 0; c < grid; ++c) idle[c] = grid - 1 - c;
-    std::multimap<double, std::vector<uint32_t>> running;  // CTAs of a system by when it ends
-    double now = 0.0;
-    while (!waiting.empty()) {
-        auto fits = waiting.upper_bound((uint32_t)idle.size());
-        if (fits == waiting.begin()) {
-            now = running.begin()->first;
-            idle.insert(idle.end(), running.begin()->second.rbegin(), running.begin()->second.rend());
-            running.erase(running.begin());
-            continue;
+    struct Run {
+        std::vector<std::vector<TeamItem>> lists;
+        uint32_t parts = 1, smem = 0;  // parts a CTA of the launch, its shared memory
+        double end = 0.0;
+    };
+    auto parts_of = [&](const Slot &sl, bool pairs) {
+        return sl.team > sms || (pairs && sl.team > 1 && sl.team_tiles[1]) ? 2u : 1u;
+    };
+    auto simulate = [&](bool pairs) {
+        Run run;
+        std::map<uint32_t, std::vector<uint32_t>> waiting;  // by CTAs, the first to start last
+        uint64_t total = 0;
+        for (auto it = ids.rbegin(); it != ids.rend(); ++it) {
+            const Slot &sl = *slots_[*it];
+            const uint32_t parts = parts_of(sl, pairs), ctas = (sl.team + parts - 1) / parts;
+            waiting[ctas].push_back(*it);
+            total += ctas;
+            run.parts = std::max(run.parts, parts);
         }
-        --fits;
-        const uint32_t s = fits->second.back(), team = fits->first;
-        fits->second.pop_back();
-        if (fits->second.empty()) waiting.erase(fits);
-        const Slot &sl = *slots_[s];
-        std::vector<uint32_t> ctas(idle.rbegin(), idle.rbegin() + team);
-        idle.resize(idle.size() - team);
-        for (uint32_t k = 0; k < team; ++k) lists[ctas[k]].push_back({s, k, team, 0u});
-        running.emplace(now + std::pow((double)sl.A->n, 0.25) * (160.0 + team), std::move(ctas));
+        for (uint32_t s : ids) run.smem = std::max(run.smem, slots_[s]->team_smem(run.parts, parts_of(*slots_[s], pairs)));
+        const uint32_t grid = (uint32_t)std::min<uint64_t>(total, sms);
+        run.lists.resize(grid);
+        std::vector<uint32_t> idle(grid);
+        for (uint32_t c = 0; c < grid; ++c) idle[c] = grid - 1 - c;
+        std::multimap<double, std::vector<uint32_t>> running;  // CTAs of a system by when it ends
+        double now = 0.0;
+        while (!waiting.empty()) {
+            auto fits = waiting.upper_bound((uint32_t)idle.size());
+            if (fits == waiting.begin()) {
+                now = running.begin()->first;
+                idle.insert(idle.end(), running.begin()->second.rbegin(), running.begin()->second.rend());
+                running.erase(running.begin());
+                continue;
+            }
+            --fits;
+            const uint32_t s = fits->second.back(), width = fits->first;
+            fits->second.pop_back();
+            if (fits->second.empty()) waiting.erase(fits);
+            const Slot &sl = *slots_[s];
+            const uint32_t parts = parts_of(sl, pairs);
+            std::vector<uint32_t> ctas(idle.rbegin(), idle.rbegin() + width);
+            idle.resize(idle.size() - width);
+            for (uint32_t k = 0; k < width; ++k) run.lists[ctas[k]].push_back({s, k * parts, sl.team, parts});
+            const double us = width == 1 ? 3.0 * parts : parts == 1 ? 4.1 + 0.021 * width : 5.9 + 0.033 * width;
+            const double end = now + us * std::min<double>(limit, 20.0 * std::pow((double)sl.A->n, 0.25));
+            run.end = std::max(run.end, end);
+            running.emplace(end, std::move(ctas));
+        }
+        return run;
+    };
+    Run run = simulate(false);
+    const bool crowded = std::any_of(run.lists.begin(), run.lists.end(), [](const auto &l) { return l.size() > 1; });
+    if (crowded) {
+        Run pairs = simulate(true);
+        if (pairs.end < run.end) run = std::move(pairs);
     }
+    const auto &lists = run.lists;
+    const uint32_t grid = (uint32_t)lists.size();
     size_t items = 0;
     for (const auto &l : lists) items += l.size();
     const size_t head = ((size_t)grid + 1 + 3) & ~size_t(3), words = head + 4 * items;
@@ -891,8 +928,8 @@ int Engine::launch_team(const std::vector<uint32_t> &ids, uint32_t limit) {
     const TeamItem *ditems = reinterpret_cast<const TeamItem *>(d_team_ + head);
     const uint32_t *doff = d_team_;
     void *args[] = {&dsys, &dsp, &ditems, &doff, &limit};
-    WSB_CUDA_TRY(ctx_, cudaLaunchCooperativeKernel(team_kernel(warps), dim3(grid), dim3(team_threads(warps)), args,
-                                                   (size_t)smem, stream_));
+    WSB_CUDA_TRY(ctx_, cudaLaunchCooperativeKernel(team_kernel((int)run.parts), dim3(grid), dim3(kTeamThreads), args,
+                                                   (size_t)run.smem, stream_));
     launches_ += 1;
     return WSB_OK;
 }

@@ -5,7 +5,7 @@
 // dependent launches, each with its ramp, its chain of work-item loads and its
 // last-CTA sum. Here an iteration is two exchanges between resident CTAs and
 // the latency of one row sum and one block solve:
-//   - a lane owns a row: x, r, z and p stay in registers; the matrix, p at
+//   - a lane owns a row (or two): x, r, z and p stay in registers; the matrix, p at
 //     every block's columns and the blocks' LU factors stay in shared memory,
 //     so an iteration reads only other CTAs' z from the L2, each block of it
 //     once a CTA (all row warps fetch, then all read it from shared memory);
@@ -18,14 +18,17 @@
 //     next product. Every CTA forms p = z + beta p for the block columns it
 //     multiplies (same operation, same bits as the owner's), so p is never
 //     exchanged.
-// Measured (B200, us an iteration, loop kernels -> here): 4^3 nodes 24.4 -> 2.9,
-// 9^3 23.5 -> 4.5, 12^3 24.8 -> 5.0, 17^3 25.7 -> 5.9, 20^3 27.2 -> 7.2,
-// 23^3 28 -> 8.7. 48 systems of 4^3 to 24^3 nodes at once: 27.6 ms -> 22.0.
+// Measured (B200, us an iteration, loop kernels -> here): 4^3 nodes 24.4 -> 2.8,
+// 9^3 23.5 -> 4.4, 12^3 24.8 -> 4.8, 17^3 25.7 -> 5.4, 21^3 27.5 -> 6.9; with
+// two parts a CTA 9^3 6.1, 14^3 6.8 (one: 4.9), 20^3 8.2 (6.8), and 22^3 8.1,
+// 24^3 9.0, 26^3 9.8 (in k_stream 11.5, 12.2, 12.6). 48 systems of 4^3 to 24^3
+// nodes at once: 27.6 ms -> 15.6.
 // What is left is latency (7 of 13 warps wait at a barrier at any time, issue
 // slots 28 % used): per iteration two hops through the L2 (800 cycles for
 // 8 CTAs, 1,400 for 31), the FP64 sums (nine cycles an add, 36 with the shuffle
 // between lanes), two FP64 divisions and the block solve. So products are
-// added through shared memory, 14 or 18 per lane, before the lanes; a block
+// added through shared memory, 14 per lane as a tree, before the lanes, and two
+// parts' side by side (one after the other: 22^3 8.7 us, 20^3 8.8); a block
 // is solved by one lane from shared memory (no shuffles between its steps); and
 // all waits are warp-uniform loops: lanes that leave such a loop one by one
 // stay apart and made the code after it up to ten times slower.
@@ -54,7 +57,7 @@ struct TeamShared {
     // Scalars of the recurrence, kept by one thread (the same in every CTA).
     double bb, rz_old, pap, alpha_d, rr, rel2, abs2;
     uint32_t iter, max_iter, status, breakdown;
-    uint32_t bytes[kTeamWarpsWide];  // shared memory of each warp tile
+    uint32_t bytes[2 * kTeamWarps];  // shared memory of each warp tile
     alignas(16) double v[1];     // the rows' products of a reduction, twice 32 a warp tile
 };
 
@@ -63,70 +66,83 @@ struct WaitCtl {
     long long lim;
 };
 
-// Sum of one value per row of the CTA, by one warp: lane l adds a pair per two
-// warp tiles, those of the first kTeamWarps as a tree, then (wide) the others,
-// then the lanes; valid in lane 0. Warp tiles that a narrow CTA does not have
-// are zeros in a wide one: the same sum.
-template <int kWarps>
-__device__ __forceinline__ double cta_sum(const double *v, uint32_t lane) {
+// Sums of one value per row of each of kT parts (v: 32 kTeamWarps a part), by
+// one warp: lane l adds a pair per two warp tiles, as a tree, then the lanes;
+// valid in lane 0. The parts' sums run side by side.
+template <int kT>
+__device__ __forceinline__ void part_sums(const double *v, uint32_t lane, double (&sum)[kT]) {
     constexpr int kPairs = kTeamWarps / 2;
+    static_assert(kTeamWarps % 2 == 0, "pairs");
     const double2 *v2 = reinterpret_cast<const double2 *>(v) + lane;
-    double s[kPairs];
+    double s[kT][kPairs];
 #pragma unroll
-    for (int k = 0; k < kPairs; ++k) {
-        const double2 a = v2[32 * k];
-        s[k] = a.x + a.y;
-    }
+    for (int k = 0; k < kPairs; ++k)
+#pragma unroll
+        for (int t = 0; t < kT; ++t) {
+            const double2 a = v2[16 * kTeamWarps * t + 32 * k];
+            s[t][k] = a.x + a.y;
+        }
 #pragma unroll
     for (int n = kPairs; n > 1; n = (n + 1) / 2)
 #pragma unroll
-        for (int k = 0; k < n / 2; ++k) s[k] += s[k + (n + 1) / 2];
-    if (kWarps > kTeamWarps) {
-        double t = 0.0;
+        for (int k = 0; k < n / 2; ++k)
 #pragma unroll
-        for (int k = kPairs; k < kWarps / 2; ++k) {
-            const double2 a = v2[32 * k];
-            t += a.x + a.y;
-        }
-        s[0] += t;
-    }
-    return warp_sum(s[0]);
+            for (int t = 0; t < kT; ++t) s[t][k] += s[t][k + (n + 1) / 2];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int t = 0; t < kT; ++t) s[t][0] += __shfl_down_sync(kFull, s[t][0], o);
+#pragma unroll
+    for (int t = 0; t < kT; ++t) sum[t] = s[t][0];
 }
-static_assert(kTeamWarps % 2 == 0 && kTeamWarpsWide % 2 == 0, "cta_sum");
 
 // One system, this CTA's rows, up to `limit` iterations.
-template <int kWarps>
+template <int kT>
 __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamItem it, uint32_t limit, TeamShared &S,
                                                  char *dyn, const WaitCtl &w) {
     constexpr int kAhead = 8;  // block columns a lane handles at once
+    constexpr uint32_t kRows = 32u * kTeamWarps;  // places for the rows of a part
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     SysState *st = D.st;
     if (!st->active) return;
-    const uint32_t nbr = D.n / 6u, tw = D.team_warps, cta_brows = tw * (uint32_t)kTeamWarpBrows;
-    const bool lead = it.rank == 0, alone = it.size == 1;
-    const uint32_t br0 = min(it.rank * cta_brows, nbr), br1 = min(br0 + cta_brows, nbr);
+    const uint32_t nbr = D.n / 6u, tw = D.team_warps, part_brows = tw * (uint32_t)kTeamWarpBrows;
+    const bool lead = it.rank == 0, alone = it.parts >= it.size;
+    const uint32_t br0 = min(it.rank * part_brows, nbr), br1 = min(br0 + it.parts * part_brows, nbr);
     const bool fresh = st->fresh != 0;
-    // The lane's row.
+    // The warps with rows; the last two warps have none: they reduce. The
+    // first of them sums p.Ap and r.r and decides, the second sums r.z and
+    // forms beta.
+    const bool rows = warp < (uint32_t)kTeamWarps, red_a = warp == (uint32_t)kTeamWarps, red_b = warp == (uint32_t)kTeamWarps + 1u;
+    // The lane's rows, one a part.
     const uint32_t bo = lane / 6u, a = lane % 6u;
-    const uint32_t br = br0 + warp * (uint32_t)kTeamWarpBrows + bo;
-    const bool on = lane < (uint32_t)kTeamWarpRows && warp < tw && br < br1;
-    const uint32_t row = on ? 6u * br + a : 0u;
-    uint32_t k0 = 0, nk = 0;
-    float x = 0.f, r = 0.f, z = 0.f, p = 0.f;
-    if (on) {
-        k0 = D.brow_ptr[br];
-        nk = D.brow_ptr[br + 1] - k0;
-        x = D.x[row];
-        if (!fresh) {
-            r = D.r[row];
-            z = D.z[row];
-            p = D.p[row];
+    bool on[kT];
+    uint32_t row[kT], k0[kT], nk[kT], cols[kT], most = 0;  // cols: most blocks of a block row of the warp tile
+    float x[kT], r[kT], z[kT], p[kT];
+#pragma unroll
+    for (int t = 0; t < kT; ++t) {
+        const uint32_t br = br0 + (t * tw + warp) * (uint32_t)kTeamWarpBrows + bo;
+        on[t] = lane < (uint32_t)kTeamWarpRows && warp < tw && (uint32_t)t < it.parts && br < br1;
+        row[t] = on[t] ? 6u * br + a : 0u;
+        k0[t] = nk[t] = 0;
+        x[t] = r[t] = z[t] = p[t] = 0.0f;
+        if (on[t]) {
+            k0[t] = D.brow_ptr[br];
+            nk[t] = D.brow_ptr[br + 1] - k0[t];
+            x[t] = D.x[row[t]];
+            if (!fresh) {
+                r[t] = D.r[row[t]];
+                z[t] = D.z[row[t]];
+                p[t] = D.p[row[t]];
+            }
         }
+        cols[t] = __reduce_max_sync(kFull, nk[t]);
+        most = max(most, cols[t]);
+        if (lane == 0 && rows) S.bytes[t * kTeamWarps + warp] = team_tile_bytes(cols[t]);
     }
-    const uint32_t cols = __reduce_max_sync(kFull, nk);  // of the warp tile
-    if (lane == 0 && warp < (uint32_t)kWarps) S.bytes[warp] = team_tile_bytes(cols);
-    double *const v0 = S.v, *const v1 = S.v + 32 * kWarps;
-    if (warp < (uint32_t)kWarps) v0[tid] = v1[tid] = 0.0;
+    double *const v0 = S.v, *const v1 = S.v + kT * kRows;
+    if (rows)
+#pragma unroll
+        for (int t = 0; t < kT; ++t) v0[t * kRows + tid] = v1[t * kRows + tid] = 0.0;
     if (tid == 0) S.ext = 0;
     __syncthreads();
     // Dynamic shared memory: z of the CTA's rows (first r, then z, 32 a warp
@@ -135,55 +151,70 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
     // short division, and for block j of its block rows, lane by lane (no bank
     // conflicts), the row's first four values, its last two, p at the block's
     // columns, and where z of the block's columns is.
+    const uint32_t most_ext = D.team_ext[it.parts - 1u];
     float *const zx = reinterpret_cast<float *>(dyn);
-    uint32_t *const ext = reinterpret_cast<uint32_t *>(zx + 32 * kWarps + 6u * D.team_ext);
-    uint32_t before = 0;
-    for (uint32_t q = 0; q < min(warp, tw); ++q) before += S.bytes[q];
-    char *mine = dyn + team_z_bytes(kWarps, D.team_ext) + before;
-    // (cols == 0: a warp without rows; it touches none of this.)
-    float *const lu = reinterpret_cast<float *>(mine);
-    float *const rd = lu + 36 * kTeamWarpBrows;
-    mine += kTeamLuBytes;
-    const uint32_t colp = (cols + 7u) & ~7u;
-    float4 *b4 = reinterpret_cast<float4 *>(mine) + lane;
-    float2 *b2 = reinterpret_cast<float2 *>(mine + (size_t)cols * 16u * kTeamWarpRows) + lane;
-    float *xg = reinterpret_cast<float *>(mine + (size_t)cols * 24u * kTeamWarpRows) + 8u * bo;
-    uint32_t *bc = reinterpret_cast<uint32_t *>(mine + (size_t)cols * kTeamColBytes);
-    for (uint32_t j = lane; j < colp * (uint32_t)(kTeamWarpBrows + 1); j += 32u) bc[j] = 0;  // past a row's end
-    bc += colp * bo;
-    __syncwarp();
-    if (on) {
-        // p (or x0 for a fresh system) at the block columns, one component a lane.
-        const float *src = (fresh ? D.x : D.p) + a;
+    uint32_t *const ext = reinterpret_cast<uint32_t *>(zx + kT * kRows + 6u * most_ext);
+    char *const tiles = dyn + team_z_bytes(kT, most_ext);
+    // (cols == 0: a warp tile without rows; it touches none of this.)
+    float *lu[kT], *xg[kT];
+    float4 *b4[kT];
+    float2 *b2[kT];
+    uint32_t *bc[kT];
+#pragma unroll
+    for (int t = 0; t < kT; ++t) {
+        uint32_t before = 0;
+        for (uint32_t q = 0; q < t * tw + min(warp, tw); ++q) before += S.bytes[q < tw ? q : kTeamWarps + q - tw];
+        char *mine = tiles + before;
+        lu[t] = reinterpret_cast<float *>(mine);
+        mine += kTeamLuBytes;
+        const uint32_t colp = (cols[t] + 7u) & ~7u;
+        b4[t] = reinterpret_cast<float4 *>(mine) + lane;
+        b2[t] = reinterpret_cast<float2 *>(mine + (size_t)cols[t] * 16u * kTeamWarpRows) + lane;
+        xg[t] = reinterpret_cast<float *>(mine + (size_t)cols[t] * 24u * kTeamWarpRows) + 8u * bo;
+        bc[t] = reinterpret_cast<uint32_t *>(mine + (size_t)cols[t] * kTeamColBytes);
+        for (uint32_t j = lane; j < colp * (uint32_t)(kTeamWarpBrows + 1); j += 32u) bc[t][j] = 0;  // past a row's end
+        bc[t] += colp * bo;
+        __syncwarp();
+        if (on[t]) {
+            // p (or x0 for a fresh system) at the block columns, one component a lane.
+            const float *src = (fresh ? D.x : D.p) + a;
 #pragma unroll 1
-        for (uint32_t j = 0; j < nk; ++j) {
-            const float *v = D.bval + (size_t)(k0 + j) * 36u + 6u * a;
-            float4 *d4 = b4 + j * kTeamWarpRows;
-            cp_async8(d4, v);
-            cp_async8(reinterpret_cast<float2 *>(d4) + 1, v + 2);
-            cp_async8(b2 + j * kTeamWarpRows, v + 4);
-            const uint32_t c = D.bcol[k0 + j];
-            cp_async4(xg + 8u * kTeamWarpBrows * j + a, src + 6u * (size_t)c);
-            if (a == 0) {
-                if (c >= br0 && c < br1) {
-                    bc[j] = 32u * ((c - br0) / kTeamWarpBrows) + 6u * ((c - br0) % kTeamWarpBrows);
-                } else {
-                    const uint32_t e = atomicAdd(&S.ext, 1u);  // (the order changes no value)
-                    bc[j] = 32u * kWarps + 6u * e;
-                    ext[e] = 6u * c;
+            for (uint32_t j = 0; j < nk[t]; ++j) {
+                const float *v = D.bval + (size_t)(k0[t] + j) * 36u + 6u * a;
+                float4 *d4 = b4[t] + j * kTeamWarpRows;
+                cp_async8(d4, v);
+                cp_async8(reinterpret_cast<float2 *>(d4) + 1, v + 2);
+                cp_async8(b2[t] + j * kTeamWarpRows, v + 4);
+                const uint32_t c = D.bcol[k0[t] + j];
+                cp_async4(xg[t] + 8u * kTeamWarpBrows * j + a, src + 6u * (size_t)c);
+                if (a == 0) {
+                    if (c >= br0 && c < br1) {
+                        const uint32_t q = (c - br0) / kTeamWarpBrows, part = q >= tw ? 1u : 0u;
+                        bc[t][j] = part * kRows + 32u * (q - part * tw) + 6u * ((c - br0) % kTeamWarpBrows);
+                    } else {
+                        const uint32_t e = atomicAdd(&S.ext, 1u);  // (the order changes no value)
+                        bc[t][j] = kT * kRows + 6u * e;
+                        ext[e] = 6u * c;
+                    }
                 }
             }
-        }
-        // The lane's row of the LU factors; lane a == 0 solves the block.
+            // The lane's row of the LU factors.
+            const uint32_t br = row[t] / 6u;
 #pragma unroll
-        for (int q = 0; q < 3; ++q) cp_async8(lu + 36u * bo + 6u * a + 2 * q, D.lu + (size_t)br * 36u + 6u * a + 2 * q);
+            for (int q = 0; q < 3; ++q) cp_async8(lu[t] + 36u * bo + 6u * a + 2 * q, D.lu + (size_t)br * 36u + 6u * a + 2 * q);
+        }
     }
     cp_async_wait_all();
     __syncwarp();
-    const uint32_t sbo = min(lane, (uint32_t)kTeamWarpBrows - 1u);  // the block row that this lane solves
-    const bool solver = lane < (uint32_t)kTeamWarpBrows && warp < tw && br0 + warp * (uint32_t)kTeamWarpBrows + lane < br1;
-    const float *const slu = lu + 36u * sbo;
-    float *const srd = rd + 8u * sbo;
+    // The block row that this lane solves: lanes 0..4 the first part's, 5..9
+    // the second's.
+    const uint32_t st_part = min(lane / (uint32_t)kTeamWarpBrows, (uint32_t)kT - 1u);
+    const uint32_t sbo = lane < (uint32_t)(kT * kTeamWarpBrows) ? lane % (uint32_t)kTeamWarpBrows : 0u;
+    const bool solver = lane < (uint32_t)(kT * kTeamWarpBrows) && warp < tw && st_part < it.parts &&
+                        br0 + (st_part * tw + warp) * (uint32_t)kTeamWarpBrows + sbo < br1;
+    float *const slu0 = kT > 1 && st_part ? lu[kT - 1] : lu[0];
+    const float *const slu = slu0 + 36u * sbo;
+    float *const srd = slu0 + 36 * kTeamWarpBrows + 8u * sbo;
     if (solver) {
         float dlo = kDivLo;
 #pragma unroll
@@ -198,43 +229,61 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
     const uint32_t n_ext = 6u * S.ext;
 
     // y = (row) . xg: products rounded, added in index order; the operands of
-    // the next block are loaded before this block's products are added.
-    auto row_sum = [&]() {
-        float acc = 0.0f;
-        const float4 *B4 = b4;
-        const float2 *B2 = b2;
-        const float4 *X = reinterpret_cast<const float4 *>(xg);
-        float4 v, x;
-        float2 v2, x2;
-        if (nk) v = B4[0], v2 = B2[0], x = X[0], x2 = *reinterpret_cast<const float2 *>(X + 1);
-#pragma unroll 2
-        for (uint32_t j = 0; j < nk; ++j) {
-            const float2 q0 = mul2_rn(make_float2(v.x, v.y), make_float2(x.x, x.y));
-            const float2 q1 = mul2_rn(make_float2(v.z, v.w), make_float2(x.z, x.w));
-            const float2 q2 = mul2_rn(v2, x2);
-            if (j + 1 < nk) {
-                B4 += kTeamWarpRows, B2 += kTeamWarpRows, X += 2 * kTeamWarpBrows;
-                v = *B4, v2 = *B2, x = X[0], x2 = *reinterpret_cast<const float2 *>(X + 1);
-            }
-            acc = __fadd_rn(acc, q0.x);
-            acc = __fadd_rn(acc, q0.y);
-            acc = __fadd_rn(acc, q1.x);
-            acc = __fadd_rn(acc, q1.y);
-            acc = __fadd_rn(acc, q2.x);
-            acc = __fadd_rn(acc, q2.y);
+    // the next block are loaded before this block's products are added. Two
+    // rows' sums run side by side.
+    float ap[kT];
+    auto row_sums = [&]() {
+        const float4 *B4[kT], *X[kT];
+        const float2 *B2[kT];
+        float4 v[kT], xv[kT];
+        float2 v2[kT], x2[kT];
+#pragma unroll
+        for (int t = 0; t < kT; ++t) {
+            ap[t] = 0.0f;
+            B4[t] = b4[t];
+            B2[t] = b2[t];
+            X[t] = reinterpret_cast<const float4 *>(xg[t]);
+            if (nk[t]) v[t] = B4[t][0], v2[t] = B2[t][0], xv[t] = X[t][0], x2[t] = *reinterpret_cast<const float2 *>(X[t] + 1);
         }
-        return acc;
+#pragma unroll 2
+        for (uint32_t j = 0; j < (kT == 1 ? nk[0] : most); ++j) {
+            float2 q0[kT], q1[kT], q2[kT];
+#pragma unroll
+            for (int t = 0; t < kT; ++t) {
+                q0[t] = mul2_rn(make_float2(v[t].x, v[t].y), make_float2(xv[t].x, xv[t].y));
+                q1[t] = mul2_rn(make_float2(v[t].z, v[t].w), make_float2(xv[t].z, xv[t].w));
+                q2[t] = mul2_rn(v2[t], x2[t]);
+            }
+#pragma unroll
+            for (int t = 0; t < kT; ++t)
+                if (j + 1 < nk[t]) {
+                    B4[t] += kTeamWarpRows, B2[t] += kTeamWarpRows, X[t] += 2 * kTeamWarpBrows;
+                    v[t] = *B4[t], v2[t] = *B2[t], xv[t] = X[t][0], x2[t] = *reinterpret_cast<const float2 *>(X[t] + 1);
+                }
+#pragma unroll
+            for (int t = 0; t < kT; ++t) {
+                float s = ap[t];
+                s = __fadd_rn(s, q0[t].x);
+                s = __fadd_rn(s, q0[t].y);
+                s = __fadd_rn(s, q1[t].x);
+                s = __fadd_rn(s, q1[t].y);
+                s = __fadd_rn(s, q2[t].x);
+                s = __fadd_rn(s, q2[t].y);
+                ap[t] = kT == 1 || j < nk[t] ? s : ap[t];
+            }
+        }
     };
-    // z = U^-1 L^-1 r of the warp tile's blocks, one lane a block, in the
-    // order of block_jacobi.wgsl:93-126; r comes and z goes through S.z.
-    float *const wz = zx + 32u * min(warp, (uint32_t)kWarps - 1u);
+    // z = U^-1 L^-1 r of the warp tiles' blocks, one lane a block, in the order
+    // of block_jacobi.wgsl:93-126; r comes and z goes through zx.
+    float *const wz = zx + 32u * min(warp, (uint32_t)kTeamWarps - 1u);
     auto block_solve = [&]() {
-        wz[lane] = r;
+#pragma unroll
+        for (int t = 0; t < kT; ++t) wz[t * kRows + lane] = r[t];
         __syncwarp();
         if (solver) {
             float y[6], pr[6];
             bool ok = true;
-            float *const rz = wz + 6u * sbo;
+            float *const rz = wz + st_part * kRows + 6u * sbo;
             float l[36];
 #pragma unroll
             for (int q = 0; q < 9; ++q) {
@@ -269,18 +318,39 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
             }
         }
         __syncwarp();
-        return wz[lane];
+#pragma unroll
+        for (int t = 0; t < kT; ++t) z[t] = wz[t * kRows + lane];
     };
 
     uint32_t tag = st->epoch;
-    // This CTA's copy of the partials, and where lane l < copies stores copy l.
-    const uint32_t copies = team_copies(it.size);
-    const RedEntry *const red = D.red + (size_t)(it.rank % copies) * kRedEntries * it.size;
-    RedEntry *const out = D.red + (size_t)(lane % copies) * kRedEntries * it.size + it.rank;
+    // Published partials: one a part, or the sum of the CTA's two where the
+    // system never has one part a CTA. This CTA's copy of them; lane l stores to
+    // copy l % copies the CTA's partial l / copies.
+    const bool pairs = kT > 1 && D.team_pairs;
+    const uint32_t copies = team_copies(it.size), mine = lane / copies;
+    const uint32_t entries = pairs ? (it.size + 1u) / 2u : it.size, first = pairs ? it.rank / 2u : it.rank;
+    const bool publisher = mine < (pairs ? 1u : it.parts) && first + mine < entries;
+    const RedEntry *const red = D.red + (size_t)(it.rank / it.parts % copies) * kRedEntries * it.size;
+    RedEntry *const out = D.red + (size_t)(lane % copies) * kRedEntries * it.size + first + mine;
     unsigned long long *const zpk = D.zpk;
-    // The last two warps have no rows: they reduce. The first of them sums
-    // p.Ap and r.r and decides, the second sums r.z and forms beta.
-    const bool red_a = warp == (uint32_t)kWarps, red_b = warp == (uint32_t)kWarps + 1u;
+    // Sum over the system of one value a row, by one warp: the partials of all
+    // CTAs in one fixed order (a CTA that holds all adds its two the same way).
+    // Valid in lane 0.
+    auto all_reduce = [&](const double *v, uint32_t slot, uint32_t tag) {
+        double sums[kT];
+        part_sums<kT>(v, lane, sums);
+        double s = sums[0];
+        if (kT > 1 && (alone || pairs)) s += sums[kT - 1];  // (an absent part's is 0)
+        if (alone) return s;
+        s = __shfl_sync(kFull, s, 0);
+        if (kT > 1 && !pairs) {
+            const double second = __shfl_sync(kFull, sums[kT - 1], 0);
+            s = mine ? second : s;
+        }
+        if (publisher) st_entry(out + slot * it.size, s, tag);
+        __syncwarp();
+        return team_gather(&S.err, red + slot * it.size, entries, tag, w.sp, w.lim);
+    };
     if (red_a && lane == 0) {
         S.bb = st->bb;
         S.rr = S.pap = S.alpha_d = S.beta = 0.0;
@@ -324,29 +394,33 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
 #pragma unroll
             for (uint32_t q = 0; q < kBatch; ++q) {
                 const uint32_t i = b + q * step + tid;
-                if (i < n_ext) zx[32 * kWarps + i] = __uint_as_float((uint32_t)zin[q]);
+                if (i < n_ext) zx[kT * kRows + i] = __uint_as_float((uint32_t)zin[q]);
             }
         }
     };
-    // p = z + beta p of the lane's row and of its block columns (p = z when
+    // p = z + beta p of the lane's rows and of their block columns (p = z when
     // first). All operands come before the first store, which the compiler
     // could not move a load across.
     auto advance = [&](bool first, float bf) {
-        p = first ? z : __fadd_rn(__fmul_rn(p, bf), z);
+#pragma unroll
+        for (int t = 0; t < kT; ++t) {
+            p[t] = first ? z[t] : __fadd_rn(__fmul_rn(p[t], bf), z[t]);
 #pragma unroll 1
-        for (uint32_t j0 = 0; j0 < cols; j0 += kAhead) {
-            float *dst = xg + 8u * kTeamWarpBrows * j0 + a;
-            float pn[kAhead], zn[kAhead];
+            for (uint32_t j0 = 0; j0 < cols[t]; j0 += kAhead) {
+                float *dst = xg[t] + 8u * kTeamWarpBrows * j0 + a;
+                float pn[kAhead], zn[kAhead];
 #pragma unroll
-            for (int q = 0; q < kAhead / 4; ++q) {
-                const uint4 c = reinterpret_cast<const uint4 *>(bc + j0)[q];
-                zn[4 * q] = zx[c.x + a], zn[4 * q + 1] = zx[c.y + a], zn[4 * q + 2] = zx[c.z + a], zn[4 * q + 3] = zx[c.w + a];
+                for (int q = 0; q < kAhead / 4; ++q) {
+                    const uint4 c = reinterpret_cast<const uint4 *>(bc[t] + j0)[q];
+                    zn[4 * q] = zx[c.x + a], zn[4 * q + 1] = zx[c.y + a], zn[4 * q + 2] = zx[c.z + a], zn[4 * q + 3] = zx[c.w + a];
+                }
+#pragma unroll
+                for (int j = 0; j < kAhead; ++j) pn[j] = j0 + j < nk[t] ? dst[8u * kTeamWarpBrows * j] : 0.0f;
+#pragma unroll
+                for (int j = 0; j < kAhead; ++j)
+                    if (j0 + j < nk[t])
+                        dst[8u * kTeamWarpBrows * j] = first ? zn[j] : __fadd_rn(__fmul_rn(pn[j], bf), zn[j]);
             }
-#pragma unroll
-            for (int j = 0; j < kAhead; ++j) pn[j] = j0 + j < nk ? dst[8u * kTeamWarpBrows * j] : 0.0f;
-#pragma unroll
-            for (int j = 0; j < kAhead; ++j)
-                if (j0 + j < nk) dst[8u * kTeamWarpBrows * j] = first ? zn[j] : __fadd_rn(__fmul_rn(pn[j], bf), zn[j]);
         }
         __syncwarp();
     };
@@ -359,27 +433,25 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
     uint32_t done = 0;
     for (;;) {
         ++tag;
-        float ap = 0.0f;
-        if (!red_a && !red_b) {
-            ap = row_sum();
+        if (rows) {
+            row_sums();
             __syncwarp();
         }
         if (init) {
-            const float bi = on ? __ldg(D.b + row) : 0.0f;
-            r = __fsub_rn(bi, ap);
-            if (!red_a && !red_b) v0[tid] = (double)bi * (double)bi;
+            if (rows)
+#pragma unroll
+                for (int t = 0; t < kT; ++t) {
+                    const float bi = on[t] ? __ldg(D.b + row[t]) : 0.0f;
+                    r[t] = __fsub_rn(bi, ap[t]);
+                    v0[t * kRows + tid] = (double)bi * (double)bi;
+                }
         } else {
-            if (!red_a && !red_b) v0[tid] = (double)p * (double)ap;
+            if (rows)
+#pragma unroll
+                for (int t = 0; t < kT; ++t) v0[t * kRows + tid] = (double)p[t] * (double)ap[t];
             __syncthreads();
             if (red_a) {
-                const double rz_old = S.rz;
-                double pap = cta_sum<kWarps>(v0, lane);
-                if (!alone) {
-                    pap = __shfl_sync(kFull, pap, 0);
-                    if (lane < copies) st_entry(out, pap, tag);
-                    __syncwarp();
-                    pap = team_gather(&S.err, red, it.size, tag, w.sp, w.lim);
-                }
+                const double rz_old = S.rz, pap = all_reduce(v0, 0, tag);
                 if (lane == 0) {
                     const double alpha = quotient(rz_old, pap);
                     S.rz_old = rz_old;
@@ -392,27 +464,26 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
             const uint2 al2 = S.alpha;
             if (!al2.y) break;
             const float al = __uint_as_float(al2.x), ma = -al;
-            x = __fadd_rn(x, __fmul_rn(al, p));
-            r = __fadd_rn(r, __fmul_rn(ma, ap));
-            if (!on) r = 0.0f;
+            if (rows)
+#pragma unroll
+                for (int t = 0; t < kT; ++t) {
+                    x[t] = __fadd_rn(x[t], __fmul_rn(al, p[t]));
+                    r[t] = __fadd_rn(r[t], __fmul_rn(ma, ap[t]));
+                    if (!on[t]) r[t] = 0.0f;
+                }
         }
-        if (!red_a && !red_b) {
-            z = block_solve();
-            if (on && !alone) st_packet(zpk + row, z, tag);
-            if (!init) v0[tid] = (double)r * (double)r;
-            v1[tid] = (double)r * (double)z;
+        if (rows) {
+            block_solve();
+#pragma unroll
+            for (int t = 0; t < kT; ++t) {
+                if (on[t] && !alone) st_packet(zpk + row[t], z[t], tag);
+                if (!init) v0[t * kRows + tid] = (double)r[t] * (double)r[t];
+                v1[t * kRows + tid] = (double)r[t] * (double)z[t];
+            }
         }
         __syncthreads();
         if (red_a || red_b) {
-            const double *v = red_a ? v0 : v1;
-            const uint32_t slot = (red_a ? 1u : 2u) * it.size;
-            double sum = cta_sum<kWarps>(v, lane);
-            if (!alone) {
-                sum = __shfl_sync(kFull, sum, 0);
-                if (lane < copies) st_entry(out + slot, sum, tag);
-                __syncwarp();
-                sum = team_gather(&S.err, red + slot, it.size, tag, w.sp, w.lim);
-            }
+            const double sum = all_reduce(red_a ? v0 : v1, red_a ? 1u : 2u, tag);
             if (lane == 0 && red_b) {
                 const double beta = quotient(sum, S.rz);
                 S.beta = beta;
@@ -449,7 +520,7 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
         }
         __syncthreads();
         if (!S.go) break;
-        if (!red_a && !red_b) advance(init, S.beta_f);
+        if (rows) advance(init, S.beta_f);
         if (!init && ++done >= limit) break;
         init = false;
     }
@@ -458,12 +529,14 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
         if (tid == 0) atomicOr(&w.sp->error, kErrTeamWait);
         return;
     }
-    if (on) {
-        D.x[row] = x;
-        D.r[row] = r;
-        D.z[row] = z;
-        D.p[row] = p;
-    }
+#pragma unroll
+    for (int t = 0; t < kT; ++t)
+        if (on[t]) {
+            D.x[row[t]] = x[t];
+            D.r[row[t]] = r[t];
+            D.z[row[t]] = z[t];
+            D.p[row[t]] = p[t];
+        }
     if (lead && red_a && lane == 0) {
         const bool running = S.status == ST_RUNNING, none = S.iter == 0;  // none: stopped before the first iteration
         st->bb = S.bb;
@@ -484,8 +557,8 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
     }
 }
 
-template <int kWarps>
-__global__ void __launch_bounds__(team_threads(kWarps), 1)
+template <int kT>
+__global__ void __launch_bounds__(kTeamThreads, 1)
     k_team(const SysDesc *__restrict__ sys, StepParams *sp, const TeamItem *__restrict__ items,
            const uint32_t *__restrict__ item_off, uint32_t limit) {
     static_assert(offsetof(TeamShared, v) <= 512, "fixed shared memory");
@@ -498,7 +571,7 @@ __global__ void __launch_bounds__(team_threads(kWarps), 1)
     const uint32_t i1 = item_off[blockIdx.x + 1];
     for (uint32_t i = item_off[blockIdx.x]; i < i1; ++i) {
         const TeamItem it = items[i];
-        team_system_bsr6<kWarps>(sys[it.sys], it, limit, S, smem + team_fixed_bytes(kWarps), w);
+        team_system_bsr6<kT>(sys[it.sys], it, limit, S, smem + team_fixed_bytes(kT), w);
         __syncthreads();
         if (S.err) return;  // every CTA's later waits would run out as well
     }
@@ -506,8 +579,6 @@ __global__ void __launch_bounds__(team_threads(kWarps), 1)
 
 }  // namespace
 
-const void *team_kernel(int warps) {
-    return warps <= kTeamWarps ? (const void *)k_team<kTeamWarps> : (const void *)k_team<kTeamWarpsWide>;
-}
+const void *team_kernel(int parts) { return parts == 1 ? (const void *)k_team<1> : (const void *)k_team<2>; }
 
 }  // namespace wsb

@@ -141,8 +141,9 @@ struct SysDesc {
     SysState *st;
     double *history;                   // hist_cap entries or null
     uint32_t algo;                     // Algo
-    uint32_t team_warps;               // k_team: warp tiles a CTA holds
-    uint32_t team_ext;                 // k_team: most blocks a CTA holds
+    uint32_t team_warps;               // k_team: warp tiles of a part
+    uint32_t team_ext[2];              // k_team: most blocks outside a CTA's rows that it multiplies with, one or two parts a CTA
+    uint32_t team_pairs;               // k_team: always two parts a CTA, one partial for both
     float *s;                          // single reduction: s = A p (by recurrence)
     unsigned long long *zpk;           // k_team: z of each row with the tag of its all-reduce (value low, tag high)
     float *p2;                         // k_stream: the other buffer of p
@@ -151,10 +152,10 @@ struct SysDesc {
     RedEntry *red;                     // k_team, k_stream: published partials (team_red_entries)
 };
 
-// One CTA's part of one system in a k_team launch: member `rank` of the `size`
-// CTAs that share system `sys`.
+// One CTA's share of one system in a k_team launch: `parts` of the system's
+// `size` parts (fewer at its end), from part `rank`.
 struct TeamItem {
-    uint32_t sys, rank, size, pad;
+    uint32_t sys, rank, size, parts;
 };
 
 // Bits of StepParams::error. The wait bits mean a bounded mbarrier wait ran
