@@ -165,7 +165,13 @@ struct Engine::Slot {
     // one and of two parts, the most blocks a CTA multiplies and the most bytes
     // of its warp tiles (0: two parts do not fit).
     uint32_t team = 0, team_warps = 0, team_ext[2] = {0, 0}, team_tiles[2] = {0, 0};
+    // CSR: its warp tiles (first rows, first blocks, offsets of their columns'
+    // places) and the columns outside a part that the plan has room for.
+    bool team_csr = false;
+    std::vector<uint32_t> tile_row, tile_blk, tile_off;
+    uint32_t ext_cap = 0;
     uint32_t team_smem(uint32_t launch_parts, uint32_t parts) const {
+        if (team_csr) return (uint32_t)team_fixed_bytes(1) + team_csr_z_bytes(team_ext[0]) + team_tiles[0];
         return (uint32_t)team_fixed_bytes(launch_parts) + team_z_bytes(launch_parts, team_ext[parts - 1]) + team_tiles[parts - 1];
     }
     // k_stream (stream > 0): CTAs; its second buffer of p and partials.
@@ -205,7 +211,8 @@ Engine::Engine(Context *ctx, cudaStream_t stream) : ctx_(ctx), stream_(stream) {
     max_grid_b_ = std::max(1, occ_b) * std::max(1, ctx->sm_count);
     max_grid_c_ = std::max(1, occ_c) * std::max(1, ctx->sm_count);
     for (int parts : {1, 2})
-        cudaFuncSetAttribute(team_kernel(parts), cudaFuncAttributeMaxDynamicSharedMemorySize, kTeamSmemMax);
+        cudaFuncSetAttribute(team_kernel(parts, false), cudaFuncAttributeMaxDynamicSharedMemorySize, kTeamSmemMax);
+    cudaFuncSetAttribute(team_kernel(1, true), cudaFuncAttributeMaxDynamicSharedMemorySize, kTeamSmemMax);
     for (bool sr : {false, true})
         cudaFuncSetAttribute(stream_kernel(sr), cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmem);
     const char *loop_env = getenv("WSB_LOOP");
@@ -228,8 +235,10 @@ Engine::~Engine() {
     cudaFree(d_state_);
     cudaFree(d_sp_);
     cudaFree(d_work_);
-    cudaFree(d_team_);
-    cudaFreeHost(h_team_);
+    for (TeamLists &l : team_lists_) {
+        cudaFree(l.dev);
+        cudaFreeHost(l.host);
+    }
     cudaFreeHost(h_sys_);
     cudaFreeHost(h_state_);
     cudaFreeHost(h_sp_);
@@ -298,9 +307,9 @@ int Engine::push_changes() {
 // enough blocks for the shared memory of one CTA an SM in shared memory.
 void Engine::team_plan(Slot *sl) const {
     const MatA &A = *sl->A;
-    if (!team_on_ || !use_graph_ || A.layout != LAYOUT_BSR6 || A.n == 0 || sl->M->nb != A.n / 6 ||
-        sl->cfg.algorithm != WSB_ALG_CLASSIC)
-        return;
+    if (!team_on_ || !use_graph_ || A.n == 0 || sl->cfg.algorithm != WSB_ALG_CLASSIC) return;
+    if (A.layout == LAYOUT_CSR) return team_plan_rows(sl);
+    if (A.layout != LAYOUT_BSR6 || sl->M->nb != A.n / 6) return;
     const uint32_t nbr = A.n / 6, tiles = (nbr + kTeamWarpBrows - 1) / kTeamWarpBrows, sms = (uint32_t)ctx_->sm_count;
     if (tiles > 2 * sms * kTeamWarps) return;
     std::vector<uint32_t> cols(tiles, 0u);  // blocks of each warp tile's longest block row
@@ -332,6 +341,83 @@ void Engine::team_plan(Slot *sl) const {
             sl->team = size;
             return;
         }
+}
+
+// The same for a CSR system whose blocks have 1 to 6 rows: warp tiles of whole
+// blocks, one part a CTA, and room for the columns outside a part's rows.
+// Whether they fit is found out by the plan on the device (finish_team_plan).
+void Engine::team_plan_rows(Slot *sl) const {
+    const MatA &A = *sl->A;
+    const std::vector<uint32_t> &bs = sl->M->h_bs;
+    const uint32_t nb = sl->M->nb, sms = (uint32_t)ctx_->sm_count;
+    if (bs.size() != (size_t)nb + 1 || nb == 0 || bs[0] != 0 || bs[nb] != A.n || A.n > 32u * sms * kTeamWarps) return;
+    std::vector<uint32_t> row{0}, blk{0}, off{0}, bytes;
+    auto close = [&](uint32_t end, uint32_t end_blk) {
+        uint32_t cols = 0;
+        for (uint32_t r = row.back(); r < end; ++r) cols = std::max(cols, A.h_rows[r + 1] - A.h_rows[r]);
+        if (cols > (uint32_t)kTeamSmemMax / 192u) return false;
+        bytes.push_back(team_csr_tile_bytes(cols, end_blk - blk.back()));
+        off.push_back(off.back() + 32u * ((cols + 3u) & ~3u));
+        row.push_back(end);
+        blk.push_back(end_blk);
+        return true;
+    };
+    for (uint32_t k = 0; k < nb; ++k) {
+        if (bs[k + 1] <= bs[k] || bs[k + 1] - bs[k] > 6u) return;
+        if (bs[k + 1] - row.back() > 32u && !close(bs[k], k)) return;
+    }
+    if (!close(A.n, nb)) return;
+    const uint32_t tiles = (uint32_t)bytes.size();
+    for (uint32_t w = kTeamWarps; w >= 1; --w) {
+        const uint32_t size = (tiles + w - 1) / w;
+        if (size > sms) return;
+        uint64_t most = 0;
+        for (uint32_t c = 0; c < size; ++c) {
+            uint64_t sum = 0;
+            for (uint32_t q = c * w; q < std::min((c + 1) * w, tiles); ++q) sum += bytes[q];
+            most = std::max(most, sum);
+        }
+        // A part multiplies with at most its rows' places, and usually far
+        // fewer columns outside: 2,048 of them must fit.
+        const uint64_t used = (uint64_t)team_fixed_bytes(1) + team_csr_z_bytes(0) + most;
+        const uint32_t need = std::min(A.n, kTeamMaxExt / 2);
+        if (used + 12ull * need + 16u > (uint64_t)kTeamSmemMax) continue;
+        sl->team_csr = true;
+        sl->ext_cap = (uint32_t)std::min<uint64_t>(std::min(A.n, kTeamMaxExt), (kTeamSmemMax - 16u - used) / 12u);
+        sl->team = size;
+        sl->team_warps = w;
+        sl->team_tiles[0] = (uint32_t)most;
+        sl->tile_row = std::move(row);
+        sl->tile_blk = std::move(blk);
+        sl->tile_off = std::move(off);
+        return;
+    }
+}
+
+// Where the columns of a CSR system's nonzeros are in its CTAs' shared memory,
+// once for all its solves; a system with too many columns outside a part goes
+// to the loop kernels.
+int Engine::finish_team_plan(Slot *sl, SysDesc *d, uint32_t *tiles_mem, uint32_t *count) {
+    const size_t nt = sl->tile_row.size(), words = 3 * nt;
+    std::vector<uint32_t> h(words);
+    std::copy(sl->tile_row.begin(), sl->tile_row.end(), h.begin());
+    std::copy(sl->tile_blk.begin(), sl->tile_blk.end(), h.begin() + nt);
+    std::copy(sl->tile_off.begin(), sl->tile_off.end(), h.begin() + 2 * nt);
+    WSB_CUDA_TRY(ctx_, cudaMemcpyAsync(tiles_mem, h.data(), sizeof(uint32_t) * words, cudaMemcpyHostToDevice, stream_));
+    d->n_tiles = (uint32_t)nt - 1;
+    d->ext_cap = sl->ext_cap;
+    d->tile_row = tiles_mem;
+    d->tile_blk = tiles_mem + nt;
+    d->tile_off = tiles_mem + 2 * nt;
+    d->ext_count = count;
+    WSB_CUDA_TRY(ctx_, team_plan_csr(*d, count, sl->team, stream_));
+    launches_ += 1;
+    uint32_t found[2] = {0, 0};
+    WSB_CUDA_TRY(ctx_, cudaMemcpyAsync(found, count + sl->team, sizeof found, cudaMemcpyDeviceToHost, stream_));
+    WSB_CUDA_TRY(ctx_, cudaStreamSynchronize(stream_));
+    sl->team_ext[0] = found[1];
+    if (found[0]) sl->team = 0;
+    return WSB_OK;
 }
 
 // Whether k_stream iterates a system that k_team does not: BSR6, more block
@@ -397,7 +483,7 @@ int Engine::add(const MatA *A, const Precond *M, const SolveCfg &cfg, uint32_t *
     sl->hist_cap = std::min<uint64_t>(cfg.hist_cap, max_hist);
     team_plan(sl.get());
     stream_plan(sl.get());
-    size_t off[15], tot = 0;
+    size_t off[19], tot = 0;
     auto take = [&](int k, size_t bytes) {
         off[k] = tot;
         tot += a256(bytes);
@@ -417,6 +503,11 @@ int Engine::add(const MatA *A, const Precond *M, const SolveCfg &cfg, uint32_t *
     take(12, sl->team ? sizeof(unsigned long long) * n : 0);  // z packets
     take(13, team_red_bytes(sl->red_ctas()));                 // published partials
     take(14, sl->stream && cfg.algorithm == WSB_ALG_CLASSIC ? vf : 0);  // the other buffer of p
+    const size_t tile_words = sl->team_csr ? 3 * sl->tile_row.size() : 0;
+    take(15, sizeof(uint32_t) * tile_words);  // CSR: warp tiles
+    take(16, sl->team_csr ? sizeof(uint16_t) * sl->tile_off.back() : 0);                   // places of the columns
+    take(17, sl->team_csr ? sizeof(uint32_t) * (size_t)sl->team * sl->ext_cap : 0);        // columns outside
+    take(18, sl->team_csr ? sizeof(uint32_t) * (sl->team + 2) : 0);                        // their counts
     void *mem = nullptr;
     cudaError_t e = cudaMallocAsync(&mem, tot, stream_);
     if (e != cudaSuccess)
@@ -483,6 +574,13 @@ int Engine::add(const MatA *A, const Precond *M, const SolveCfg &cfg, uint32_t *
     d.algo = (uint32_t)cfg.algorithm;
     d.s = sl->s;
     d.team_warps = sl->team_warps;
+    d.tile_idx = (uint16_t *)(base + off[16]);
+    d.ext_cols = (uint32_t *)(base + off[17]);
+    if (sl->team_csr &&
+        (rc = finish_team_plan(sl.get(), &d, (uint32_t *)(base + off[15]), (uint32_t *)(base + off[18])))) {
+        cudaFreeAsync(mem, stream_);
+        return rc;
+    }
     d.team_ext[0] = sl->team_ext[0];
     d.team_ext[1] = sl->team_ext[1];
     d.team_pairs = sl->team > (uint32_t)ctx_->sm_count;
@@ -840,7 +938,7 @@ int Engine::finish_slot(uint32_t s, int status) {
 // root of its rows in iterations; the time of one is fitted to measured ones.
 // Every CTA's list is in the order in which systems start, so no two systems
 // wait for each other whatever the times turn out to be.
-int Engine::launch_team(const std::vector<uint32_t> &ids, uint32_t limit) {
+int Engine::launch_team(const std::vector<uint32_t> &ids, bool csr, uint32_t limit) {
     if (ids.empty()) return WSB_OK;
     const uint32_t sms = (uint32_t)std::max(1, ctx_->sm_count);
     struct Run {
@@ -895,7 +993,7 @@ int Engine::launch_team(const std::vector<uint32_t> &ids, uint32_t limit) {
     };
     Run run = simulate(false);
     const bool crowded = std::any_of(run.lists.begin(), run.lists.end(), [](const auto &l) { return l.size() > 1; });
-    if (crowded) {
+    if (crowded && !csr) {
         Run pairs = simulate(true);
         if (pairs.end < run.end) run = std::move(pairs);
     }
@@ -904,31 +1002,31 @@ int Engine::launch_team(const std::vector<uint32_t> &ids, uint32_t limit) {
     size_t items = 0;
     for (const auto &l : lists) items += l.size();
     const size_t head = ((size_t)grid + 1 + 3) & ~size_t(3), words = head + 4 * items;
-    if (words > team_cap_) {
+    TeamLists &mem = team_lists_[csr];  // (a step may launch both kernels)
+    if (words > mem.cap) {
         WSB_CUDA_TRY(ctx_, cudaStreamSynchronize(stream_));
-        cudaFree(d_team_);
-        cudaFreeHost(h_team_);
-        d_team_ = h_team_ = nullptr;
-        team_cap_ = 0;
+        cudaFree(mem.dev);
+        cudaFreeHost(mem.host);
+        mem = TeamLists();
         const size_t nc = std::max<size_t>(1024, 2 * words);
-        WSB_CUDA_TRY(ctx_, cudaMalloc(&d_team_, sizeof(uint32_t) * nc));
-        WSB_CUDA_TRY(ctx_, cudaMallocHost(&h_team_, sizeof(uint32_t) * nc));
-        team_cap_ = nc;
+        WSB_CUDA_TRY(ctx_, cudaMalloc(&mem.dev, sizeof(uint32_t) * nc));
+        WSB_CUDA_TRY(ctx_, cudaMallocHost(&mem.host, sizeof(uint32_t) * nc));
+        mem.cap = nc;
     }
-    TeamItem *it = reinterpret_cast<TeamItem *>(h_team_ + head);
+    TeamItem *it = reinterpret_cast<TeamItem *>(mem.host + head);
     uint32_t at = 0;
     for (uint32_t c = 0; c < grid; ++c) {
-        h_team_[c] = at;
+        mem.host[c] = at;
         for (const TeamItem &q : lists[c]) it[at++] = q;
     }
-    h_team_[grid] = at;
-    WSB_CUDA_TRY(ctx_, cudaMemcpyAsync(d_team_, h_team_, sizeof(uint32_t) * words, cudaMemcpyHostToDevice, stream_));
+    mem.host[grid] = at;
+    WSB_CUDA_TRY(ctx_, cudaMemcpyAsync(mem.dev, mem.host, sizeof(uint32_t) * words, cudaMemcpyHostToDevice, stream_));
     const SysDesc *dsys = d_sys_;
     StepParams *dsp = d_sp_;
-    const TeamItem *ditems = reinterpret_cast<const TeamItem *>(d_team_ + head);
-    const uint32_t *doff = d_team_;
+    const TeamItem *ditems = reinterpret_cast<const TeamItem *>(mem.dev + head);
+    const uint32_t *doff = mem.dev;
     void *args[] = {&dsys, &dsp, &ditems, &doff, &limit};
-    WSB_CUDA_TRY(ctx_, cudaLaunchCooperativeKernel(team_kernel((int)run.parts), dim3(grid), dim3(kTeamThreads), args,
+    WSB_CUDA_TRY(ctx_, cudaLaunchCooperativeKernel(team_kernel((int)run.parts, csr), dim3(grid), dim3(kTeamThreads), args,
                                                    (size_t)run.smem, stream_));
     launches_ += 1;
     return WSB_OK;
@@ -1041,10 +1139,10 @@ int Engine::step(uint32_t loop_limit, bool *any_left, uint32_t team_limit) {
     if ((rc = push_changes())) return rc;
     // k_team forms its systems' first residual itself.
     init.erase(std::remove_if(init.begin(), init.end(), [&](uint32_t s) { return slots_[s]->team != 0; }), init.end());
-    std::vector<uint32_t> team, streamed;
+    std::vector<uint32_t> team, team_csr, streamed;
     for (uint32_t s = 0; s < slots_.size(); ++s) {
         if (!slots_[s] || slots_[s]->phase != Slot::RUNNING) continue;
-        if (slots_[s]->team) team.push_back(s);
+        if (slots_[s]->team) (slots_[s]->team_csr ? team_csr : team).push_back(s);
         if (slots_[s]->stream) streamed.push_back(s);
     }
     uint32_t starting = 0;  // systems of the loop kernels that start
@@ -1076,7 +1174,8 @@ int Engine::step(uint32_t loop_limit, bool *any_left, uint32_t team_limit) {
     h_sp_->loop_count = 0;
     h_sp_->loop_limit = limit;
     WSB_CUDA_TRY(ctx_, cudaMemcpyAsync(d_sp_, h_sp_, sizeof(StepParams), cudaMemcpyHostToDevice, stream_));
-    if ((rc = launch_team(team, std::max<uint32_t>(1, team_limit)))) return rc;
+    if ((rc = launch_team(team, false, std::max<uint32_t>(1, team_limit)))) return rc;
+    if ((rc = launch_team(team_csr, true, std::max<uint32_t>(1, team_limit)))) return rc;
     if (!init.empty()) {
         const uint32_t ga = std::min<uint32_t>(h_sp_->w_init_a, (uint32_t)max_grid_a_);
         const uint32_t gb = std::min<uint32_t>(h_sp_->w_init_b, (uint32_t)max_grid_b_);

@@ -162,9 +162,11 @@ class Engine {
     int read_states(const std::vector<uint32_t> &slots);
     int finish_slot(uint32_t slot, int status);
     void team_plan(Slot *sl) const;
+    void team_plan_rows(Slot *sl) const;
+    int finish_team_plan(Slot *sl, SysDesc *d, uint32_t *tiles, uint32_t *count);
     void stream_plan(Slot *sl) const;
     int launch_stream(const std::vector<uint32_t> &slots, uint32_t limit);
-    int launch_team(const std::vector<uint32_t> &slots, uint32_t limit);
+    int launch_team(const std::vector<uint32_t> &slots, bool csr, uint32_t limit);
 
     Context *ctx_;
     cudaStream_t stream_;
@@ -184,8 +186,13 @@ class Engine {
     bool desc_dirty_ = false, state_dirty_ = false;  // host mirrors changed since the last upload
     bool use_graph_ = true;   // WSB_LOOP=launch: plain launches + host polling
     bool team_on_ = true;     // small systems take k_team
-    uint32_t *d_team_ = nullptr, *h_team_ = nullptr;  // k_team lists: item offsets, then items
-    size_t team_cap_ = 0;                             // words of d_team_ / h_team_
+    // Lists of the k_team launches (BSR6, CSR) of a step: item offsets, then
+    // items. The host's is rewritten by the next step, after its sync.
+    struct TeamLists {
+        uint32_t *dev = nullptr, *host = nullptr;
+        size_t cap = 0;  // words
+    };
+    TeamLists team_lists_[2];
     cudaGraph_t graph_ = nullptr;
     cudaGraphExec_t exec_ = nullptr;
     uint32_t graph_grid_a_ = 0, graph_grid_b_ = 0, graph_grid_c_ = 0;

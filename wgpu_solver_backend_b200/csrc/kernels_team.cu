@@ -97,17 +97,21 @@ __device__ __forceinline__ void part_sums(const double *v, uint32_t lane, double
 }
 
 // One system, this CTA's rows, up to `limit` iterations.
-template <int kT>
-__device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamItem it, uint32_t limit, TeamShared &S,
+template <int kT, bool kCsr>
+__device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it, uint32_t limit, TeamShared &S,
                                                  char *dyn, const WaitCtl &w) {
+    static_assert(!kCsr || kT == 1, "CSR: one part a CTA");
     constexpr int kAhead = 8;  // block columns a lane handles at once
     constexpr uint32_t kRows = 32u * kTeamWarps;  // places for the rows of a part
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     SysState *st = D.st;
     if (!st->active) return;
-    const uint32_t nbr = D.n / 6u, tw = D.team_warps, part_brows = tw * (uint32_t)kTeamWarpBrows;
+    const uint32_t tw = D.team_warps;
     const bool lead = it.rank == 0, alone = it.parts >= it.size;
-    const uint32_t br0 = min(it.rank * part_brows, nbr), br1 = min(br0 + it.parts * part_brows, nbr);
+    // The CTA's block rows (BSR6) or rows (CSR).
+    const uint32_t part_brows = tw * (uint32_t)kTeamWarpBrows, tile0 = it.rank * tw;
+    const uint32_t br0 = kCsr ? D.tile_row[tile0] : min(it.rank * part_brows, D.n / 6u);
+    const uint32_t br1 = kCsr ? D.tile_row[min(tile0 + tw, D.n_tiles)] : min(br0 + it.parts * part_brows, D.n / 6u);
     const bool fresh = st->fresh != 0;
     // The warps with rows; the last two warps have none: they reduce. The
     // first of them sums p.Ap and r.r and decides, the second sums r.z and
@@ -118,16 +122,25 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
     bool on[kT];
     uint32_t row[kT], k0[kT], nk[kT], cols[kT], most = 0;  // cols: most blocks of a block row of the warp tile
     float x[kT], r[kT], z[kT], p[kT];
+    // CSR: the warp tile's first row and block, its rows and blocks.
+    uint32_t row0 = 0, blk0 = 0, n_rows = 0, n_blk = 0;
+    if (kCsr && warp < tw && tile0 + warp < D.n_tiles) {
+        row0 = D.tile_row[tile0 + warp];
+        blk0 = D.tile_blk[tile0 + warp];
+        n_rows = D.tile_row[tile0 + warp + 1u] - row0;
+        n_blk = D.tile_blk[tile0 + warp + 1u] - blk0;
+    }
 #pragma unroll
     for (int t = 0; t < kT; ++t) {
         const uint32_t br = br0 + (t * tw + warp) * (uint32_t)kTeamWarpBrows + bo;
-        on[t] = lane < (uint32_t)kTeamWarpRows && warp < tw && (uint32_t)t < it.parts && br < br1;
-        row[t] = on[t] ? 6u * br + a : 0u;
+        on[t] = kCsr ? lane < n_rows : lane < (uint32_t)kTeamWarpRows && warp < tw && (uint32_t)t < it.parts && br < br1;
+        row[t] = !on[t] ? 0u : kCsr ? row0 + lane : 6u * br + a;
         k0[t] = nk[t] = 0;
         x[t] = r[t] = z[t] = p[t] = 0.0f;
         if (on[t]) {
-            k0[t] = D.brow_ptr[br];
-            nk[t] = D.brow_ptr[br + 1] - k0[t];
+            const uint32_t *ptr = kCsr ? D.row_ptr + row[t] : D.brow_ptr + br;
+            k0[t] = ptr[0];
+            nk[t] = ptr[1] - k0[t];
             x[t] = D.x[row[t]];
             if (!fresh) {
                 r[t] = D.r[row[t]];
@@ -137,7 +150,7 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
         }
         cols[t] = __reduce_max_sync(kFull, nk[t]);
         most = max(most, cols[t]);
-        if (lane == 0 && rows) S.bytes[t * kTeamWarps + warp] = team_tile_bytes(cols[t]);
+        if (lane == 0 && rows) S.bytes[t * kTeamWarps + warp] = kCsr ? team_csr_tile_bytes(cols[t], n_blk) : team_tile_bytes(cols[t]);
     }
     double *const v0 = S.v, *const v1 = S.v + kT * kRows;
     if (rows)
@@ -151,20 +164,60 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
     // short division, and for block j of its block rows, lane by lane (no bank
     // conflicts), the row's first four values, its last two, p at the block's
     // columns, and where z of the block's columns is.
+    // CSR: z and p of the CTA's rows and of the columns outside, and those
+    // columns; then for each warp tile the factors (absent rows of a block are
+    // rows of I), and four by four the rows' values and the places of their
+    // columns in z and p.
     const uint32_t most_ext = D.team_ext[it.parts - 1u];
     float *const zx = reinterpret_cast<float *>(dyn);
-    uint32_t *const ext = reinterpret_cast<uint32_t *>(zx + kT * kRows + 6u * most_ext);
-    char *const tiles = dyn + team_z_bytes(kT, most_ext);
+    float *const px = zx + kRows + most_ext;  // (CSR)
+    uint32_t *const ext = reinterpret_cast<uint32_t *>(kCsr ? px + kRows + most_ext : zx + kT * kRows + 6u * most_ext);
+    char *const tiles = dyn + (kCsr ? team_csr_z_bytes(most_ext) : team_z_bytes(kT, most_ext));
+    const float4 *val4 = nullptr;  // (CSR)
+    const ushort4 *idx4 = nullptr;
     // (cols == 0: a warp tile without rows; it touches none of this.)
     float *lu[kT], *xg[kT];
     float4 *b4[kT];
     float2 *b2[kT];
     uint32_t *bc[kT];
-#pragma unroll
-    for (int t = 0; t < kT; ++t) {
+    auto tile_at = [&](int t) {
         uint32_t before = 0;
         for (uint32_t q = 0; q < t * tw + min(warp, tw); ++q) before += S.bytes[q < tw ? q : kTeamWarps + q - tw];
-        char *mine = tiles + before;
+        return tiles + before;
+    };
+    auto load_csr = [&]() {
+        char *const mine = tile_at(0);
+        lu[0] = reinterpret_cast<float *>(mine);
+        const uint32_t colp = (cols[0] + 3u) & ~3u;
+        float *const val = reinterpret_cast<float *>(mine + n_blk * (uint32_t)kTeamBlockLu);
+        uint16_t *const idx = reinterpret_cast<uint16_t *>(val + 32u * colp);
+        val4 = reinterpret_cast<const float4 *>(val) + lane;
+        idx4 = reinterpret_cast<const ushort4 *>(idx) + lane;
+        if (n_rows) {
+            if (on[0]) px[32u * warp + lane] = fresh ? x[0] : p[0];
+#pragma unroll 1
+            for (uint32_t j = 0; j < nk[0]; ++j) cp_async4(val + 4u * (32u * (j >> 2) + lane) + (j & 3u), D.val + k0[0] + j);
+            const char *from = reinterpret_cast<const char *>(D.tile_idx + D.tile_off[tile0 + warp]);
+            for (uint32_t q = lane; q < 4u * colp; q += 32u) cp_async16(reinterpret_cast<char *>(idx) + 16u * q, from + 16u * q);
+            if (lane < n_blk) {
+                const uint32_t m = D.bstart[blk0 + lane + 1u] - D.bstart[blk0 + lane];
+#pragma unroll
+                for (uint32_t q = 0; q < 36u; ++q)
+                    lu[0][36u * lane + q] =
+                        q / 6u < m && q % 6u < m ? D.lu[36u * (size_t)(blk0 + lane) + q] : q % 7u == 0 ? 1.0f : 0.0f;
+            }
+        }
+        // The columns outside, their first entries of p (x0 when fresh).
+        const uint32_t n = D.ext_count[it.rank];
+        if (tid == 0) S.ext = n;
+        for (uint32_t i = tid; i < n; i += (uint32_t)kTeamThreads) {
+            const uint32_t c = D.ext_cols[(size_t)it.rank * D.ext_cap + i];
+            ext[i] = c;
+            px[kRows + i] = (fresh ? D.x : D.p)[c];
+        }
+    };
+    auto load_bsr = [&](int t) {
+        char *mine = tile_at(t);
         lu[t] = reinterpret_cast<float *>(mine);
         mine += kTeamLuBytes;
         const uint32_t colp = (cols[t] + 7u) & ~7u;
@@ -203,18 +256,26 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
 #pragma unroll
             for (int q = 0; q < 3; ++q) cp_async8(lu[t] + 36u * bo + 6u * a + 2 * q, D.lu + (size_t)br * 36u + 6u * a + 2 * q);
         }
-    }
+    };
+    if (kCsr) load_csr();
+    else
+#pragma unroll
+        for (int t = 0; t < kT; ++t) load_bsr(t);
     cp_async_wait_all();
     __syncwarp();
-    // The block row that this lane solves: lanes 0..4 the first part's, 5..9
-    // the second's.
-    const uint32_t st_part = min(lane / (uint32_t)kTeamWarpBrows, (uint32_t)kT - 1u);
-    const uint32_t sbo = lane < (uint32_t)(kT * kTeamWarpBrows) ? lane % (uint32_t)kTeamWarpBrows : 0u;
-    const bool solver = lane < (uint32_t)(kT * kTeamWarpBrows) && warp < tw && st_part < it.parts &&
-                        br0 + (st_part * tw + warp) * (uint32_t)kTeamWarpBrows + sbo < br1;
+    // The block that this lane solves (BSR6: lanes 0..4 the first part's, 5..9
+    // the second's), its rows, and the first of them in the warp tile.
+    const uint32_t st_part = kCsr ? 0u : min(lane / (uint32_t)kTeamWarpBrows, (uint32_t)kT - 1u);
+    const uint32_t sbo = kCsr ? min(lane, max(n_blk, 1u) - 1u)
+                              : lane < (uint32_t)(kT * kTeamWarpBrows) ? lane % (uint32_t)kTeamWarpBrows : 0u;
+    const bool solver = kCsr ? lane < n_blk
+                             : lane < (uint32_t)(kT * kTeamWarpBrows) && warp < tw && st_part < it.parts &&
+                                   br0 + (st_part * tw + warp) * (uint32_t)kTeamWarpBrows + sbo < br1;
+    const uint32_t s_first = kCsr && solver ? D.bstart[blk0 + lane] - row0 : 6u * sbo;
+    const uint32_t s_rows = kCsr && solver ? D.bstart[blk0 + lane + 1u] - D.bstart[blk0 + lane] : 6u;
     float *const slu0 = kT > 1 && st_part ? lu[kT - 1] : lu[0];
     const float *const slu = slu0 + 36u * sbo;
-    float *const srd = slu0 + 36 * kTeamWarpBrows + 8u * sbo;
+    float *const srd = slu0 + 36u * (kCsr ? n_blk : (uint32_t)kTeamWarpBrows) + 8u * sbo;
     if (solver) {
         float dlo = kDivLo;
 #pragma unroll
@@ -226,13 +287,42 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
         srd[6] = dlo;
     }
     __syncthreads();
-    const uint32_t n_ext = 6u * S.ext;
+    const uint32_t n_ext = (kCsr ? 1u : 6u) * S.ext;
 
     // y = (row) . xg: products rounded, added in index order; the operands of
     // the next block are loaded before this block's products are added. Two
     // rows' sums run side by side.
     float ap[kT];
-    auto row_sums = [&]() {
+    auto row_sums_csr = [&]() {
+        float acc = 0.0f;
+        const float4 *V = val4;
+        const ushort4 *I = idx4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f), q = v;
+        ushort4 i = make_ushort4(0, 0, 0, 0);
+        if (most) {
+            v = V[0];
+            i = I[0];
+            q = make_float4(px[i.x], px[i.y], px[i.z], px[i.w]);
+            if (most > 4u) i = I[32];
+        }
+#pragma unroll 2
+        for (uint32_t j = 0; j < most; j += 4u) {
+            const float2 p01 = mul2_rn(make_float2(v.x, v.y), make_float2(q.x, q.y));
+            const float2 p23 = mul2_rn(make_float2(v.z, v.w), make_float2(q.z, q.w));
+            V += 32, I += 32;
+            if (j + 4u < most) {
+                v = *V;
+                q = make_float4(px[i.x], px[i.y], px[i.z], px[i.w]);
+                if (j + 8u < most) i = I[32];
+            }
+            acc = j < nk[0] ? __fadd_rn(acc, p01.x) : acc;
+            acc = j + 1u < nk[0] ? __fadd_rn(acc, p01.y) : acc;
+            acc = j + 2u < nk[0] ? __fadd_rn(acc, p23.x) : acc;
+            acc = j + 3u < nk[0] ? __fadd_rn(acc, p23.y) : acc;
+        }
+        ap[0] = acc;
+    };
+    auto row_sums_bsr = [&]() {
         const float4 *B4[kT], *X[kT];
         const float2 *B2[kT];
         float4 v[kT], xv[kT];
@@ -283,24 +373,32 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
         if (solver) {
             float y[6], pr[6];
             bool ok = true;
-            float *const rz = wz + st_part * kRows + 6u * sbo;
+            float *const rz = wz + st_part * kRows + s_first;
             float l[36];
 #pragma unroll
             for (int q = 0; q < 9; ++q) {
                 const float4 v = reinterpret_cast<const float4 *>(slu)[q];
                 l[4 * q] = v.x, l[4 * q + 1] = v.y, l[4 * q + 2] = v.z, l[4 * q + 3] = v.w;
             }
+            if (kCsr) {
 #pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                const float2 v = reinterpret_cast<const float2 *>(rz)[i];
-                y[2 * i] = v.x, y[2 * i + 1] = v.y;
+                for (int i = 0; i < 6; ++i) y[i] = (uint32_t)i < s_rows ? rz[i] : 0.0f;
+            } else {
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    const float2 v = reinterpret_cast<const float2 *>(rz)[i];
+                    y[2 * i] = v.x, y[2 * i + 1] = v.y;
+                }
             }
             const float4 d0 = reinterpret_cast<const float4 *>(srd)[0], d1 = reinterpret_cast<const float4 *>(srd)[1];
             const float rdiag[6] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y}, dlo = d1.z;
+            // (CSR: what an absent row gives is 0 also beside infinities.)
 #pragma unroll
-            for (int i = 1; i < 6; ++i)
+            for (int i = 1; i < 6; ++i) {
 #pragma unroll
                 for (int q = 0; q < i; ++q) y[i] = __fsub_rn(y[i], __fmul_rn(l[6 * i + q], y[q]));
+                if (kCsr && (uint32_t)i >= s_rows) y[i] = 0.0f;
+            }
 #pragma unroll
             for (int i = 5; i >= 0; --i) {
                 float v = y[i];
@@ -308,13 +406,18 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
                 for (int q = i + 1; q < 6; ++q) v = __fsub_rn(v, __fmul_rn(l[6 * i + q], pr[q]));
                 pr[i] = div_by(v, l[7 * i], rdiag[i], dlo, &ok);
             }
-            if (ok) {
+            if (kCsr) {
+#pragma unroll
+                for (int i = 0; i < 6; ++i)
+                    if ((uint32_t)i < s_rows) rz[i] = ok ? pr[i] : y[i];
+                if (!ok) back_general(slu, rz, rz, s_rows);
+            } else if (ok) {
 #pragma unroll
                 for (int i = 0; i < 3; ++i) reinterpret_cast<float2 *>(rz)[i] = make_float2(pr[2 * i], pr[2 * i + 1]);
             } else {
 #pragma unroll
                 for (int i = 0; i < 6; ++i) rz[i] = y[i];
-                back_general(slu, rz, rz);
+                back_general(slu, rz, rz, 6);
             }
         }
         __syncwarp();
@@ -380,7 +483,7 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
                 for (uint32_t q = 0; q < kBatch; ++q) {
                     const uint32_t i = b + q * step + tid, e = i / 6u;
                     const bool want = i < n_ext;
-                    zin[q] = ld_packet_if(zpk + (want ? ext[e] + (i - 6u * e) : 0u), want, (unsigned long long)tag << 32);
+                    zin[q] = ld_packet_if(zpk + (!want ? 0u : kCsr ? ext[i] : ext[e] + (i - 6u * e)), want, (unsigned long long)tag << 32);
                 }
 #pragma unroll
                 for (uint32_t q = 0; q < kBatch; ++q) bad |= (uint32_t)(zin[q] >> 32) ^ tag;
@@ -401,7 +504,7 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
     // p = z + beta p of the lane's rows and of their block columns (p = z when
     // first). All operands come before the first store, which the compiler
     // could not move a load across.
-    auto advance = [&](bool first, float bf) {
+    auto advance_bsr = [&](bool first, float bf) {
 #pragma unroll
         for (int t = 0; t < kT; ++t) {
             p[t] = first ? z[t] : __fadd_rn(__fmul_rn(p[t], bf), z[t]);
@@ -425,6 +528,14 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
         __syncwarp();
     };
 
+    // CSR: p at every column, once a CTA.
+    auto advance_csr = [&](bool first, float bf) {
+        p[0] = first ? z[0] : __fadd_rn(__fmul_rn(p[0], bf), z[0]);
+        px[32u * warp + lane] = p[0];
+        for (uint32_t i = kRows + tid; i < kRows + n_ext; i += kRows)
+            px[i] = first ? zx[i] : __fadd_rn(__fmul_rn(px[i], bf), zx[i]);
+    };
+
     // Results of a reduction are written between its two barriers and read by
     // all after the second; S.err may change at any time. The first pass of a
     // fresh system has xg = x0 and stands for k_init: r = b - A x0, z = M r,
@@ -434,7 +545,8 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
     for (;;) {
         ++tag;
         if (rows) {
-            row_sums();
+            if (kCsr) row_sums_csr();
+            else row_sums_bsr();
             __syncwarp();
         }
         if (init) {
@@ -520,7 +632,12 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
         }
         __syncthreads();
         if (!S.go) break;
-        if (rows) advance(init, S.beta_f);
+        if (kCsr) {
+            if (rows) advance_csr(init, S.beta_f);
+            __syncthreads();  // p is shared by the CTA
+        } else if (rows) {
+            advance_bsr(init, S.beta_f);
+        }
         if (!init && ++done >= limit) break;
         init = false;
     }
@@ -557,7 +674,7 @@ __device__ __forceinline__ void team_system_bsr6(const SysDesc &D, const TeamIte
     }
 }
 
-template <int kT>
+template <int kT, bool kCsr>
 __global__ void __launch_bounds__(kTeamThreads, 1)
     k_team(const SysDesc *__restrict__ sys, StepParams *sp, const TeamItem *__restrict__ items,
            const uint32_t *__restrict__ item_off, uint32_t limit) {
@@ -571,14 +688,93 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
     const uint32_t i1 = item_off[blockIdx.x + 1];
     for (uint32_t i = item_off[blockIdx.x]; i < i1; ++i) {
         const TeamItem it = items[i];
-        team_system_bsr6<kT>(sys[it.sys], it, limit, S, smem + team_fixed_bytes(kT), w);
+        team_system<kT, kCsr>(sys[it.sys], it, limit, S, smem + team_fixed_bytes(kT), w);
         __syncthreads();
         if (S.err) return;  // every CTA's later waits would run out as well
     }
 }
 
+// The columns of one part (one CTA) that are not its own rows, each once, and
+// for each nonzero the place of its column among the part's rows and those, in
+// the order in which k_team keeps the values. The numbers come in any order:
+// they choose places, not values. More than D.ext_cap such columns: count[size]
+// says so (and count[size + 1] the most of any part).
+constexpr uint32_t kPlanHash = 2 * kTeamMaxExt, kPlanThreads = 512;
+static_assert((kPlanHash & (kPlanHash - 1)) == 0 && kTeamMaxExt + kPlanThreads < kPlanHash, "the table never fills");
+__global__ void __launch_bounds__(kPlanThreads) k_team_plan_csr(SysDesc D, uint32_t *count, uint32_t size) {
+    extern __shared__ uint32_t table[];  // keys, then places
+    __shared__ uint32_t found, first[kTeamWarps + 1];
+    uint32_t *const place = table + kPlanHash;
+    const uint32_t tid = threadIdx.x, tw = D.team_warps, tile0 = blockIdx.x * tw, tiles = min(tw, D.n_tiles - tile0);
+    for (uint32_t i = tid; i < kPlanHash; i += kPlanThreads) table[i] = 0xffffffffu;
+    if (tid <= tiles) first[tid] = D.tile_row[tile0 + tid];
+    if (tid == 0) found = 0;
+    __syncthreads();
+    const uint32_t r0 = first[0], r1 = first[tiles], k0 = D.row_ptr[r0], k1 = D.row_ptr[r1];
+    const volatile uint32_t *const now = &found;
+    for (uint32_t k = k0 + tid; k < k1; k += kPlanThreads) {
+        const uint32_t c = D.col[k];
+        if (c >= r0 && c < r1) continue;
+        uint32_t h = (c * 2654435761u) & (kPlanHash - 1u);
+        while (*now <= D.ext_cap) {
+            const uint32_t old = atomicCAS(&table[h], 0xffffffffu, c);
+            if (old == c) break;
+            if (old == 0xffffffffu) {
+                const uint32_t e = atomicAdd(&found, 1u);
+                place[h] = kTeamWarps * 32u + e;
+                if (e < D.ext_cap) D.ext_cols[(size_t)blockIdx.x * D.ext_cap + e] = c;
+                break;
+            }
+            h = (h + 1u) & (kPlanHash - 1u);
+        }
+    }
+    __syncthreads();
+    if (tid == 0) {
+        count[blockIdx.x] = min(found, D.ext_cap);
+        if (found > D.ext_cap) count[size] = 1u;
+        atomicMax(&count[size + 1u], found);
+    }
+    if (found > D.ext_cap) return;
+    for (uint32_t t = 0; t < tiles; ++t) {
+        uint16_t *const idx = D.tile_idx + D.tile_off[tile0 + t];
+        const uint32_t lane = tid & 31u, nr = first[t + 1] - first[t];
+        uint32_t s = 0, nk = 0;
+        if (lane < nr) {
+            s = D.row_ptr[first[t] + lane];
+            nk = D.row_ptr[first[t] + lane + 1u] - s;
+        }
+        const uint32_t colp = (__reduce_max_sync(kFull, nk) + 3u) & ~3u;
+        for (uint32_t j = tid >> 5; j < colp; j += kPlanThreads / 32u) {
+            uint32_t at = 0;  // (past a row's end: not used)
+            if (j < nk) {
+                const uint32_t c = D.col[s + j];
+                if (c >= r0 && c < r1) {
+                    uint32_t q = 0;
+                    while (c >= first[q + 1]) ++q;
+                    at = 32u * q + (c - first[q]);
+                } else {
+                    uint32_t h = (c * 2654435761u) & (kPlanHash - 1u);
+                    while (table[h] != c) h = (h + 1u) & (kPlanHash - 1u);
+                    at = place[h];
+                }
+            }
+            idx[4u * (32u * (j >> 2) + lane) + (j & 3u)] = (uint16_t)at;
+        }
+    }
+}
+
 }  // namespace
 
-const void *team_kernel(int parts) { return parts == 1 ? (const void *)k_team<1> : (const void *)k_team<2>; }
+const void *team_kernel(int parts, bool csr) {
+    return csr ? (const void *)k_team<1, true> : parts == 1 ? (const void *)k_team<1, false> : (const void *)k_team<2, false>;
+}
+
+cudaError_t team_plan_csr(const SysDesc &D, uint32_t *count, uint32_t parts, cudaStream_t st) {
+    constexpr int bytes = 8 * (int)kPlanHash;
+    cudaError_t e = cudaFuncSetAttribute(k_team_plan_csr, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return e;
+    k_team_plan_csr<<<parts, kPlanThreads, bytes, st>>>(D, count, parts);
+    return cudaGetLastError();
+}
 
 }  // namespace wsb

@@ -36,6 +36,19 @@ __host__ __device__ constexpr uint32_t team_z_bytes(int parts, uint32_t ext) {
 __host__ __device__ constexpr uint32_t team_tile_bytes(uint32_t cols) {
     return kTeamLuBytes + kTeamColBytes * cols + kTeamIdxBytes * ((cols + 7u) / 8u);
 }
+// CSR: 32 rows at most a warp tile, its blocks (1 to 6 rows) kTeamBlockLu bytes
+// each, then 6 bytes a place of its longest row's length (a multiple of four)
+// times 32; before the tiles z and p of the CTA's rows and of at most
+// kTeamMaxExt columns outside, and those columns.
+constexpr int kTeamBlockLu = 144 + 32;
+constexpr uint32_t kTeamMaxExt = 4096;
+__host__ __device__ constexpr uint32_t team_csr_tile_bytes(uint32_t cols, uint32_t blocks) {
+    return (uint32_t)kTeamBlockLu * blocks + 192u * ((cols + 3u) & ~3u);
+}
+__host__ __device__ constexpr uint32_t team_csr_z_bytes(uint32_t ext) {
+    return (8u * 32u * kTeamWarps + 12u * ext + 15u) & ~15u;
+}
+static_assert(kTeamBlockLu % 16 == 0, "16-byte operands");
 static_assert(kTeamLuBytes % 16 == 0 && kTeamColBytes % 16 == 0 && kTeamIdxBytes % 16 == 0, "16-byte operands");
 
 // Copies of the published partials of a team, each read by every copies-th
@@ -56,6 +69,11 @@ __host__ __device__ constexpr uint64_t team_red_entries(uint32_t size) {
 // not fit in what L1 the shared memory leaves: 26 systems of 9^3 nodes 13.5 us
 // an iteration against 10.7; so did one CTA of 24 warp tiles, 4^3 nodes 5.5 us
 // against 2.9.)
-const void *team_kernel(int parts);
+const void *team_kernel(int parts, bool csr);
+// Fills D.tile_idx, D.ext_cols and D.ext_count (= count) of a CSR system whose
+// tiles are set, `parts` parts of D.team_warps tiles. count[parts] is set when a
+// part has more than D.ext_cap columns outside (nothing is iterated from such a
+// plan), count[parts + 1] to the most of any part; both start as 0.
+cudaError_t team_plan_csr(const SysDesc &D, uint32_t *count, uint32_t parts, cudaStream_t st);
 
 }  // namespace wsb

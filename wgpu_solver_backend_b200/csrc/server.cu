@@ -69,6 +69,16 @@ uint64_t estimate_bytes(const Request &r) {
     // (for teams of one warp tile a CTA at most).
     v += 8 * (n + kPadElems) + sizeof(RedEntry) * team_red_entries((uint32_t)std::min<uint64_t>(n / (6 * kTeamWarpBrows) + 1, 512));
     v += 8 * std::min<uint64_t>(r.cfg.hist_cap, r.cfg.max_iter + 1);
+    // k_team, CSR: warp tiles of at least 27 rows, a place of two bytes for each
+    // column (padded to the tile's longest row; a third of a CTA's shared memory
+    // at most), the columns outside each part.
+    if (n <= 32ull * kTeamWarps * 160) {
+        const uint64_t tiles = n / 27 + 1, parts = std::min<uint64_t>(tiles, 160);
+        uint64_t longest = 0;
+        for (uint64_t i = 0; i < n; ++i) longest = std::max<uint64_t>(longest, r.p_row_ptr[i + 1] - r.p_row_ptr[i]);
+        v += 12 * (tiles + 1) + std::min(64 * tiles * (longest + 3), parts * (kTeamSmemMax / 3)) +
+             4 * parts * std::min<uint64_t>(n, kTeamMaxExt);
+    }
     return a + m + v;
 }
 

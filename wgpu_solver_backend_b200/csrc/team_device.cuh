@@ -52,6 +52,10 @@ __device__ __forceinline__ void cp_async4(void *dst, const void *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
                  : "memory");
 }
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // Two FP32 products in one packed instruction, each rounded to nearest.
@@ -136,13 +140,13 @@ __device__ __forceinline__ float div_by(float v, float u, float y, float lo, boo
     *ok = *ok && ((av >= lo && av <= kDivHi) || (av == 0.0f && lo <= kDivHi));
     return av == 0.0f ? q0 : q;
 }
-// Backward substitution with plain divisions.
-__device__ __noinline__ void back_general(const float *lu, const float *y, float *x) {
+// Backward substitution of m rows with plain divisions.
+__device__ __noinline__ void back_general(const float *lu, const float *y, float *x, int m) {
 #pragma unroll 1
-    for (int i = 5; i >= 0; --i) {
+    for (int i = m - 1; i >= 0; --i) {
         float v = y[i];
 #pragma unroll 1
-        for (int q = i + 1; q < 6; ++q) v = __fsub_rn(v, __fmul_rn(lu[6 * i + q], x[q]));
+        for (int q = i + 1; q < m; ++q) v = __fsub_rn(v, __fmul_rn(lu[6 * i + q], x[q]));
         x[i] = __fdiv_rn(v, lu[7 * i]);
     }
 }

@@ -144,6 +144,14 @@ struct SysDesc {
     uint32_t team_warps;               // k_team: warp tiles of a part
     uint32_t team_ext[2];              // k_team: most blocks outside a CTA's rows that it multiplies with, one or two parts a CTA
     uint32_t team_pairs;               // k_team: always two parts a CTA, one partial for both
+    // k_team, CSR: first row and first block of each warp tile (n_tiles + 1),
+    // where its columns' places start in tile_idx, the places; of each part the
+    // columns outside its rows (ext_cap a part) and how many.
+    uint32_t n_tiles, ext_cap;
+    const uint32_t *tile_row, *tile_blk, *tile_off;
+    uint16_t *tile_idx;
+    uint32_t *ext_cols;
+    const uint32_t *ext_count;
     float *s;                          // single reduction: s = A p (by recurrence)
     unsigned long long *zpk;           // k_team: z of each row with the tag of its all-reduce (value low, tag high)
     float *p2;                         // k_stream: the other buffer of p
