@@ -167,7 +167,7 @@ struct Engine::Slot {
     uint32_t team = 0, team_warps = 0, team_ext[2] = {0, 0}, team_tiles[2] = {0, 0};
     // CSR: its warp tiles (first rows, first blocks, offsets of their columns'
     // places) and the columns outside a part that the plan has room for.
-    bool team_csr = false;
+    bool team_csr = false, planning = false;
     std::vector<uint32_t> tile_row, tile_blk, tile_off;
     uint32_t ext_cap = 0;
     uint32_t team_smem(uint32_t launch_parts, uint32_t parts) const {
@@ -235,6 +235,8 @@ Engine::~Engine() {
     cudaFree(d_state_);
     cudaFree(d_sp_);
     cudaFree(d_work_);
+    cudaFree(d_plan_);
+    cudaFreeHost(h_plan_);
     for (TeamLists &l : team_lists_) {
         cudaFree(l.dev);
         cudaFreeHost(l.host);
@@ -256,6 +258,10 @@ int Engine::ensure_capacity(uint32_t need) {
     SysState *dst = nullptr, *hst = nullptr;
     WSB_CUDA_TRY(ctx_, cudaMalloc(&ds, sizeof(SysDesc) * nc));
     WSB_CUDA_TRY(ctx_, cudaMalloc(&dst, sizeof(SysState) * nc));
+    uint32_t *dp = nullptr, *hp = nullptr;
+    WSB_CUDA_TRY(ctx_, cudaMalloc(&dp, 2 * sizeof(uint32_t) * nc));
+    WSB_CUDA_TRY(ctx_, cudaMallocHost(&hp, 2 * sizeof(uint32_t) * nc));
+    if (cap_) WSB_CUDA_TRY(ctx_, cudaMemcpyAsync(dp, d_plan_, 2 * sizeof(uint32_t) * cap_, cudaMemcpyDeviceToDevice, stream_));
     WSB_CUDA_TRY(ctx_, cudaMallocHost(&hs, sizeof(SysDesc) * nc));
     WSB_CUDA_TRY(ctx_, cudaMallocHost(&hst, sizeof(SysState) * nc));
     std::memset(hs, 0, sizeof(SysDesc) * nc);
@@ -273,8 +279,12 @@ int Engine::ensure_capacity(uint32_t need) {
     WSB_CUDA_TRY(ctx_, cudaStreamSynchronize(stream_));
     cudaFree(d_sys_);
     cudaFree(d_state_);
+    cudaFree(d_plan_);
+    cudaFreeHost(h_plan_);
     cudaFreeHost(h_sys_);
     cudaFreeHost(h_state_);
+    d_plan_ = dp;
+    h_plan_ = hp;
     d_sys_ = ds;
     d_state_ = dst;
     h_sys_ = hs;
@@ -345,7 +355,7 @@ void Engine::team_plan(Slot *sl) const {
 
 // The same for a CSR system whose blocks have 1 to 6 rows: warp tiles of whole
 // blocks, one part a CTA, and room for the columns outside a part's rows.
-// Whether they fit is found out by the plan on the device (finish_team_plan).
+// Whether they fit is found out by the plan on the device (start_team_plan).
 void Engine::team_plan_rows(Slot *sl) const {
     const MatA &A = *sl->A;
     const std::vector<uint32_t> &bs = sl->M->h_bs;
@@ -394,29 +404,45 @@ void Engine::team_plan_rows(Slot *sl) const {
     }
 }
 
-// Where the columns of a CSR system's nonzeros are in its CTAs' shared memory,
-// once for all its solves; a system with too many columns outside a part goes
-// to the loop kernels.
-int Engine::finish_team_plan(Slot *sl, SysDesc *d, uint32_t *tiles_mem, uint32_t *count) {
+// Starts the plan of where the columns of a CSR system's nonzeros are in its
+// CTAs' shared memory (once for all its solves); what it found out is read
+// before the system's first step, for all that were added (finish_team_plans).
+int Engine::start_team_plan(uint32_t s, Slot *sl, SysDesc *d, uint32_t *tiles_mem, uint32_t *count) {
     const size_t nt = sl->tile_row.size(), words = 3 * nt;
     std::vector<uint32_t> h(words);
     std::copy(sl->tile_row.begin(), sl->tile_row.end(), h.begin());
     std::copy(sl->tile_blk.begin(), sl->tile_blk.end(), h.begin() + nt);
     std::copy(sl->tile_off.begin(), sl->tile_off.end(), h.begin() + 2 * nt);
     WSB_CUDA_TRY(ctx_, cudaMemcpyAsync(tiles_mem, h.data(), sizeof(uint32_t) * words, cudaMemcpyHostToDevice, stream_));
+    WSB_CUDA_TRY(ctx_, cudaMemsetAsync(d_plan_ + 2 * s, 0, 2 * sizeof(uint32_t), stream_));
     d->n_tiles = (uint32_t)nt - 1;
     d->ext_cap = sl->ext_cap;
     d->tile_row = tiles_mem;
     d->tile_blk = tiles_mem + nt;
     d->tile_off = tiles_mem + 2 * nt;
     d->ext_count = count;
-    WSB_CUDA_TRY(ctx_, team_plan_csr(*d, count, sl->team, stream_));
+    WSB_CUDA_TRY(ctx_, team_plan_csr(*d, count, d_plan_ + 2 * s, sl->team, stream_));
     launches_ += 1;
-    uint32_t found[2] = {0, 0};
-    WSB_CUDA_TRY(ctx_, cudaMemcpyAsync(found, count + sl->team, sizeof found, cudaMemcpyDeviceToHost, stream_));
+    sl->planning = plans_pending_ = true;
+    return WSB_OK;
+}
+
+// A system with more columns outside a part than fit goes to the loop kernels.
+int Engine::finish_team_plans() {
+    if (!plans_pending_) return WSB_OK;
+    WSB_CUDA_TRY(ctx_, cudaMemcpyAsync(h_plan_, d_plan_, 2 * sizeof(uint32_t) * cap_, cudaMemcpyDeviceToHost, stream_));
     WSB_CUDA_TRY(ctx_, cudaStreamSynchronize(stream_));
-    sl->team_ext[0] = found[1];
-    if (found[0]) sl->team = 0;
+    for (uint32_t s = 0; s < slots_.size(); ++s) {
+        if (!slots_[s] || !slots_[s]->planning) continue;
+        Slot &sl = *slots_[s];
+        sl.planning = false;
+        sl.team_ext[0] = h_plan_[2 * s];
+        if (h_plan_[2 * s + 1]) sl.team = 0;
+        h_sys_[s].team_ext[0] = sl.team_ext[0];
+        h_sys_[s].path = sl.team ? PATH_TEAM : PATH_LOOP;
+        desc_dirty_ = true;
+    }
+    plans_pending_ = false;
     return WSB_OK;
 }
 
@@ -507,7 +533,7 @@ int Engine::add(const MatA *A, const Precond *M, const SolveCfg &cfg, uint32_t *
     take(15, sizeof(uint32_t) * tile_words);  // CSR: warp tiles
     take(16, sl->team_csr ? sizeof(uint16_t) * sl->tile_off.back() : 0);                   // places of the columns
     take(17, sl->team_csr ? sizeof(uint32_t) * (size_t)sl->team * sl->ext_cap : 0);        // columns outside
-    take(18, sl->team_csr ? sizeof(uint32_t) * (sl->team + 2) : 0);                        // their counts
+    take(18, sl->team_csr ? sizeof(uint32_t) * sl->team : 0);                        // their counts
     void *mem = nullptr;
     cudaError_t e = cudaMallocAsync(&mem, tot, stream_);
     if (e != cudaSuccess)
@@ -577,7 +603,7 @@ int Engine::add(const MatA *A, const Precond *M, const SolveCfg &cfg, uint32_t *
     d.tile_idx = (uint16_t *)(base + off[16]);
     d.ext_cols = (uint32_t *)(base + off[17]);
     if (sl->team_csr &&
-        (rc = finish_team_plan(sl.get(), &d, (uint32_t *)(base + off[15]), (uint32_t *)(base + off[18])))) {
+        (rc = start_team_plan(s, sl.get(), &d, (uint32_t *)(base + off[15]), (uint32_t *)(base + off[18])))) {
         cudaFreeAsync(mem, stream_);
         return rc;
     }
@@ -1049,6 +1075,7 @@ int Engine::launch_stream(const std::vector<uint32_t> &ids, uint32_t limit) {
 
 int Engine::step(uint32_t loop_limit, bool *any_left, uint32_t team_limit) {
     int rc;
+    if ((rc = finish_team_plans())) return rc;
     // The lists change only when the active set does (work_dirty_); the
     // layout is not free (a linear pass over every tile of every active
     // system), so it is not redone every step.

@@ -163,7 +163,8 @@ class Engine {
     int finish_slot(uint32_t slot, int status);
     void team_plan(Slot *sl) const;
     void team_plan_rows(Slot *sl) const;
-    int finish_team_plan(Slot *sl, SysDesc *d, uint32_t *tiles, uint32_t *count);
+    int start_team_plan(uint32_t s, Slot *sl, SysDesc *d, uint32_t *tiles, uint32_t *count);
+    int finish_team_plans();
     void stream_plan(Slot *sl) const;
     int launch_stream(const std::vector<uint32_t> &slots, uint32_t limit);
     int launch_team(const std::vector<uint32_t> &slots, bool csr, uint32_t limit);
@@ -193,6 +194,10 @@ class Engine {
         size_t cap = 0;  // words
     };
     TeamLists team_lists_[2];
+    // Of each slot's CSR plan: the most columns outside a part, and whether
+    // that is too many; not read yet for some slot.
+    uint32_t *d_plan_ = nullptr, *h_plan_ = nullptr;
+    bool plans_pending_ = false;
     cudaGraph_t graph_ = nullptr;
     cudaGraphExec_t exec_ = nullptr;
     uint32_t graph_grid_a_ = 0, graph_grid_b_ = 0, graph_grid_c_ = 0;

@@ -697,11 +697,11 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
 // The columns of one part (one CTA) that are not its own rows, each once, and
 // for each nonzero the place of its column among the part's rows and those, in
 // the order in which k_team keeps the values. The numbers come in any order:
-// they choose places, not values. More than D.ext_cap such columns: count[size]
-// says so (and count[size + 1] the most of any part).
+// they choose places, not values. most[0]: the most such columns of a part;
+// most[1]: more than D.ext_cap (nothing is iterated from such a plan).
 constexpr uint32_t kPlanHash = 2 * kTeamMaxExt, kPlanThreads = 512;
 static_assert((kPlanHash & (kPlanHash - 1)) == 0 && kTeamMaxExt + kPlanThreads < kPlanHash, "the table never fills");
-__global__ void __launch_bounds__(kPlanThreads) k_team_plan_csr(SysDesc D, uint32_t *count, uint32_t size) {
+__global__ void __launch_bounds__(kPlanThreads) k_team_plan_csr(SysDesc D, uint32_t *count, uint32_t *most) {
     extern __shared__ uint32_t table[];  // keys, then places
     __shared__ uint32_t found, first[kTeamWarps + 1];
     uint32_t *const place = table + kPlanHash;
@@ -731,8 +731,8 @@ __global__ void __launch_bounds__(kPlanThreads) k_team_plan_csr(SysDesc D, uint3
     __syncthreads();
     if (tid == 0) {
         count[blockIdx.x] = min(found, D.ext_cap);
-        if (found > D.ext_cap) count[size] = 1u;
-        atomicMax(&count[size + 1u], found);
+        if (found > D.ext_cap) most[1] = 1u;
+        atomicMax(most, found);
     }
     if (found > D.ext_cap) return;
     for (uint32_t t = 0; t < tiles; ++t) {
@@ -769,11 +769,11 @@ const void *team_kernel(int parts, bool csr) {
     return csr ? (const void *)k_team<1, true> : parts == 1 ? (const void *)k_team<1, false> : (const void *)k_team<2, false>;
 }
 
-cudaError_t team_plan_csr(const SysDesc &D, uint32_t *count, uint32_t parts, cudaStream_t st) {
+cudaError_t team_plan_csr(const SysDesc &D, uint32_t *count, uint32_t *most, uint32_t parts, cudaStream_t st) {
     constexpr int bytes = 8 * (int)kPlanHash;
     cudaError_t e = cudaFuncSetAttribute(k_team_plan_csr, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
-    k_team_plan_csr<<<parts, kPlanThreads, bytes, st>>>(D, count, parts);
+    k_team_plan_csr<<<parts, kPlanThreads, bytes, st>>>(D, count, most);
     return cudaGetLastError();
 }
 

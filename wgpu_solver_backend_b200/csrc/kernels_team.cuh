@@ -71,9 +71,9 @@ __host__ __device__ constexpr uint64_t team_red_entries(uint32_t size) {
 // against 2.9.)
 const void *team_kernel(int parts, bool csr);
 // Fills D.tile_idx, D.ext_cols and D.ext_count (= count) of a CSR system whose
-// tiles are set, `parts` parts of D.team_warps tiles. count[parts] is set when a
-// part has more than D.ext_cap columns outside (nothing is iterated from such a
-// plan), count[parts + 1] to the most of any part; both start as 0.
-cudaError_t team_plan_csr(const SysDesc &D, uint32_t *count, uint32_t parts, cudaStream_t st);
+// tiles are set, `parts` parts of D.team_warps tiles. most[0] becomes the most
+// columns outside a part, most[1] whether that is more than D.ext_cap (nothing
+// is iterated from such a plan); both start as 0.
+cudaError_t team_plan_csr(const SysDesc &D, uint32_t *count, uint32_t *most, uint32_t parts, cudaStream_t st);
 
 }  // namespace wsb

@@ -241,6 +241,7 @@ struct wsb_server {
             for (Request *r : admit) {
                 int rc = eng->add(r->A.get(), r->M.get(), r->cfg, &r->slot);
                 if (!rc) rc = eng->set_rhs(r->slot, r->p_b, r->p_x0, false);
+                if (rc) cudaStreamSynchronize(stream);  // what add started may read the matrix
                 std::lock_guard<std::mutex> lk(mu);
                 if (rc) {
                     r->A.reset();
