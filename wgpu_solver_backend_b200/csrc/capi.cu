@@ -71,10 +71,101 @@ static int solve_status_message(Context *ctx, int status, int breakdown, uint64_
 }
 
 // ---------------------------------------------------------------------------
-// Reference-arithmetic solve: the reference's passes one by one
-// (compute.rs:226-489) with the scalars and stop test kept on the device.
-// The iteration body runs inside a CUDA graph while loop.
+// Reference-arithmetic solve (compute.rs:226-489) with the scalars and stop
+// test kept on the device: one launch of k_ref_pcg, or the reference's passes
+// one by one, the iteration body inside a CUDA graph while loop (30 us an
+// iteration on 12^3 nodes, 6 in k_ref_pcg).
 // ---------------------------------------------------------------------------
+// The passes one by one; the loop is a graph, which the caller keeps until it
+// has ended.
+static int reference_passes(Context *ctx, const MatA &A, const Precond &M, uint32_t n, float *db, float *dx, float *dr, float *dp,
+                            float *dz, float *dap, float *scratch, float *s, RefState *dst, double *dhist, uint64_t hist_cap,
+                            std::unique_ptr<CUgraph_st, cudaError_t (*)(cudaGraph_t)> *gguard,
+                            std::unique_ptr<CUgraphExec_st, cudaError_t (*)(cudaGraphExec_t)> *eguard) {
+    cudaStream_t st = ctx->stream;
+    const unsigned gb = grid_for(n, 256), gblk = grid_for(M.nb, 128);
+    // The passes one by one: 1) ||b||^2 (compute.rs:228-250), 2) init (compute.rs:283-331).
+    WSB_CUDA_TRY(ctx, ref_dot(st, n, db, db, scratch, s + 0));
+    k_ref_after_bnorm<<<1, 32, 0, st>>>(dst, s);
+    if (n) WSB_CUDA_TRY(ctx, cudaMemcpyAsync(dr, db, sizeof(float) * n, cudaMemcpyDeviceToDevice, st));
+    k_ref_spmv<<<gb, 256, 0, st>>>(n, A.row_ptr, A.col, A.val, dx, dap);
+    k_ref_axpy<<<gb, 256, 0, st>>>(n, -1.0f, dap, dr);
+    k_ref_block_jacobi<<<gblk, 128, 0, st>>>(n, M.nb, M.lu, M.bs, dr, dz);
+    if (n) WSB_CUDA_TRY(ctx, cudaMemcpyAsync(dp, dz, sizeof(float) * n, cudaMemcpyDeviceToDevice, st));
+    WSB_CUDA_TRY(ctx, ref_dot(st, n, dr, dz, scratch, s + 3));
+    k_ref_after_init<<<1, 32, 0, st>>>(dst, s);
+    WSB_CUDA_TRY(ctx, cudaGetLastError());
+    // 3) the loop (compute.rs:336-489) as a graph: gate + while(body).
+    cudaGraph_t g = nullptr;
+    cudaGraphExec_t ge = nullptr;
+    WSB_CUDA_TRY(ctx, cudaGraphCreate(&g, 0));
+    gguard->reset(g);
+    cudaGraphConditionalHandle h;
+    WSB_CUDA_TRY(ctx, cudaGraphConditionalHandleCreate(&h, g, 0, 0));
+    cudaKernelNodeParams kp = {};
+    const RefState *cst = dst;
+    void *gate_args[] = {(void *)&cst, &h};
+    kp.func = (void *)k_ref_gate;
+    kp.gridDim = dim3(1);
+    kp.blockDim = dim3(32);
+    kp.kernelParams = gate_args;
+    cudaGraphNode_t gate, wn;
+    WSB_CUDA_TRY(ctx, cudaGraphAddKernelNode(&gate, g, nullptr, 0, &kp));
+    cudaGraphNodeParams cp = {};
+    cp.type = cudaGraphNodeTypeConditional;
+    cp.conditional.handle = h;
+    cp.conditional.type = cudaGraphCondTypeWhile;
+    cp.conditional.size = 1;
+    WSB_CUDA_TRY(ctx, cudaGraphAddNode(&wn, g, &gate, 1, &cp));
+    cudaGraph_t body = cp.conditional.phGraph_out[0];
+    cudaStream_t cs;
+    WSB_CUDA_TRY(ctx, cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
+    cudaError_t ce = cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed);
+    if (ce == cudaSuccess) {
+        k_ref_spmv<<<gb, 256, 0, cs>>>(n, A.row_ptr, A.col, A.val, dp, dap);            // A
+        ref_dot(cs, n, dp, dap, scratch, s + 0);                                        // B
+        k_ref_write_rz_old<<<1, 32, 0, cs>>>(dst, s);                                    // C
+        k_ref_update_scalars<<<1, 32, 0, cs>>>(s, 0, 2, 3, 4, 5, 6);                     // D
+        k_ref_axpy_s<<<gb, 256, 0, cs>>>(n, dp, dx, s, 4);                               // E
+        k_ref_axpy_s<<<gb, 256, 0, cs>>>(n, dap, dr, s, 5);
+        ref_dot(cs, n, dr, dr, scratch, s + 1);                                         // F
+        k_ref_block_jacobi<<<gblk, 128, 0, cs>>>(n, M.nb, M.lu, M.bs, dr, dz);         // G
+        ref_dot(cs, n, dr, dz, scratch, s + 2);                                         // H
+        k_ref_update_scalars<<<1, 32, 0, cs>>>(s, 0, 2, 3, 4, 5, 6);                     // I
+        k_ref_scale_s<<<gb, 256, 0, cs>>>(n, dp, s, 6);                                  // J
+        k_ref_axpy<<<gb, 256, 0, cs>>>(n, 1.0f, dz, dp);
+        k_ref_check<<<1, 32, 0, cs>>>(dst, s, dhist, hist_cap, h);  // readback + checks
+        ce = cudaStreamEndCapture(cs, &body);
+    }
+    cudaStreamDestroy(cs);
+    if (ce != cudaSuccess) return fail(ctx, WSB_ERR_CUDA, "capturing the reference loop failed: %s", cudaGetErrorString(ce));
+    WSB_CUDA_TRY(ctx, cudaGraphInstantiate(&ge, g, 0));
+    eguard->reset(ge);
+    WSB_CUDA_TRY(ctx, cudaGraphLaunch(ge, st));
+    return WSB_OK;
+}
+
+// Whether k_ref_pcg solves this system (*width_plus_1: nonzeros of its longest
+// row, plus one; else 0): its CTAs, a workgroup of 256 rows each, are resident
+// together with their rows in shared memory, and every block starts after the
+// one before.
+static int ref_resident(Context *ctx, const MatA &A, const Precond &M, int *width_plus_1) {
+    *width_plus_1 = 0;
+    const uint32_t n = A.n, sms = (uint32_t)ctx->sm_count;
+    if (n == 0 || (n + 255u) / 256u > 2u * sms || M.h_bs.size() != (size_t)M.nb + 1) return WSB_OK;
+    for (uint32_t k = 0; k < M.nb; ++k)
+        if (M.h_bs[k + 1] <= M.h_bs[k]) return WSB_OK;
+    if (M.h_bs[M.nb] > n) return WSB_OK;
+    uint32_t width = 0;
+    for (uint32_t i = 0; i < n; ++i) width = std::max(width, A.h_rows[i + 1] - A.h_rows[i]);
+    if (width > 200u || ref_pcg_smem(width) > (uint32_t)kTeamSmemMax) return WSB_OK;
+    int per_sm = 0;
+    WSB_CUDA_TRY(ctx, cudaFuncSetAttribute(ref_pcg_kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, kTeamSmemMax));
+    WSB_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ref_pcg_kernel(), kRefThreads, ref_pcg_smem(width)));
+    if ((n + 255u) / 256u <= (uint32_t)per_sm * sms) *width_plus_1 = (int)width + 1;
+    return WSB_OK;
+}
+
 static int solve_reference(Context *ctx, const MatA &A, const Precond &M, const float *b, float *x, bool dev,
                            uint64_t max_iter, float rel_tol, float abs_tol, bool always_x, SolveOutcome *out,
                            double *hist_host, uint64_t hist_cap, uint64_t *hist_len, double *device_ms) {
@@ -117,65 +208,20 @@ static int solve_reference(Context *ctx, const MatA &A, const Precond &M, const 
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     cudaEventRecord(e0, st);
-    const unsigned gb = grid_for(n, 256), gblk = grid_for(M.nb, 128);
-    // 1) ||b||^2 (compute.rs:228-250), 2) init (compute.rs:283-331).
-    WSB_CUDA_TRY(ctx, ref_dot(st, n, db, db, scratch, s + 0));
-    k_ref_after_bnorm<<<1, 32, 0, st>>>(dst, s);
-    if (n) WSB_CUDA_TRY(ctx, cudaMemcpyAsync(dr, db, sizeof(float) * n, cudaMemcpyDeviceToDevice, st));
-    k_ref_spmv<<<gb, 256, 0, st>>>(n, A.row_ptr, A.col, A.val, dx, dap);
-    k_ref_axpy<<<gb, 256, 0, st>>>(n, -1.0f, dap, dr);
-    k_ref_block_jacobi<<<gblk, 128, 0, st>>>(n, M.nb, M.lu, M.bs, dr, dz);
-    if (n) WSB_CUDA_TRY(ctx, cudaMemcpyAsync(dp, dz, sizeof(float) * n, cudaMemcpyDeviceToDevice, st));
-    WSB_CUDA_TRY(ctx, ref_dot(st, n, dr, dz, scratch, s + 3));
-    k_ref_after_init<<<1, 32, 0, st>>>(dst, s);
-    WSB_CUDA_TRY(ctx, cudaGetLastError());
-    // 3) the loop (compute.rs:336-489) as a graph: gate + while(body).
-    cudaGraph_t g = nullptr;
-    cudaGraphExec_t ge = nullptr;
-    WSB_CUDA_TRY(ctx, cudaGraphCreate(&g, 0));
-    std::unique_ptr<CUgraph_st, cudaError_t (*)(cudaGraph_t)> gguard(g, cudaGraphDestroy);
-    cudaGraphConditionalHandle h;
-    WSB_CUDA_TRY(ctx, cudaGraphConditionalHandleCreate(&h, g, 0, 0));
-    cudaKernelNodeParams kp = {};
-    const RefState *cst = dst;
-    void *gate_args[] = {(void *)&cst, &h};
-    kp.func = (void *)k_ref_gate;
-    kp.gridDim = dim3(1);
-    kp.blockDim = dim3(32);
-    kp.kernelParams = gate_args;
-    cudaGraphNode_t gate, wn;
-    WSB_CUDA_TRY(ctx, cudaGraphAddKernelNode(&gate, g, nullptr, 0, &kp));
-    cudaGraphNodeParams cp = {};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = h;
-    cp.conditional.type = cudaGraphCondTypeWhile;
-    cp.conditional.size = 1;
-    WSB_CUDA_TRY(ctx, cudaGraphAddNode(&wn, g, &gate, 1, &cp));
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    cudaStream_t cs;
-    WSB_CUDA_TRY(ctx, cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-    cudaError_t ce = cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed);
-    if (ce == cudaSuccess) {
-        k_ref_spmv<<<gb, 256, 0, cs>>>(n, A.row_ptr, A.col, A.val, dp, dap);            // A
-        ref_dot(cs, n, dp, dap, scratch, s + 0);                                        // B
-        k_ref_write_rz_old<<<1, 32, 0, cs>>>(dst, s);                                    // C
-        k_ref_update_scalars<<<1, 32, 0, cs>>>(s, 0, 2, 3, 4, 5, 6);                     // D
-        k_ref_axpy_s<<<gb, 256, 0, cs>>>(n, dp, dx, s, 4);                               // E
-        k_ref_axpy_s<<<gb, 256, 0, cs>>>(n, dap, dr, s, 5);
-        ref_dot(cs, n, dr, dr, scratch, s + 1);                                         // F
-        k_ref_block_jacobi<<<gblk, 128, 0, cs>>>(n, M.nb, M.lu, M.bs, dr, dz);         // G
-        ref_dot(cs, n, dr, dz, scratch, s + 2);                                         // H
-        k_ref_update_scalars<<<1, 32, 0, cs>>>(s, 0, 2, 3, 4, 5, 6);                     // I
-        k_ref_scale_s<<<gb, 256, 0, cs>>>(n, dp, s, 6);                                  // J
-        k_ref_axpy<<<gb, 256, 0, cs>>>(n, 1.0f, dz, dp);
-        k_ref_check<<<1, 32, 0, cs>>>(dst, s, hist_cap ? dhist : nullptr, hist_cap, h);  // readback + checks
-        ce = cudaStreamEndCapture(cs, &body);
+    int resident = 0;
+    if ((rc = ref_resident(ctx, A, M, &resident))) return rc;
+    std::unique_ptr<CUgraph_st, cudaError_t (*)(cudaGraph_t)> gguard(nullptr, cudaGraphDestroy);
+    std::unique_ptr<CUgraphExec_st, cudaError_t (*)(cudaGraphExec_t)> eguard(nullptr, cudaGraphExecDestroy);
+    if (resident) {
+        RefPcg R{n, M.nb, (uint32_t)resident - 1u, A.row_ptr, A.col, A.val, M.lu, M.bs, db, dx, dz, dp, dap,
+                 reinterpret_cast<unsigned long long *>(dr), dst, hist_cap ? dhist : nullptr, hist_cap};
+        void *args[] = {&R};
+        WSB_CUDA_TRY(ctx, cudaLaunchCooperativeKernel(ref_pcg_kernel(), dim3(grid_for(n, 256)), dim3(kRefThreads), args,
+                                                      (size_t)ref_pcg_smem(R.width), st));
+    } else {
+        rc = reference_passes(ctx, A, M, n, db, dx, dr, dp, dz, dap, scratch, s, dst, hist_cap ? dhist : nullptr, hist_cap, &gguard, &eguard);
+        if (rc) return rc;
     }
-    cudaStreamDestroy(cs);
-    if (ce != cudaSuccess) return fail(ctx, WSB_ERR_CUDA, "capturing the reference loop failed: %s", cudaGetErrorString(ce));
-    WSB_CUDA_TRY(ctx, cudaGraphInstantiate(&ge, g, 0));
-    std::unique_ptr<CUgraphExec_st, cudaError_t (*)(cudaGraphExec_t)> eguard(ge, cudaGraphExecDestroy);
-    WSB_CUDA_TRY(ctx, cudaGraphLaunch(ge, st));
     cudaEventRecord(e1, st);
     WSB_CUDA_TRY(ctx, cudaMemcpyAsync(&hs, dst, sizeof hs, cudaMemcpyDeviceToHost, st));
     WSB_CUDA_TRY(ctx, cudaStreamSynchronize(st));
@@ -191,6 +237,7 @@ static int solve_reference(Context *ctx, const MatA &A, const Precond &M, const 
     out->breakdown = (int)hs.breakdown;
     out->status = hs.status == ST_CONVERGED ? WSB_OK : hs.status == ST_BREAKDOWN ? WSB_ERR_BREAKDOWN : WSB_ERR_NOT_CONVERGED;
     if (hs.status == ST_RUNNING) out->status = WSB_ERR_CUDA;
+    if (hs.error) return fail(ctx, WSB_ERR_TIMEOUT, "a wait of the solve kernel ran out");
     // b.b == 0 returns Ok(0) with x untouched (compute.rs:252-254).
     const bool x_changed = !(hs.status == ST_CONVERGED && hs.iter == 0);
     if (n && x_changed && (out->status == WSB_OK || always_x))

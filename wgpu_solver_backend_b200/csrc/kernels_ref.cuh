@@ -10,7 +10,7 @@ struct RefState {
     float b_norm2, rel2, abs2, rz_old;
     float rel_tol, abs_tol, last_rr, pad;
     uint32_t iter, max_iter, status, active;
-    uint32_t breakdown, pad2[3];
+    uint32_t breakdown, error, pad2[2];  // error: a wait of k_ref_pcg ran out
 };
 
 __global__ void k_ref_spmv(uint32_t n, const uint32_t *__restrict__ row_ptr, const uint32_t *__restrict__ col,
@@ -39,5 +39,28 @@ __global__ void k_ref_gate(const RefState *st, cudaGraphConditionalHandle h);
 // scratch needs ceil(n/256) + ceil(n/65536) + 2 floats.
 cudaError_t ref_dot(cudaStream_t st, uint32_t n, const float *a, const float *b, float *scratch, float *s_out);
 size_t ref_dot_scratch_floats(uint64_t n);
+
+// A whole solve in one cooperative launch, one CTA of kRefThreads threads per
+// 256 rows (per workgroup of the dot products).
+struct RefPcg {
+    uint32_t n, nb, width;  // width: nonzeros of the longest row
+    const uint32_t *row_ptr, *col;
+    const float *val, *lu;
+    const uint32_t *bs;     // block starts, strictly increasing
+    const float *b;
+    float *x, *z, *p0, *p1;            // x: x0, then the solution
+    unsigned long long *parts;         // 3 x CTAs published partials, zero at first
+    RefState *st;                      // tolerances and limit; the outcome
+    double *history;
+    uint64_t hist_cap;
+};
+constexpr int kRefThreads = 288;  // a thread a row, and 32 for the rows beside the CTA's
+constexpr uint32_t kRefCols = 1280, kRefHash = 2048;
+constexpr uint32_t kRefWin = 272;  // rows of blocks that a CTA shares: 5 + 256 + 5
+__host__ __device__ constexpr uint32_t ref_pcg_smem(uint32_t width) {
+    return 1024u + 4u * (2u * kRefWin + 2u * 256u + 2u * kRefCols + kRefHash) + 2u * kRefHash +
+           6u * kRefThreads * ((width + 1u) & ~1u);
+}
+const void *ref_pcg_kernel();
 
 }  // namespace wsb
