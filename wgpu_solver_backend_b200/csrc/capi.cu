@@ -282,19 +282,20 @@ struct wsb_matrix {
     std::unique_ptr<Engine> eng;
     uint32_t slot = 0;
     SolveCfg slot_cfg;
-    // wsb_matrix_spmv_device: the plain SpMV kernel's one-system descriptor
-    // and error word (device), allocated on the first call and owned by the
-    // matrix; a pinned host copy of the error word refreshed after every
-    // launch, and the event that marks that copy.
-    SysDesc *spmv_dd = nullptr;
+    // wsb_matrix_spmv_device: the plain SpMV kernel's parameters (device) and
+    // its error word (mapped host memory), allocated on the first call and
+    // owned by the matrix, and an event after the last launch. (With copies of
+    // the descriptor and the error word around each launch a call on 41^3 nodes
+    // took 16.4 us, 14.1 without.)
     StepParams *spmv_sp = nullptr;
-    uint32_t *spmv_err_h = nullptr;
+    volatile uint32_t *spmv_err_h = nullptr;
+    uint32_t spmv_grid_max = 0;  // resident CTAs of the kernel
+    bool spmv_ready = false;
     cudaEvent_t spmv_err_ev = nullptr;
     bool spmv_err_pending = false;
     ~wsb_matrix() {
-        dev_free(spmv_dd);
         dev_free(spmv_sp);
-        if (spmv_err_h) cudaFreeHost(spmv_err_h);
+        if (spmv_err_h) cudaFreeHost((void *)spmv_err_h);
         if (spmv_err_ev) cudaEventDestroy(spmv_err_ev);
     }
 };
@@ -881,13 +882,12 @@ extern "C" int wsb_solve_device(wsb_context *ctx, wsb_matrix *m, const float *d_
     return matrix_solve(ctx, m, d_b, d_x, true, max_iter, rel, abs_tol, o, res);
 }
 
-// The error word of the plain SpMV kernel is sticky: launches OR their codes
-// into it and only a reported error clears it, so a code survives later
-// launches until a call reads it.
+// The error word of the plain SpMV kernel (mapped host memory) is sticky:
+// launches OR their codes into it and only a reported error clears it, so a
+// code survives later launches until a call reads it.
 static int spmv_error_status(wsb_matrix *m, uint32_t code) {
     m->spmv_err_pending = false;
     *m->spmv_err_h = 0;
-    cudaMemsetAsync(&m->spmv_sp->error, 0, sizeof(uint32_t), m->ctx->stream);
     return fail(m->ctx, (code & kErrWaitMask) ? WSB_ERR_TIMEOUT : WSB_ERR_CUDA,
                 "an earlier wsb_matrix_spmv_device launch on this matrix failed (kernel code %u)", code);
 }
@@ -898,26 +898,33 @@ extern "C" int wsb_matrix_spmv_device(wsb_context *ctx, wsb_matrix *m, const flo
     if (m->ctx->device != ctx->device)
         return fail(ctx, WSB_ERR_BAD_INPUT, "the matrix lives on device %d, the context on device %d", m->ctx->device,
                     ctx->device);
-    if (!m->spmv_dd) {
-        void *dd = nullptr, *sp = nullptr;
-        WSB_CUDA_TRY(ctx, cudaMalloc(&dd, sizeof(SysDesc)));
-        m->spmv_dd = static_cast<SysDesc *>(dd);
-        WSB_CUDA_TRY(ctx, cudaMalloc(&sp, sizeof(StepParams)));
-        m->spmv_sp = static_cast<StepParams *>(sp);
-        WSB_CUDA_TRY(ctx, cudaMemsetAsync(m->spmv_sp, 0, sizeof(StepParams), ctx->stream));
-        WSB_CUDA_TRY(ctx, cudaHostAlloc((void **)&m->spmv_err_h, sizeof(uint32_t), cudaHostAllocDefault));
+    if (!m->spmv_ready) {
+        if (!m->spmv_sp) {
+            void *sp = nullptr;
+            WSB_CUDA_TRY(ctx, cudaMalloc(&sp, sizeof(StepParams)));
+            m->spmv_sp = static_cast<StepParams *>(sp);
+        }
+        if (!m->spmv_err_h)
+            WSB_CUDA_TRY(ctx, cudaHostAlloc((void **)&m->spmv_err_h, sizeof(uint32_t), cudaHostAllocMapped | cudaHostAllocPortable));
         *m->spmv_err_h = 0;
-        WSB_CUDA_TRY(ctx, cudaEventCreateWithFlags(&m->spmv_err_ev, cudaEventDisableTiming));
+        StepParams h;
+        std::memset(&h, 0, sizeof h);
+        WSB_CUDA_TRY(ctx, cudaHostGetDevicePointer((void **)&h.host_error, (void *)m->spmv_err_h, 0));
+        WSB_CUDA_TRY(ctx, cudaMemcpyAsync(m->spmv_sp, &h, sizeof h, cudaMemcpyHostToDevice, ctx->stream));
+        if (!m->spmv_err_ev) WSB_CUDA_TRY(ctx, cudaEventCreateWithFlags(&m->spmv_err_ev, cudaEventDisableTiming));
         WSB_CUDA_TRY(ctx, cudaFuncSetAttribute(k_spmv_plain, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)kSpmvSmem));
+        int occ = 0;
+        WSB_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_spmv_plain, kSpmvThreads, kSpmvSmem));
+        m->spmv_grid_max = (uint32_t)(std::max(occ, 1) * ctx->sm_count);
+        // (Later calls may come on other streams.)
+        WSB_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+        m->spmv_ready = true;
     }
-    // A finished read-back of the error word with a code in it: report it.
-    if (m->spmv_err_pending && cudaEventQuery(m->spmv_err_ev) == cudaSuccess) {
-        m->spmv_err_pending = false;
-        if (*m->spmv_err_h) return spmv_error_status(m, *m->spmv_err_h);
-    }
-    // The one-system descriptor (rewritten every call: the tiles may have
-    // been rebuilt by the autotuner since the last one).
+    // An earlier launch has failed: report it.
+    if (*m->spmv_err_h) return spmv_error_status(m, *m->spmv_err_h);
+    // The one-system descriptor, with the launch (the tiles may have been
+    // rebuilt by the autotuner since the last one).
     SysDesc d;
     std::memset(&d, 0, sizeof d);
     d.n = m->A.n;
@@ -930,14 +937,9 @@ extern "C" int wsb_matrix_spmv_device(wsb_context *ctx, wsb_matrix *m, const flo
     d.bval = m->A.bval;
     d.stiles = m->A.stiles;
     d.n_stiles = m->A.n_stiles;
-    WSB_CUDA_TRY(ctx, cudaMemcpyAsync(m->spmv_dd, &d, sizeof d, cudaMemcpyHostToDevice, ctx->stream));
-    int occ = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_spmv_plain, kSpmvThreads, kSpmvSmem);
-    const uint32_t g = std::max<uint32_t>(1, std::min<uint32_t>(m->A.n_stiles, (uint32_t)(std::max(occ, 1) * ctx->sm_count)));
-    k_spmv_plain<<<g, kSpmvThreads, kSpmvSmem, ctx->stream>>>(m->spmv_dd, m->spmv_sp, d_x, d_y);
+    const uint32_t g = std::max<uint32_t>(1, std::min<uint32_t>(m->A.n_stiles, m->spmv_grid_max));
+    k_spmv_plain<<<g, kSpmvThreads, kSpmvSmem, ctx->stream>>>(d, m->spmv_sp, d_x, d_y);
     WSB_CUDA_TRY(ctx, cudaGetLastError());
-    WSB_CUDA_TRY(ctx, cudaMemcpyAsync(m->spmv_err_h, &m->spmv_sp->error, sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                                      ctx->stream));
     WSB_CUDA_TRY(ctx, cudaEventRecord(m->spmv_err_ev, ctx->stream));
     m->spmv_err_pending = true;
     return WSB_OK;

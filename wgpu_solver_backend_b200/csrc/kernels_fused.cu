@@ -302,6 +302,12 @@ __device__ __forceinline__ bool take_ticket(uint32_t *counter, uint32_t cnt, uin
     return last;
 }
 
+// Records an error code; a plain product's also where its host reads it.
+__device__ __noinline__ void report_error(StepParams *sp, uint32_t code) {
+    atomicOr(&sp->error, code);
+    if (sp->host_error) atomicOr_system(sp->host_error, code);
+}
+
 // ---------------------------------------------------------------------------
 // SpMV tiles
 // ---------------------------------------------------------------------------
@@ -732,7 +738,7 @@ __device__ __forceinline__ void spmv_producer(const SysDesc *__restrict__ sys, S
             for (uint32_t i = 0; i < n_out; ++i) {
                 const uint32_t s = k % NS;
                 if (k >= NS && !mbar_wait(&empty[s], ((k / NS) - 1) & 1u, lim)) {
-                    atomicOr(&sp->error, kErrSpmvProducerWait);
+                    report_error(sp, kErrSpmvProducerWait);
                     err = true;
                     break;
                 }
@@ -779,7 +785,7 @@ __device__ __forceinline__ void spmv_gatherer(const SysDesc *__restrict__ sys, S
         if (lane == 0) ok = mbar_wait(&meta[s], par, lim) ? 1u : 0u;
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (!ok) {
-            if (lane == 0) atomicOr(&sp->error, kErrGatherWait);
+            if (lane == 0) report_error(sp, kErrGatherWait);
             break;
         }
         mbar_observe(&meta[s], par, lim);  // completed: the descriptor is visible
@@ -841,7 +847,7 @@ __device__ __forceinline__ void spmv_pipeline(const SysDesc *__restrict__ sys, S
         if (tid == 0) s_ok[k & 1u] = (mbar_wait(&gath[s], par, lim) && mbar_wait(&full[s], par, lim)) ? 1 : 0;
         csync<NC>();
         if (!s_ok[k & 1u]) {
-            if (tid == 0) atomicOr(&sp->error, kErrSpmvConsumerWait);
+            if (tid == 0) report_error(sp, kErrSpmvConsumerWait);
             return;
         }
         mbar_observe(&gath[s], par, lim);
@@ -1522,10 +1528,10 @@ __global__ void __launch_bounds__(kSpmvThreads, kSpmvMinCtas) k_spmv_init(const 
     spmv_pipeline<M_INIT>(sys, sp, nullptr, nullptr, smem);
 }
 
-__global__ void __launch_bounds__(kSpmvThreads, kSpmvMinCtas) k_spmv_plain(const SysDesc *__restrict__ sys, StepParams *sp,
+__global__ void __launch_bounds__(kSpmvThreads, kSpmvMinCtas) k_spmv_plain(const __grid_constant__ SysDesc sys, StepParams *sp,
                                                          const float *__restrict__ x, float *__restrict__ y) {
     extern __shared__ __align__(128) float smem[];
-    spmv_pipeline<M_PLAIN>(sys, sp, x, y, smem);
+    spmv_pipeline<M_PLAIN>(&sys, sp, x, y, smem);
 }
 
 __global__ void __launch_bounds__(kUpdThreads, kUpdMinCtas) k_update(const SysDesc *__restrict__ sys, StepParams *sp) {

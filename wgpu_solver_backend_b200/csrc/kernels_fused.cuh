@@ -83,9 +83,9 @@ __global__ void k_resid64(const SysDesc *__restrict__ sys, StepParams *sp);
 __global__ void k_refine(const SysDesc *__restrict__ sys, StepParams *sp);
 __global__ void k_x64_to_x32(const SysDesc *__restrict__ sys, StepParams *sp);
 
-// Plain y = A x of one system (sys[0]) over its own tiles (no reduction);
-// sp receives the error code of a timed-out wait.
-__global__ void k_spmv_plain(const SysDesc *__restrict__ sys, StepParams *sp, const float *__restrict__ x,
+// Plain y = A x of one system over its own tiles (no reduction); sp receives
+// the error code of a timed-out wait.
+__global__ void k_spmv_plain(const __grid_constant__ SysDesc sys, StepParams *sp, const float *__restrict__ x,
                              float *__restrict__ y);
 
 }  // namespace wsb

@@ -208,6 +208,7 @@ struct StepParams {
     uint32_t num_sys;                  // entries of the SysDesc array (work items are checked against it)
     uint32_t tail_ticket;              // single reduction: CTAs of the update kernel done (last one ends the step)
     unsigned long long wait_cycles;    // limit of one pipeline wait in SM clock cycles; 0: the default (~2 s)
+    uint32_t *host_error;              // plain products: error once more, in mapped host memory
 };
 
 // ---------------------------------------------------------------------------
