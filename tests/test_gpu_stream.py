@@ -47,9 +47,9 @@ def ring_system(nbr, offsets, seed):
 
 
 # Block rows: the fewest; 80 a CTA less one, exactly (16 warps with one product
-# tile each), plus one; the same with 100; several update tiles a warp, an odd
+# tile each), plus one; the same with 100 and 160; several update tiles a warp, an odd
 # count.
-@pytest.mark.parametrize("nbr", [10361, 11839, 11840, 11841, 13321, 14799, 14800, 14801, 75777])
+@pytest.mark.parametrize("nbr", [10361, 11839, 11840, 11841, 13321, 14799, 14800, 14801, 19241, 23679, 23680, 23681, 75777])
 def test_single_reduction(ctx, nbr):
     rp, ci, v, bs, b = ring_system(nbr, (1, 3, 170), nbr)
     n = len(rp) - 1

@@ -129,3 +129,28 @@ def test_more_teams_than_the_device_holds(ctx):
         xb, rb = batch.result(i, m.n)
         assert rb["iterations"] == r["iterations"]
         assert np.array_equal(xb.view(np.uint32), x.view(np.uint32))
+
+
+# One CTA, one part a CTA, two parts a CTA; cut into steps by a server.
+@pytest.mark.parametrize("nbr, layout", [(1, "BSR6"), (71, "BSR6"), (2000, "BSR6"), (10361, "BSR6"), (71, "CSR"),
+                                         (2000, "CSR")])
+def test_single_reduction(ctx, nbr, layout):
+    rp, ci, v, bs, b = block_system(nbr, 1, nbr)
+    n = len(rp) - 1
+    x0 = np.random.default_rng(1).standard_normal(n).astype(np.float32)
+    kw = dict(max_iter=4000, rel_tol=1e-6, algorithm=wsb.ALG_SINGLE_REDUCTION)
+    m = wsb.Matrix.create(ctx, rp, ci, v, bs, layout=getattr(wsb, "LAYOUT_" + layout))
+    x, r = m.solve(b, x0=x0, history_capacity=4000, **kw)
+    lu = wsb.build_lu_blocks_from_csr_block_starts_6(n, rp, ci, v, bs)
+    f64 = oracle.pcg_single_reduction_f64dot(rp, ci, v, lu, bs, b, x0, 4000, 1e-6, 0.0)
+    assert r["iterations"] == f64["iterations"]
+    assert rel(x, f64["x"]) < 1e-6
+    np.testing.assert_allclose(r["history"], f64["history"], rtol=1e-6)
+    if layout == "BSR6":
+        srv = wsb.Server(ctx, iters_per_step=3)
+        try:
+            xs, rs = srv.wait(srv.submit(rp, ci, v, bs, b, x0=x0, **kw), 60.0)
+        finally:
+            srv.close()
+        assert rs["iterations"] == r["iterations"]
+        assert np.array_equal(xs.view(np.uint32), x.view(np.uint32))

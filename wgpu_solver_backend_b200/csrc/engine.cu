@@ -210,11 +210,6 @@ Engine::Engine(Context *ctx, cudaStream_t stream) : ctx_(ctx), stream_(stream) {
     max_grid_a_ = std::max(1, occ_a) * std::max(1, ctx->sm_count);
     max_grid_b_ = std::max(1, occ_b) * std::max(1, ctx->sm_count);
     max_grid_c_ = std::max(1, occ_c) * std::max(1, ctx->sm_count);
-    for (int parts : {1, 2})
-        cudaFuncSetAttribute(team_kernel(parts, false), cudaFuncAttributeMaxDynamicSharedMemorySize, kTeamSmemMax);
-    cudaFuncSetAttribute(team_kernel(1, true), cudaFuncAttributeMaxDynamicSharedMemorySize, kTeamSmemMax);
-    for (bool sr : {false, true})
-        cudaFuncSetAttribute(stream_kernel(sr), cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmem);
     const char *loop_env = getenv("WSB_LOOP");
     use_graph_ = !(loop_env && std::strcmp(loop_env, "launch") == 0);
     cudaMallocHost(&h_sp_, sizeof(StepParams));
@@ -313,11 +308,11 @@ int Engine::push_changes() {
 }
 
 // Whether k_team iterates this system, and the team it needs: BSR6 (its
-// blocks are the preconditioner's blocks), the classic recurrence, and few
-// enough blocks for the shared memory of one CTA an SM in shared memory.
+// blocks are the preconditioner's blocks), few enough of them for the shared
+// memory of one CTA an SM.
 void Engine::team_plan(Slot *sl) const {
     const MatA &A = *sl->A;
-    if (!team_on_ || !use_graph_ || A.n == 0 || sl->cfg.algorithm != WSB_ALG_CLASSIC) return;
+    if (!team_on_ || !use_graph_ || A.n == 0) return;
     if (A.layout == LAYOUT_CSR) return team_plan_rows(sl);
     if (A.layout != LAYOUT_BSR6 || sl->M->nb != A.n / 6) return;
     const uint32_t nbr = A.n / 6, tiles = (nbr + kTeamWarpBrows - 1) / kTeamWarpBrows, sms = (uint32_t)ctx_->sm_count;
@@ -452,8 +447,7 @@ int Engine::finish_team_plans() {
 // where one system fills it: 22^3 nodes 11.5 us an iteration alone, 25 us in
 // the loop kernels, which need 9 us a system-iteration at 20^3 when eight share
 // them.)
-// The loop kernels keep what is left: CSR, longer block rows, and small
-// systems of the single-reduction recurrence.
+// The loop kernels keep what is left: large CSR systems, longer block rows.
 void Engine::stream_plan(Slot *sl) const {
     const MatA &A = *sl->A;
     if (!team_on_ || !use_graph_ || sl->team || A.layout != LAYOUT_BSR6 || A.n == 0 || sl->M->nb != A.n / 6) return;
@@ -1023,6 +1017,8 @@ int Engine::launch_team(const std::vector<uint32_t> &ids, bool csr, uint32_t lim
         Run pairs = simulate(true);
         if (pairs.end < run.end) run = std::move(pairs);
     }
+    const void *kernel = team_kernel((int)run.parts, csr, algo_ == (uint32_t)WSB_ALG_SINGLE_REDUCTION);
+    WSB_CUDA_TRY(ctx_, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTeamSmemMax));
     const auto &lists = run.lists;
     const uint32_t grid = (uint32_t)lists.size();
     size_t items = 0;
@@ -1052,7 +1048,7 @@ int Engine::launch_team(const std::vector<uint32_t> &ids, bool csr, uint32_t lim
     const TeamItem *ditems = reinterpret_cast<const TeamItem *>(mem.dev + head);
     const uint32_t *doff = mem.dev;
     void *args[] = {&dsys, &dsp, &ditems, &doff, &limit};
-    WSB_CUDA_TRY(ctx_, cudaLaunchCooperativeKernel(team_kernel((int)run.parts, csr), dim3(grid), dim3(kTeamThreads), args,
+    WSB_CUDA_TRY(ctx_, cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kTeamThreads), args,
                                                    (size_t)run.smem, stream_));
     launches_ += 1;
     return WSB_OK;
@@ -1065,8 +1061,9 @@ int Engine::launch_stream(const std::vector<uint32_t> &ids, uint32_t limit) {
         StepParams *dsp = d_sp_;
         uint32_t system = s;
         void *args[] = {&dsys, &dsp, &system, &limit};
-        WSB_CUDA_TRY(ctx_, cudaLaunchCooperativeKernel(stream_kernel(slots_[s]->cfg.algorithm == WSB_ALG_SINGLE_REDUCTION),
-                                                       dim3(slots_[s]->stream), dim3(kStreamThreads), args,
+        const void *kernel = stream_kernel(slots_[s]->cfg.algorithm == WSB_ALG_SINGLE_REDUCTION);
+        WSB_CUDA_TRY(ctx_, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmem));
+        WSB_CUDA_TRY(ctx_, cudaLaunchCooperativeKernel(kernel, dim3(slots_[s]->stream), dim3(kStreamThreads), args,
                                                        (size_t)kStreamSmem, stream_));
         launches_ += 1;
     }

@@ -21,8 +21,9 @@
 // Measured (B200, us an iteration, loop kernels -> here): 4^3 nodes 24.4 -> 2.8,
 // 9^3 23.5 -> 4.4, 12^3 24.8 -> 4.8, 17^3 25.7 -> 5.4, 21^3 27.5 -> 6.9; with
 // two parts a CTA 9^3 6.1, 14^3 6.8 (one: 4.9), 20^3 8.2 (6.8), and 22^3 8.1,
-// 24^3 9.0, 26^3 9.8 (in k_stream 11.5, 12.2, 12.6). 48 systems of 4^3 to 24^3
-// nodes at once: 27.6 ms -> 15.6.
+// 24^3 9.0, 26^3 9.8 (in k_stream 11.5, 12.2, 12.6). CSR: 4^3 21.3 -> 3.3, 19^3
+// 28.6 -> 6.7. Single reduction: 4^3 24.6 -> 3.2, 16^3 25.8 -> 5.2, 26^3 28.6 ->
+// 10.3. 48 systems of 4^3 to 24^3 nodes at once: 27.6 ms -> 15.6.
 // What is left is latency (7 of 13 warps wait at a barrier at any time, issue
 // slots 28 % used): per iteration two hops through the L2 (800 cycles for
 // 8 CTAs, 1,400 for 31), the FP64 sums (nine cycles an add, 36 with the shuffle
@@ -34,6 +35,13 @@
 // stay apart and made the code after it up to ten times slower.
 // Arithmetic is that of kernels_fused.cu operation by operation; only the
 // grouping of the FP64 sums differs.
+//
+// CSR (kCsr): rows of different lengths have no blocks of columns to share, so z
+// and p are kept once a CTA for every column it multiplies with, and each value
+// has the 16-bit place of its column (k_team_plan_csr).
+//
+// Single reduction (kSr): the product multiplies u = M r (in z), p and s = A p
+// are formed in the update; the exchanges are the same two.
 //
 // All CTAs of a launch are resident (cooperative launch); a CTA takes its
 // items in list order, and the lists are cut from one global order of systems,
@@ -58,6 +66,7 @@ struct TeamShared {
     double bb, rz_old, pap, alpha_d, rr, rel2, abs2;
     uint32_t iter, max_iter, status, breakdown;
     uint32_t bytes[2 * kTeamWarps];  // shared memory of each warp tile
+    double rz_prev;             // kSr: the r.z before rz_old
     alignas(16) double v[1];     // the rows' products of a reduction, twice 32 a warp tile
 };
 
@@ -97,7 +106,7 @@ __device__ __forceinline__ void part_sums(const double *v, uint32_t lane, double
 }
 
 // One system, this CTA's rows, up to `limit` iterations.
-template <int kT, bool kCsr>
+template <int kT, bool kCsr, bool kSr>
 __device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it, uint32_t limit, TeamShared &S,
                                                  char *dyn, const WaitCtl &w) {
     static_assert(!kCsr || kT == 1, "CSR: one part a CTA");
@@ -121,7 +130,7 @@ __device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it,
     const uint32_t bo = lane / 6u, a = lane % 6u;
     bool on[kT];
     uint32_t row[kT], k0[kT], nk[kT], cols[kT], most = 0;  // cols: most blocks of a block row of the warp tile
-    float x[kT], r[kT], z[kT], p[kT];
+    float x[kT], r[kT], z[kT], p[kT], s[kT];  // (s: kSr)
     // CSR: the warp tile's first row and block, its rows and blocks.
     uint32_t row0 = 0, blk0 = 0, n_rows = 0, n_blk = 0;
     if (kCsr && warp < tw && tile0 + warp < D.n_tiles) {
@@ -136,7 +145,7 @@ __device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it,
         on[t] = kCsr ? lane < n_rows : lane < (uint32_t)kTeamWarpRows && warp < tw && (uint32_t)t < it.parts && br < br1;
         row[t] = !on[t] ? 0u : kCsr ? row0 + lane : 6u * br + a;
         k0[t] = nk[t] = 0;
-        x[t] = r[t] = z[t] = p[t] = 0.0f;
+        x[t] = r[t] = z[t] = p[t] = s[t] = 0.0f;
         if (on[t]) {
             const uint32_t *ptr = kCsr ? D.row_ptr + row[t] : D.brow_ptr + br;
             k0[t] = ptr[0];
@@ -146,6 +155,7 @@ __device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it,
                 r[t] = D.r[row[t]];
                 z[t] = D.z[row[t]];
                 p[t] = D.p[row[t]];
+                if (kSr) s[t] = D.s[row[t]];
             }
         }
         cols[t] = __reduce_max_sync(kFull, nk[t]);
@@ -194,7 +204,7 @@ __device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it,
         val4 = reinterpret_cast<const float4 *>(val) + lane;
         idx4 = reinterpret_cast<const ushort4 *>(idx) + lane;
         if (n_rows) {
-            if (on[0]) px[32u * warp + lane] = fresh ? x[0] : p[0];
+            if (on[0]) px[32u * warp + lane] = fresh ? x[0] : kSr ? z[0] : p[0];
 #pragma unroll 1
             for (uint32_t j = 0; j < nk[0]; ++j) cp_async4(val + 4u * (32u * (j >> 2) + lane) + (j & 3u), D.val + k0[0] + j);
             const char *from = reinterpret_cast<const char *>(D.tile_idx + D.tile_off[tile0 + warp]);
@@ -207,13 +217,13 @@ __device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it,
                         q / 6u < m && q % 6u < m ? D.lu[36u * (size_t)(blk0 + lane) + q] : q % 7u == 0 ? 1.0f : 0.0f;
             }
         }
-        // The columns outside, their first entries of p (x0 when fresh).
+        // The columns outside, their first entries of p (kSr: u; x0 when fresh).
         const uint32_t n = D.ext_count[it.rank];
         if (tid == 0) S.ext = n;
         for (uint32_t i = tid; i < n; i += (uint32_t)kTeamThreads) {
             const uint32_t c = D.ext_cols[(size_t)it.rank * D.ext_cap + i];
             ext[i] = c;
-            px[kRows + i] = (fresh ? D.x : D.p)[c];
+            px[kRows + i] = (fresh ? D.x : kSr ? D.z : D.p)[c];
         }
     };
     auto load_bsr = [&](int t) {
@@ -229,8 +239,8 @@ __device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it,
         bc[t] += colp * bo;
         __syncwarp();
         if (on[t]) {
-            // p (or x0 for a fresh system) at the block columns, one component a lane.
-            const float *src = (fresh ? D.x : D.p) + a;
+            // p (kSr: u; x0 for a fresh system) at the block columns, one component a lane.
+            const float *src = (fresh ? D.x : kSr ? D.z : D.p) + a;
 #pragma unroll 1
             for (uint32_t j = 0; j < nk[t]; ++j) {
                 const float *v = D.bval + (size_t)(k0[t] + j) * 36u + 6u * a;
@@ -459,6 +469,11 @@ __device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it,
         S.rr = S.pap = S.alpha_d = S.beta = 0.0;
         S.beta_f = 0.0f;
         S.rz = S.rz_old = st->rz_old;
+        if (kSr && !fresh) {
+            S.rz_prev = st->gamma_prev;
+            S.alpha_d = st->alpha;
+            S.beta = st->beta;
+        }
         S.rel2 = st->rel2;
         S.abs2 = st->abs2;
         S.iter = st->iter;
@@ -502,12 +517,12 @@ __device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it,
         }
     };
     // p = z + beta p of the lane's rows and of their block columns (p = z when
-    // first). All operands come before the first store, which the compiler
+    // first; kSr: u = z at the columns, p is the update's). All operands come before the first store, which the compiler
     // could not move a load across.
     auto advance_bsr = [&](bool first, float bf) {
 #pragma unroll
         for (int t = 0; t < kT; ++t) {
-            p[t] = first ? z[t] : __fadd_rn(__fmul_rn(p[t], bf), z[t]);
+            if (!kSr) p[t] = first ? z[t] : __fadd_rn(__fmul_rn(p[t], bf), z[t]);
 #pragma unroll 1
             for (uint32_t j0 = 0; j0 < cols[t]; j0 += kAhead) {
                 float *dst = xg[t] + 8u * kTeamWarpBrows * j0 + a;
@@ -518,11 +533,11 @@ __device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it,
                     zn[4 * q] = zx[c.x + a], zn[4 * q + 1] = zx[c.y + a], zn[4 * q + 2] = zx[c.z + a], zn[4 * q + 3] = zx[c.w + a];
                 }
 #pragma unroll
-                for (int j = 0; j < kAhead; ++j) pn[j] = j0 + j < nk[t] ? dst[8u * kTeamWarpBrows * j] : 0.0f;
+                for (int j = 0; j < kAhead; ++j) pn[j] = !kSr && j0 + j < nk[t] ? dst[8u * kTeamWarpBrows * j] : 0.0f;
 #pragma unroll
                 for (int j = 0; j < kAhead; ++j)
                     if (j0 + j < nk[t])
-                        dst[8u * kTeamWarpBrows * j] = first ? zn[j] : __fadd_rn(__fmul_rn(pn[j], bf), zn[j]);
+                        dst[8u * kTeamWarpBrows * j] = kSr || first ? zn[j] : __fadd_rn(__fmul_rn(pn[j], bf), zn[j]);
             }
         }
         __syncwarp();
@@ -530,10 +545,10 @@ __device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it,
 
     // CSR: p at every column, once a CTA.
     auto advance_csr = [&](bool first, float bf) {
-        p[0] = first ? z[0] : __fadd_rn(__fmul_rn(p[0], bf), z[0]);
-        px[32u * warp + lane] = p[0];
+        if (!kSr) p[0] = first ? z[0] : __fadd_rn(__fmul_rn(p[0], bf), z[0]);
+        px[32u * warp + lane] = kSr ? z[0] : p[0];
         for (uint32_t i = kRows + tid; i < kRows + n_ext; i += kRows)
-            px[i] = first ? zx[i] : __fadd_rn(__fmul_rn(px[i], bf), zx[i]);
+            px[i] = kSr || first ? zx[i] : __fadd_rn(__fmul_rn(px[i], bf), zx[i]);
     };
 
     // Results of a reduction are written between its two barriers and read by
@@ -560,14 +575,25 @@ __device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it,
         } else {
             if (rows)
 #pragma unroll
-                for (int t = 0; t < kT; ++t) v0[t * kRows + tid] = (double)p[t] * (double)ap[t];
+                for (int t = 0; t < kT; ++t) v0[t * kRows + tid] = (double)(kSr ? z[t] : p[t]) * (double)ap[t];
             __syncthreads();
             if (red_a) {
                 const double rz_old = S.rz, pap = all_reduce(v0, 0, tag);
                 if (lane == 0) {
-                    const double alpha = quotient(rz_old, pap);
+                    double den = pap;
+                    if (kSr) {
+                        // alpha, beta from gamma = (r, u) and delta = (A u, u).
+                        double beta = 0.0;
+                        if (S.iter != 0) {
+                            beta = quotient(rz_old, S.rz_prev);
+                            den = S.alpha_d != 0.0 ? pap - quotient(beta * rz_old, S.alpha_d) : 0.0;
+                        }
+                        S.beta = beta;
+                        S.beta_f = (float)beta;
+                    }
+                    const double alpha = quotient(rz_old, den);
                     S.rz_old = rz_old;
-                    S.pap = pap;
+                    S.pap = den;
                     S.alpha_d = alpha;
                     S.alpha = make_uint2(__float_as_uint((float)alpha), S.err ? 0u : 1u);
                 }
@@ -576,11 +602,17 @@ __device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it,
             const uint2 al2 = S.alpha;
             if (!al2.y) break;
             const float al = __uint_as_float(al2.x), ma = -al;
+            const float bf = kSr ? S.beta_f : 0.0f;
+            const bool first = kSr && S.iter == 0;
             if (rows)
 #pragma unroll
                 for (int t = 0; t < kT; ++t) {
+                    if (kSr) {
+                        p[t] = first ? z[t] : __fadd_rn(__fmul_rn(p[t], bf), z[t]);
+                        s[t] = first ? ap[t] : __fadd_rn(__fmul_rn(s[t], bf), ap[t]);
+                    }
                     x[t] = __fadd_rn(x[t], __fmul_rn(al, p[t]));
-                    r[t] = __fadd_rn(r[t], __fmul_rn(ma, ap[t]));
+                    r[t] = __fadd_rn(r[t], __fmul_rn(ma, kSr ? s[t] : ap[t]));
                     if (!on[t]) r[t] = 0.0f;
                 }
         }
@@ -597,9 +629,13 @@ __device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it,
         if (red_a || red_b) {
             const double sum = all_reduce(red_a ? v0 : v1, red_a ? 1u : 2u, tag);
             if (lane == 0 && red_b) {
-                const double beta = quotient(sum, S.rz);
-                S.beta = beta;
-                S.beta_f = (float)beta;
+                if (kSr) {
+                    S.rz_prev = S.rz_old;
+                } else {
+                    const double beta = quotient(sum, S.rz);
+                    S.beta = beta;
+                    S.beta_f = (float)beta;
+                }
                 S.rz = sum;
             } else if (lane == 0) {
                 uint32_t status = ST_RUNNING;
@@ -653,11 +689,13 @@ __device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it,
             D.r[row[t]] = r[t];
             D.z[row[t]] = z[t];
             D.p[row[t]] = p[t];
+            if (kSr) D.s[row[t]] = s[t];
         }
     if (lead && red_a && lane == 0) {
         const bool running = S.status == ST_RUNNING, none = S.iter == 0;  // none: stopped before the first iteration
         st->bb = S.bb;
         st->rz_old = running || none ? S.rz : S.rz_old;
+        if (kSr) st->gamma_prev = S.rz_prev;
         st->pap = S.pap;
         st->rr = S.rr;
         st->rz_new = none ? 0.0 : S.rz;
@@ -674,7 +712,7 @@ __device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it,
     }
 }
 
-template <int kT, bool kCsr>
+template <int kT, bool kCsr, bool kSr>
 __global__ void __launch_bounds__(kTeamThreads, 1)
     k_team(const SysDesc *__restrict__ sys, StepParams *sp, const TeamItem *__restrict__ items,
            const uint32_t *__restrict__ item_off, uint32_t limit) {
@@ -688,7 +726,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
     const uint32_t i1 = item_off[blockIdx.x + 1];
     for (uint32_t i = item_off[blockIdx.x]; i < i1; ++i) {
         const TeamItem it = items[i];
-        team_system<kT, kCsr>(sys[it.sys], it, limit, S, smem + team_fixed_bytes(kT), w);
+        team_system<kT, kCsr, kSr>(sys[it.sys], it, limit, S, smem + team_fixed_bytes(kT), w);
         __syncthreads();
         if (S.err) return;  // every CTA's later waits would run out as well
     }
@@ -765,8 +803,14 @@ __global__ void __launch_bounds__(kPlanThreads) k_team_plan_csr(SysDesc D, uint3
 
 }  // namespace
 
-const void *team_kernel(int parts, bool csr) {
-    return csr ? (const void *)k_team<1, true> : parts == 1 ? (const void *)k_team<1, false> : (const void *)k_team<2, false>;
+template <bool kSr>
+static const void *team_kernel_of(int parts, bool csr) {
+    return csr          ? (const void *)k_team<1, true, kSr>
+           : parts == 1 ? (const void *)k_team<1, false, kSr>
+                        : (const void *)k_team<2, false, kSr>;
+}
+const void *team_kernel(int parts, bool csr, bool single_reduction) {
+    return single_reduction ? team_kernel_of<true>(parts, csr) : team_kernel_of<false>(parts, csr);
 }
 
 cudaError_t team_plan_csr(const SysDesc &D, uint32_t *count, uint32_t *most, uint32_t parts, cudaStream_t st) {

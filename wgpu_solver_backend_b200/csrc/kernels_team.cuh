@@ -69,7 +69,7 @@ __host__ __device__ constexpr uint64_t team_red_entries(uint32_t size) {
 // not fit in what L1 the shared memory leaves: 26 systems of 9^3 nodes 13.5 us
 // an iteration against 10.7; so did one CTA of 24 warp tiles, 4^3 nodes 5.5 us
 // against 2.9.)
-const void *team_kernel(int parts, bool csr);
+const void *team_kernel(int parts, bool csr, bool single_reduction);
 // Fills D.tile_idx, D.ext_cols and D.ext_count (= count) of a CSR system whose
 // tiles are set, `parts` parts of D.team_warps tiles. most[0] becomes the most
 // columns outside a part, most[1] whether that is more than D.ext_cap (nothing
