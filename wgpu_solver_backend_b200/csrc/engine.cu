@@ -953,8 +953,8 @@ int Engine::finish_slot(uint32_t s, int status) {
 // could not start before it, so wide ones do not starve), with one or with two
 // parts a CTA, whichever run ends first: a pair takes about 1.4 times as long
 // on half the CTAs, which pays once systems wait for CTAs (B200, us a
-// system-iteration, one part against two: 24 systems of 14^3 nodes 1.74 and
-// 1.14, 13 of 9^3 0.38 and 0.49). A solve takes about twenty times the fourth
+// system-iteration, one part against two: 24 systems of 14^3 nodes 1.6 and 1.05,
+// 3 of them 1.6 and 2.2). A solve takes about twenty times the fourth
 // root of its rows in iterations; the time of one is fitted to measured ones.
 // Every CTA's list is in the order in which systems start, so no two systems
 // wait for each other whatever the times turn out to be.
@@ -1004,7 +1004,7 @@ int Engine::launch_team(const std::vector<uint32_t> &ids, bool csr, uint32_t lim
             std::vector<uint32_t> ctas(idle.rbegin(), idle.rbegin() + width);
             idle.resize(idle.size() - width);
             for (uint32_t k = 0; k < width; ++k) run.lists[ctas[k]].push_back({s, k * parts, sl.team, parts});
-            const double us = width == 1 ? 3.0 * parts : parts == 1 ? 4.1 + 0.021 * width : 5.9 + 0.033 * width;
+            const double us = width == 1 ? 3.0 * parts : parts == 1 ? 4.2 + 0.008 * width : 6.2 + 0.004 * width;
             const double end = now + us * std::min<double>(limit, 20.0 * std::pow((double)sl.A->n, 0.25));
             run.end = std::max(run.end, end);
             running.emplace(end, std::move(ctas));

@@ -4,6 +4,7 @@
 // WSB_PREC_REFERENCE_F32 solve, whose iterates are bit-identical to the CPU
 // restatement of compute.rs:189-495.
 #include "kernels_ref.cuh"
+#include "kernels_team.cuh"
 #include "team_device.cuh"
 
 namespace wsb {
@@ -240,10 +241,10 @@ cudaError_t ref_dot(cudaStream_t st, uint32_t n, const float *a, const float *b,
 // nonzero instead), so p = beta p + z is formed once for each.
 // Blocks cross the CTAs' rows: a CTA also keeps r of up to five rows on either
 // side and solves every block of its rows.
-// Measured (B200, us an iteration, passes -> here): 4^3 nodes 27.4 -> 4.7, 9^3
-// 31.1 -> 5.9, 12^3 30.8 -> 6.2, 16^3 33.6 -> 8.5; with two CTAs an SM 19^3 34.0
-// -> 14.3, 23^3 40.1 -> 17.2. What is left is latency: two exchanges, the
-// fence, the gather of p and z, one row sum, one block solve.
+// Measured (B200, us an iteration, passes -> here): 4^3 nodes 27.4 -> 4.0, 9^3
+// 31.1 -> 5.5, 12^3 30.8 -> 6.2, 16^3 33.6 -> 6.0; with two CTAs an SM 19^3 34.0
+// -> 7.6, 23^3 40.1 -> 10.7. What is left is latency: two exchanges, the fence,
+// the gather of p and z, one row sum, one block solve.
 namespace {
 
 struct RefShared {
@@ -275,24 +276,29 @@ __device__ __forceinline__ float tree256_warp(F get) {
 // `release`: the CTA's writes come before the partial.
 __device__ __forceinline__ float ref_all_sum(const float *prod, unsigned long long *parts, uint32_t tag, bool release,
                                              RefShared &S, RefState *st) {
-    const uint32_t lane = threadIdx.x & 31u, wgs = gridDim.x;
+    const uint32_t lane = threadIdx.x & 31u, wgs = gridDim.x, copies = team_copies(wgs);
     float v = tree256_warp([&](uint32_t i) { return prod[i]; });
     if (wgs == 1) return v;
     if (release) __threadfence();
-    if (lane == 0) st_packet(parts + blockIdx.x, v, tag);
+    v = __shfl_sync(kFull, v, 0);
+    if (lane < copies) st_packet(parts + (size_t)lane * 3u * wgs + blockIdx.x, v, tag);
     __syncwarp();
+    parts += (size_t)(blockIdx.x % copies) * 3u * wgs;
+    team_quiet(quiet_cycles(wgs));
     const long long t0 = clock64();
     uint32_t len = wgs;
     float mine = 0.0f;  // lane g: the tree over partials [256 g, 256 g + 256)
     for (uint32_t g = 0; 256u * g < wgs; ++g) {
         unsigned long long q[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) q[j] = 256u * g + lane + 32u * j < wgs ? 0ull : (unsigned long long)tag << 32;
 #pragma unroll 1
         for (uint32_t k = 1;; ++k) {
             bool ok = true;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                const uint32_t i = 256u * g + lane + 32u * j;
-                q[j] = ld_packet_if(parts + (i < wgs ? i : 0u), i < wgs, (unsigned long long)tag << 32);
+                const bool want = (uint32_t)(q[j] >> 32) != tag;
+                q[j] = ld_packet_if(parts + (want ? 256u * g + lane + 32u * j : 0u), want, q[j]);
             }
 #pragma unroll
             for (int j = 0; j < 8; ++j) ok = ok && (uint32_t)(q[j] >> 32) == tag;

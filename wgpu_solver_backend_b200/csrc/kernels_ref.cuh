@@ -49,7 +49,7 @@ struct RefPcg {
     const uint32_t *bs;     // block starts, strictly increasing
     const float *b;
     float *x, *z, *p0, *p1;            // x: x0, then the solution
-    unsigned long long *parts;         // 3 x CTAs published partials, zero at first
+    unsigned long long *parts;         // published partials, 3 a CTA in each of team_copies(CTAs) copies, zero at first
     RefState *st;                      // tolerances and limit; the outcome
     double *history;
     uint64_t hist_cap;

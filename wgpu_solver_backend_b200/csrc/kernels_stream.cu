@@ -21,14 +21,14 @@
 // Arithmetic is that of kernels_fused.cu operation by operation; only the
 // grouping of the FP64 sums differs (per lane over its tiles, warp, CTA, device).
 //
-// Measured (B200, us an iteration, loop kernels -> here): 24^3 nodes 27.5 ->
-// 12.2, 32^3 31.8 -> 15.0, 40^3 41.5 -> 20.8 (single reduction 39.2 -> 20.8),
-// 64^3 87.0 -> 61.5, 80^3 145.9 -> 115.5 (and 13.0, 15.8, 21.8, 65, 123 with
-// the gathers behind the wait for the tile's values). At 80^3 the product runs
-// at the copy rate of HBM; up to 40^3 the two all-reduces (1.7 us each over 148
-// CTAs, as long alone) and the latencies around them are half of the time, and
-// the product (200 cycles a tile and SM; its bytes need 70 from the L2) waits
-// for shared-memory and gather wavefronts, 60 % of what the SM can issue.
+// Measured (B200, us an iteration, loop kernels -> here): 32^3 nodes 31.8 ->
+// 13.0, 40^3 41.5 -> 19.0 (single reduction 39.2 -> 19.0), 64^3 87.0 -> 61.3,
+// 80^3 145.9 -> 114.5 (with the gathers behind the wait for the tile's values
+// 15.2, 21, 65, 122). At 80^3 the product runs at the copy rate of HBM; up to
+// 40^3 the two all-reduces (1.5 us each over 148 CTAs, as long alone) and the
+// latencies around them are half of the time, and the product (200 cycles a
+// tile and SM; its bytes need 70 from the L2) waits for shared-memory and
+// gather wavefronts, 60 % of what the SM can issue.
 //
 // Single reduction (kSr): the update phase comes first with alpha and beta of
 // the last iteration; the product multiplies u = M r (in z).
@@ -467,7 +467,7 @@ __device__ __forceinline__ void stream_system(const SysDesc &D, uint32_t limit, 
         start_u();
         if (warp < tiles_u) fetch_u(warp, p_new);
         if (warp == 0) {
-            if (gridDim.x > 1) pap = team_gather(&S.err, red, gridDim.x, tag, sp, lim);
+            if (gridDim.x > 1) pap = team_gather(&S.err, red, gridDim.x, tag, sp, lim, 0);
             if (lane == 0) {
                 double alpha;
                 if (kSr) {
@@ -512,7 +512,7 @@ __device__ __forceinline__ void stream_system(const SysDesc &D, uint32_t limit, 
         if (warp < 2) sum = publish(S, warp, out + slot, copies, tag, true);
         start_a();
         if (warp < 2 && gridDim.x > 1) {
-            sum = team_gather(&S.err, red + slot, gridDim.x, tag, sp, lim);
+            sum = team_gather(&S.err, red + slot, gridDim.x, tag, sp, lim, 0);
             __threadfence();  // what the publishers wrote is visible after this
         }
         if (warp == 1) {

@@ -19,17 +19,17 @@
 //     multiplies (same operation, same bits as the owner's), so p is never
 //     exchanged.
 // Measured (B200, us an iteration, loop kernels -> here): 4^3 nodes 24.4 -> 2.8,
-// 9^3 23.5 -> 4.4, 12^3 24.8 -> 4.8, 17^3 25.7 -> 5.4, 21^3 27.5 -> 6.9; with
-// two parts a CTA 9^3 6.1, 14^3 6.8 (one: 4.9), 20^3 8.2 (6.8), and 22^3 8.1,
-// 24^3 9.0, 26^3 9.8 (in k_stream 11.5, 12.2, 12.6). CSR: 4^3 21.3 -> 3.3, 19^3
-// 28.6 -> 6.7. Single reduction: 4^3 24.6 -> 3.2, 16^3 25.8 -> 5.2, 26^3 28.6 ->
-// 10.3. 48 systems of 4^3 to 24^3 nodes at once: 27.6 ms -> 15.6.
+// 9^3 23.5 -> 4.3, 12^3 24.8 -> 4.6, 17^3 25.7 -> 4.6, 21^3 27.5 -> 5.3; with
+// two parts a CTA 9^3 6.0, 14^3 6.5 (one: 4.6), 20^3 6.8 (5.3), and 22^3 6.7,
+// 24^3 6.7, 26^3 6.8 (in k_stream 10.5 to 11). CSR: 4^3 21.3 -> 3.2, 19^3 28.6
+// -> 5.7. Single reduction: 4^3 24.6 -> 3.2, 16^3 25.8 -> 5.0, 26^3 28.6 -> 7.2.
+// 48 systems of 4^3 to 24^3 nodes at once: 27.6 ms -> 13.7.
 // What is left is latency (7 of 13 warps wait at a barrier at any time, issue
 // slots 28 % used): per iteration two hops through the L2 (800 cycles for
 // 8 CTAs, 1,400 for 31), the FP64 sums (nine cycles an add, 36 with the shuffle
 // between lanes), two FP64 divisions and the block solve. So products are
 // added through shared memory, 14 per lane as a tree, before the lanes, and two
-// parts' side by side (one after the other: 22^3 8.7 us, 20^3 8.8); a block
+// parts' side by side (one after the other: 0.6 us more at 22^3); a block
 // is solved by one lane from shared memory (no shuffles between its steps); and
 // all waits are warp-uniform loops: lanes that leave such a loop one by one
 // stay apart and made the code after it up to ten times slower.
@@ -462,7 +462,7 @@ __device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it,
         }
         if (publisher) st_entry(out + slot * it.size, s, tag);
         __syncwarp();
-        return team_gather(&S.err, red + slot * it.size, entries, tag, w.sp, w.lim);
+        return team_gather(&S.err, red + slot * it.size, entries, tag, w.sp, w.lim, quiet_cycles(entries));
     };
     if (red_a && lane == 0) {
         S.bb = st->bb;
@@ -489,7 +489,11 @@ __device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it,
         const uint32_t step = 32u * tw;
 #pragma unroll 1
         for (uint32_t b = 0; b < n_ext; b += kBatch * step) {
+            // (Only packets that have not come are asked for again: the polls of
+            // all CTAs hold up the stores that they wait for.)
             unsigned long long zin[kBatch];
+#pragma unroll
+            for (uint32_t q = 0; q < kBatch; ++q) zin[q] = b + q * step + tid < n_ext ? 0ull : (unsigned long long)tag << 32;
             const long long t0 = clock64();
 #pragma unroll 1
             for (uint32_t k = 1;; ++k) {
@@ -497,8 +501,8 @@ __device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it,
 #pragma unroll
                 for (uint32_t q = 0; q < kBatch; ++q) {
                     const uint32_t i = b + q * step + tid, e = i / 6u;
-                    const bool want = i < n_ext;
-                    zin[q] = ld_packet_if(zpk + (!want ? 0u : kCsr ? ext[i] : ext[e] + (i - 6u * e)), want, (unsigned long long)tag << 32);
+                    const bool want = (uint32_t)(zin[q] >> 32) != tag;
+                    zin[q] = ld_packet_if(zpk + (!want ? 0u : kCsr ? ext[i] : ext[e] + (i - 6u * e)), want, zin[q]);
                 }
 #pragma unroll
                 for (uint32_t q = 0; q < kBatch; ++q) bad |= (uint32_t)(zin[q] >> 32) ^ tag;

@@ -53,9 +53,11 @@ static_assert(kTeamLuBytes % 16 == 0 && kTeamColBytes % 16 == 0 && kTeamIdxBytes
 
 // Copies of the published partials of a team, each read by every copies-th
 // CTA: with one copy, the polls of a hundred CTAs on the same few cache lines
-// hold up the stores (106 CTAs: 8.6 us an iteration against 7.5 with four);
-// fewer CTAs are faster with one store (71 CTAs: 6.1 against 6.8 with three).
-__host__ __device__ constexpr uint32_t team_copies(uint32_t size) { return size <= 96u ? 1u : 4u; }
+// hold up the stores; fewer CTAs are faster with one store (B200, us an
+// iteration with one, four and eight copies: 77 parts 5.4, 5.8, 5.7; 90 parts
+// 7.0, 5.9, 5.8; 164 parts on 82 CTAs -, 8.2, 7.9; 148 CTAs in k_stream -, 13.5,
+// 13.4).
+__host__ __device__ constexpr uint32_t team_copies(uint32_t size) { return size <= 80u ? 1u : 8u; }
 __host__ __device__ constexpr uint64_t team_red_entries(uint32_t size) {
     return (uint64_t)kRedEntries * size * team_copies(size);
 }

@@ -15,14 +15,17 @@ __device__ __forceinline__ void st_entry(RedEntry *e, double v, uint32_t tag) {
                  "l"(__double_as_longlong(v)), "l"((long long)tag)
                  : "memory");
 }
-__device__ __forceinline__ bool ld_entry(const RedEntry *e, uint32_t tag, double *v) {
-    long long lo, hi;
-    asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
-                 : "=l"(lo), "=l"(hi)
-                 : "l"(e)
-                 : "memory");
+// Loads the entry where `miss`, which is cleared when it has arrived.
+__device__ __forceinline__ void ld_entry_if(const RedEntry *e, bool &miss, uint32_t tag, double *v) {
+    long long lo = __double_as_longlong(*v), hi = tag;
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t.reg .b128 t;\n\tsetp.ne.u32 q, %3, 0;\n\tmov.b128 t, {%0, %1};\n\t"
+        "@q ld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+        : "+l"(lo), "+l"(hi)
+        : "l"(e), "r"((uint32_t)miss)
+        : "memory");
     *v = __longlong_as_double(lo);
-    return (uint32_t)hi == tag;
+    miss = miss && (uint32_t)hi != tag;
 }
 __device__ __forceinline__ void st_packet(unsigned long long *p, float v, uint32_t tag) {
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p),
@@ -74,26 +77,47 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
+constexpr int kPollBatch = 5;
+// A partial takes about 700 cycles to the L2 and on to a reader, so polls
+// before that only hold up the stores. Where the CTAs of a team publish at
+// nearly the same time (k_team, k_ref_pcg) and are many, the first poll waits
+// (B200, us an iteration without, with 350, 650 and 1000 cycles: 63 parts 4.7,
+// 4.8, 5.1, 5.5; 77 parts 5.3, 4.6, 4.9, 5.2; 124 parts 6.3, 5.9, 5.4, 5.5; 26^3
+// nodes, 136 CTAs, 8.3, 7.7, 6.9, 6.9; in k_stream, 32^3, 13.0, 13.3, 13.5, 14.0).
+__device__ __forceinline__ int quiet_cycles(uint32_t size) { return size <= 64u ? 0 : size <= 80u ? 350 : 700; }
+__device__ __forceinline__ void team_quiet(int cycles) {
+    if (cycles == 0) return;
+    const long long t0 = clock64();
+    while (clock64() - t0 < cycles) {}
+    __syncwarp();
+}
 // Sum over the team of the partials in red[0 .. size), by one warp: lane l adds
 // entries l, l + 32, ... in order, then the lanes; valid in lane 0. Each round
-// keeps kPollBatch loads a lane in flight. *err is set when the wait runs out.
-constexpr int kPollBatch = 5;
+// keeps up to kPollBatch loads a lane in flight, for the entries that have not
+// come (with all of them loaded again the polls hold up the stores they wait
+// for: k_stream, 148 CTAs, 15.0 us an iteration on 32^3 nodes against 13.5;
+// k_team, 124 CTAs, 6.7 against 6.2), the first after `quiet` cycles. *err is
+// set when the wait runs out.
 __device__ __noinline__ double team_gather(uint32_t *err, const RedEntry *red, uint32_t size, uint32_t tag, StepParams *sp,
-                                           long long lim) {
+                                           long long lim, int quiet) {
     const uint32_t lane = threadIdx.x & 31u;
     double sum = 0.0;
     const long long t0 = clock64();
+    team_quiet(quiet);
 #pragma unroll 1
     for (uint32_t b = 0; b < size; b += 32u * kPollBatch) {
-        double v[kPollBatch];
+        double v[kPollBatch] = {};
+        bool miss[kPollBatch];
+#pragma unroll
+        for (int j = 0; j < kPollBatch; ++j) miss[j] = b + 32u * j + lane < size;
 #pragma unroll 1
         for (uint32_t k = 1;; ++k) {
-            bool ok = true;
+            bool any = false;
 #pragma unroll
-            for (int j = 0; j < kPollBatch; ++j) {
-                if (b + 32u * j < size) ok = ld_entry(red + min(b + 32u * j + lane, size - 1u), tag, &v[j]) && ok;
-            }
-            if (__all_sync(kFull, ok)) break;
+            for (int j = 0; j < kPollBatch; ++j) ld_entry_if(red + min(b + 32u * j + lane, size - 1u), miss[j], tag, &v[j]);
+#pragma unroll
+            for (int j = 0; j < kPollBatch; ++j) any = any || miss[j];
+            if (!__any_sync(kFull, any)) break;
             if (__any_sync(kFull, clock64() - t0 > lim) || ((k & 255u) == 0 && __any_sync(kFull, ld_error(sp) != 0))) {
                 *err = 1;
                 return 0.0;
