@@ -314,8 +314,7 @@ __device__ __forceinline__ void stream_system(const SysDesc &D, uint32_t limit, 
     };
 
     // ---- update phase ------------------------------------------------------
-    // Slices of a stage: x, r (kSr: p, s), which come and go by bulk copies,
-    // and the new z. What the product has just written (A p and p; kSr: w) and
+    // Slices of a stage: x, r (kSr: p, s), which come and go by bulk copies. What the product has just written (A p and p; kSr: w) and
     // u = z are read and z is written by plain accesses: a bulk load of them
     // would need a proxy fence behind the product, and a bulk store of z would
     // have to be waited for before the reduction. (z as {value, tag} packets,
@@ -359,7 +358,6 @@ __device__ __forceinline__ void stream_system(const SysDesc &D, uint32_t limit, 
         for (uint32_t u = warp; u < tiles_u; u += kStreamWarps, s ^= 1u) {
             const uint32_t r0 = b0 + u * tu, nb = min(tu, b1 - r0);
             wait_stage(s);
-            float *const zs = slice(s, kVecs);
             if (lane < nb) {
                 const float ma = -al;
                 float2 *const x2 = reinterpret_cast<float2 *>(slice(s, 0)) + 3u * lane;
@@ -411,25 +409,23 @@ __device__ __forceinline__ void stream_system(const SysDesc &D, uint32_t limit, 
                     y[i] = __fdiv_rn(t, L[7 * i]);
                 }
 #pragma unroll
-                for (int q = 0; q < 3; ++q) reinterpret_cast<float2 *>(zs)[3u * lane + q] = make_float2(y[2 * q], y[2 * q + 1]);
+                for (int q = 0; q < 3; ++q)
+                    reinterpret_cast<float2 *>(D.z + 6u * (size_t)(r0 + lane))[q] = make_float2(y[2 * q], y[2 * q + 1]);
 #pragma unroll
                 for (int i = 0; i < 6; ++i) rz += (double)r[i] * (double)y[i];
             }
             // x and r (p and s) go out by bulk stores, all but the last 8
-            // bytes of an odd number of block rows; z by coalesced stores.
+            // bytes of an odd number of block rows.
             fence_proxy_smem();
             __syncwarp();
             const size_t i0 = 6u * (size_t)r0;
             const uint32_t bytes = (24u * nb) & ~15u;
-            for (uint32_t q = lane; q < bytes / 16u; q += 32u)
-                reinterpret_cast<float4 *>(D.z + i0)[q] = reinterpret_cast<const float4 *>(zs)[q];
             if (lane < kVecs) {
                 bulk_store(vec(lane) + i0, slice(s, lane), bytes);
                 bulk_commit();
             }
             if (24u * nb > bytes && lane < 2u) {
                 const uint32_t o = bytes / 4u + lane;
-                D.z[i0 + o] = zs[o];
 #pragma unroll
                 for (uint32_t v = 0; v < kVecs; ++v) vec(v)[i0 + o] = slice(s, v)[o];
                 fence_proxy_all();  // read by the next update's bulk loads

@@ -17,11 +17,11 @@ constexpr int kStreamSpmvStage = 144 * kStreamMaxBlocks;
 constexpr int kStreamColBytes = 4 * ((kStreamMaxBlocks + 3) / 4 * 4);     // a tile's block columns
 constexpr int kStreamXgBytes = 32 * (kStreamBrows + 1) * kStreamMaxCols;  // p at a tile's block columns
 // Update tiles: up to kStreamUpd(Sr)Brows block rows, one a lane: the factors,
-// the slices of x and r (kSr: p and s too) and the new z.
+// the slices of x and r (kSr: p and s too).
 constexpr int kStreamUpdBrows = 32;
-constexpr int kStreamUpdBrowsSr = 26;
-constexpr int kStreamUpdStage = kStreamUpdBrows * (144 + 3 * 24);
-static_assert(kStreamUpdBrowsSr * (144 + 5 * 24) <= kStreamUpdStage, "update stages");
+constexpr int kStreamUpdBrowsSr = 28;
+constexpr int kStreamUpdStage = kStreamUpdBrowsSr * (144 + 4 * 24);
+static_assert(kStreamUpdBrows * (144 + 2 * 24) <= kStreamUpdStage, "update stages");
 static_assert(kStreamUpdBrows % 2 == 0 && kStreamUpdBrowsSr % 2 == 0, "16-byte slices");
 // Each warp has two stages, used by both phases.
 constexpr int kStreamWarpBytes = 2 * kStreamUpdStage;
