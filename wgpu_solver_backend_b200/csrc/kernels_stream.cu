@@ -353,6 +353,24 @@ __device__ __forceinline__ void stream_system(const SysDesc &D, uint32_t limit, 
             }
         }
     };
+    // Bulk stores of a tile's x and r (p and s), all but the last 8 bytes of an
+    // odd number of block rows.
+    auto store_u = [&](uint32_t u, uint32_t s) {
+        const uint32_t r0 = b0 + u * tu, nb = min(tu, b1 - r0);
+        if (lane < kVecs) {
+            bulk_store(vec(lane) + 6u * (size_t)r0, slice(s, lane), (24u * nb) & ~15u);
+            bulk_commit();
+        }
+    };
+    // Those of the warp's last tile wait until the partials are published: the
+    // fence before that would wait for them.
+    uint32_t last_u = 0, last_s = 0;
+    auto finish_u = [&]() {
+        if (warp < tiles_u) store_u(last_u, last_s);
+        if (lane < kVecs) bulk_wait_read();  // the stages are free
+        fence_proxy_smem();
+        __syncwarp();
+    };
     auto update = [&](float al, float bf, bool first, const float *pn, double &rr, double &rz) {
         uint32_t s = 0;
         for (uint32_t u = warp; u < tiles_u; u += kStreamWarps, s ^= 1u) {
@@ -414,16 +432,13 @@ __device__ __forceinline__ void stream_system(const SysDesc &D, uint32_t limit, 
 #pragma unroll
                 for (int i = 0; i < 6; ++i) rz += (double)r[i] * (double)y[i];
             }
-            // x and r (p and s) go out by bulk stores, all but the last 8
-            // bytes of an odd number of block rows.
             fence_proxy_smem();
             __syncwarp();
             const size_t i0 = 6u * (size_t)r0;
             const uint32_t bytes = (24u * nb) & ~15u;
-            if (lane < kVecs) {
-                bulk_store(vec(lane) + i0, slice(s, lane), bytes);
-                bulk_commit();
-            }
+            last_u = u;
+            last_s = s;
+            if (u + kStreamWarps < tiles_u) store_u(u, s);
             if (24u * nb > bytes && lane < 2u) {
                 const uint32_t o = bytes / 4u + lane;
 #pragma unroll
@@ -438,9 +453,6 @@ __device__ __forceinline__ void stream_system(const SysDesc &D, uint32_t limit, 
                 issue_u(u + 2 * kStreamWarps, s);
             }
         }
-        if (lane < kVecs) bulk_wait_read();  // the stages are free
-        fence_proxy_smem();
-        __syncwarp();
     };
 
     // ---- iterations --------------------------------------------------------
@@ -495,7 +507,10 @@ __device__ __forceinline__ void stream_system(const SysDesc &D, uint32_t limit, 
         rr = warp_sum(rr);
         rz = warp_sum(rz);
         asked = go;
-        if (!go) break;
+        if (!go) {
+            finish_u();
+            break;
+        }
         if (lane == 0) {
             S.w[0][warp] = rr;
             S.w[1][warp] = rz;
@@ -506,6 +521,7 @@ __device__ __forceinline__ void stream_system(const SysDesc &D, uint32_t limit, 
         const uint32_t slot = (warp + 1u) * gridDim.x;
         double sum = 0.0;
         if (warp < 2) sum = publish(S, warp, out + slot, copies, tag, true);
+        finish_u();
         start_a();
         if (warp < 2 && gridDim.x > 1) {
             sum = team_gather(&S.err, red + slot, gridDim.x, tag, sp, lim, 0);
