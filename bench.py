@@ -258,7 +258,7 @@ def run_plain(args, world, rank, local):
                      "peak_kind": peak_kind, **spmv_traffic(info["spmv_bytes"]),
                      "algorithmic_bytes_per_launch": info["spmv_bytes"], "launch_us": spmv_s * 1e6},
         "iteration_gbs": iter_gbs, "iteration_frac": iter_gbs / peak, "kernels": kernels,
-        "gpu_launches": args.steps * (2 + 1 + 3 * iters),
+        "gpu_launches": args.steps * int(res["kernel_launches"]),
         "clocks": clk,
     }
     if rank == 0 and world == 1:
