@@ -107,10 +107,11 @@ struct SolveOutcome {
 
 // Multi-system PCG engine. Systems are slots; each owns its Krylov vectors,
 // partial buffers and state in HBM. A slot is iterated by one of three paths,
-// chosen when it is added: systems that fit in the shared memory of a team of
-// CTAs by one cooperative launch of k_team (team_plan); larger BSR6 systems
-// one after the other by k_stream (stream_plan); the rest (CSR, long block
-// rows) together by one captured graph: a gate kernel, then a while loop of
+// chosen when it is added (CSR: before its first step): systems that fit in the
+// shared memory of a team of CTAs by one cooperative launch of k_team
+// (team_plan); larger BSR6 systems one after the other by k_stream
+// (stream_plan); the rest (large CSR systems, long block rows) together by one
+// captured graph: a gate kernel, then a while loop of
 // {k_spmv, k_update, k_pupdate} that ends when no slot is active or after
 // loop_limit iterations. Between steps the host retires finished slots,
 // restarts refinement sweeps and rebuilds the work lists.

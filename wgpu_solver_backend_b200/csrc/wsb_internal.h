@@ -142,7 +142,7 @@ struct SysDesc {
     double *history;                   // hist_cap entries or null
     uint32_t algo;                     // Algo
     uint32_t team_warps;               // k_team: warp tiles of a part
-    uint32_t team_ext[2];              // k_team: most blocks outside a CTA's rows that it multiplies with, one or two parts a CTA
+    uint32_t team_ext[2];              // k_team: most blocks (CSR: columns) a CTA may fetch z of, one or two parts a CTA
     uint32_t team_pairs;               // k_team: always two parts a CTA, one partial for both
     // k_team, CSR: first row and first block of each warp tile (n_tiles + 1),
     // where its columns' places start in tile_idx, the places; of each part the
