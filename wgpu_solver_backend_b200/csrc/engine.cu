@@ -660,7 +660,9 @@ uint32_t Engine::active_count() const {
 
 void Engine::remove(uint32_t s) {
     if (s >= slots_.size() || !slots_[s]) return;
-    if (slots_[s]->phase == Slot::RUNNING && slots_[s]->looped()) work_dirty_ = true;
+    // The work lists may still name it, also when it has stopped (step()), and the
+    // next upload of the descriptors takes this one from the device.
+    if (slots_[s]->looped()) work_dirty_ = true;
     cudaFreeAsync(slots_[s]->mem, stream_);
     slots_[s].reset();
     std::memset(h_sys_ + s, 0, sizeof(SysDesc));
