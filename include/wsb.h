@@ -74,10 +74,13 @@ int wsb_context_adapter_info(const wsb_context *ctx, wsb_adapter_info *out);
 int wsb_context_set_stream(wsb_context *ctx, void *cuda_stream);
 int wsb_context_synchronize(wsb_context *ctx);
 /* Failure detection (no counterpart in the reference, which blocks on
- * futures without a limit): every wait of the pipelined solver kernels gives
- * up after `cycles` SM clock cycles (0 restores the default of about 2 s);
- * the kernel then records the wait, drains its own copies in flight and
- * returns, and the solve reports WSB_ERR_TIMEOUT for every system in flight.
+ * futures without a limit): every wait of the solver kernels, for their own
+ * copies in flight and in the persistent kernels for the other CTAs that iterate
+ * the same system, gives up after `cycles` SM clock cycles (0 restores the
+ * default of about 2 s, which is also the most); the kernel then records the
+ * wait, drains its own copies in flight and returns, and the solve reports
+ * WSB_ERR_TIMEOUT for every system in flight. How long another system of the
+ * same batch or server iterates does not count.
  * Applies to solves, batches and servers started on this context afterwards. */
 int wsb_context_set_wait_limit(wsb_context *ctx, uint64_t cycles);
 

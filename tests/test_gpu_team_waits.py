@@ -1,0 +1,45 @@
+"""Waits of the persistent kernels (k_team): a CTA that has begun a system waits
+for those of its team that are still in another one, however long that takes."""
+import numpy as np
+import pytest
+
+import wgpu_solver_backend_b200 as wsb
+from test_gpu_stream import ring_system
+from wgpu_solver_backend_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture()
+def own_ctx():
+    c = wsb.GpuContext.create("auto", 0)  # the limit cannot reach other tests
+    yield c
+    c.set_wait_limit(0)
+
+
+def endless_chain(nbr, seed):
+    """A chain whose right-hand side has a NaN: no residual passes the test."""
+    rp, ci, v, bs, b = ring_system(nbr, (1,), seed)
+    b[5] = np.nan
+    return rp, ci, v, bs, b
+
+
+# Block rows, 70 a part. On 148 SMs the widest system (BSR6: two parts a CTA) and
+# the endless one of one part start together; of the next two, which share the
+# device, the second has the CTA of the endless one in its team. That one runs
+# for a hundred times the limit.
+@pytest.mark.parametrize("layout, wide, then", [("BSR6", 20510, (13930, 6650)), ("CSR", 10290, (7000, 3360))])
+def test_teams_wait_for_a_long_system(own_ctx, layout, wide, then):
+    systems = [ring_system(wide, (1,), 1), endless_chain(70, 2)] + [ring_system(n, (1,), n) for n in then]
+    kw = dict(max_iter=30000, rel_tol=1e-6)
+    mats = [wsb.Matrix.create(own_ctx, *s[:4], layout=getattr(wsb, "LAYOUT_" + layout)) for s in systems]
+    alone = [m.solve(s[4], raise_on_error=False, **kw) for m, s in zip(mats, systems)]
+    assert [r["rc"] for _, r in alone] == [0, _lib.NOT_CONVERGED, 0, 0]
+    own_ctx.set_wait_limit(2000000)  # about 1 ms
+    batch = wsb.Batch(own_ctx)
+    ids = [batch.add(m, s[4], **kw) for m, s in zip(mats, systems)]
+    batch.solve()
+    for i, m, (x, r) in zip(ids, mats, alone):
+        xb, rb = batch.result(i, m.n)
+        assert (rb["rc"], rb["iterations"]) == (r["rc"], r["iterations"])
+        assert np.array_equal(xb.view(np.uint32), x.view(np.uint32))

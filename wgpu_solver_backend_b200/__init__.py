@@ -121,8 +121,9 @@ class GpuContext:
         _check(_lib_handle().wsb_context_set_stream(self.handle, C.c_void_p(cuda_stream_ptr or 0)), self.handle)
 
     def set_wait_limit(self, cycles: int = 0):
-        """Limit of every pipeline wait in the solver kernels, in SM clock
-        cycles (0: the default of about 2 s). A wait that runs out ends the
+        """Limit of every wait in the solver kernels (for copies in flight and
+        for the other CTAs of the same system), in SM clock cycles (0: the
+        default of about 2 s, also the most). A wait that runs out ends the
         solves in flight with status TIMEOUT."""
         _check(_lib_handle().wsb_context_set_wait_limit(self.handle, int(cycles)), self.handle)
 

@@ -1014,11 +1014,20 @@ int Engine::launch_team(const std::vector<uint32_t> &ids, bool csr, uint32_t lim
         return run;
     };
     Run run = simulate(false);
-    const bool crowded = std::any_of(run.lists.begin(), run.lists.end(), [](const auto &l) { return l.size() > 1; });
-    if (crowded && !csr) {
+    auto longest_of = [](const Run &r) {
+        size_t most = 0;
+        for (const auto &l : r.lists) most = std::max(most, l.size());
+        return (uint32_t)most;
+    };
+    uint32_t longest = longest_of(run);
+    if (longest > 1 && !csr) {
         Run pairs = simulate(true);
         if (pairs.end < run.end) run = std::move(pairs);
+        longest = longest_of(run);
     }
+    // A CTA's wait for one in another system is bounded by the launch's
+    // iterations (36 s an item of its list with so many of them).
+    if (longest > 1) limit = std::min(limit, 1u << 20);
     const void *kernel = team_kernel((int)run.parts, csr, algo_ == (uint32_t)WSB_ALG_SINGLE_REDUCTION);
     WSB_CUDA_TRY(ctx_, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTeamSmemMax));
     const auto &lists = run.lists;
@@ -1049,7 +1058,7 @@ int Engine::launch_team(const std::vector<uint32_t> &ids, bool csr, uint32_t lim
     StepParams *dsp = d_sp_;
     const TeamItem *ditems = reinterpret_cast<const TeamItem *>(mem.dev + head);
     const uint32_t *doff = mem.dev;
-    void *args[] = {&dsys, &dsp, &ditems, &doff, &limit};
+    void *args[] = {&dsys, &dsp, &ditems, &doff, &limit, &longest};
     WSB_CUDA_TRY(ctx_, cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kTeamThreads), args,
                                                    (size_t)run.smem, stream_));
     launches_ += 1;

@@ -46,8 +46,9 @@
 // All CTAs of a launch are resident (cooperative launch); a CTA takes its
 // items in list order, and the lists are cut from one global order of systems,
 // so the first unfinished system always has all its CTAs. Every wait is
-// bounded (StepParams::wait_cycles): one that runs out sets kErrTeamWait, and
-// every CTA leaves.
+// bounded (StepParams::wait_cycles; that for a CTA which is still in another
+// system, by the iterations of the launch): one that runs out sets kErrTeamWait,
+// and every CTA leaves.
 #include "kernels_team.cuh"
 #include "team_device.cuh"
 
@@ -103,6 +104,27 @@ __device__ __forceinline__ void part_sums(const double *v, uint32_t lane, double
         for (int t = 0; t < kT; ++t) s[t][0] += __shfl_down_sync(kFull, s[t][0], o);
 #pragma unroll
     for (int t = 0; t < kT; ++t) sum[t] = s[t][0];
+}
+
+// More SM cycles than an iteration of k_team takes (34 us at 1.9 GHz).
+constexpr long long kTeamIterCycles = 65536;
+
+// Where CTAs have lists of items, one that comes to a system may have to wait for
+// one of its team that is still in others, for as long as those iterate
+// (`others` cycles at most): the team assembles, and only then the limit of a
+// wait counts. Apart from the system's own code, whose loop has no registers for
+// it (inside, two parts a CTA ran 3 % slower).
+__device__ __noinline__ void team_assemble(const SysDesc &D, uint32_t rank, uint32_t size, uint32_t parts, long long others,
+                                           uint32_t *err, StepParams *sp) {
+    if (parts >= size) return;
+    if (threadIdx.x >> 5 == (uint32_t)kTeamWarps) {
+        RedEntry *const red = D.red + (size_t)kRedEntries * team_copies(size) * size;
+        const uint32_t tag = D.st->epoch + 1u;
+        if ((threadIdx.x & 31u) == 0) st_entry(red + rank / parts, 0.0, tag);
+        __syncwarp();
+        team_gather(err, red, (size + parts - 1u) / parts, tag, sp, kTeamWaitCycles + others, 0);
+    }
+    __syncthreads();
 }
 
 // One system, this CTA's rows, up to `limit` iterations.
@@ -719,7 +741,7 @@ __device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it,
 template <int kT, bool kCsr, bool kSr>
 __global__ void __launch_bounds__(kTeamThreads, 1)
     k_team(const SysDesc *__restrict__ sys, StepParams *sp, const TeamItem *__restrict__ items,
-           const uint32_t *__restrict__ item_off, uint32_t limit) {
+           const uint32_t *__restrict__ item_off, uint32_t limit, uint32_t longest) {
     static_assert(offsetof(TeamShared, v) <= 512, "fixed shared memory");
     extern __shared__ __align__(128) char smem[];
     TeamShared &S = *reinterpret_cast<TeamShared *>(smem);
@@ -730,6 +752,11 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
     const uint32_t i1 = item_off[blockIdx.x + 1];
     for (uint32_t i = item_off[blockIdx.x]; i < i1; ++i) {
         const TeamItem it = items[i];
+        if (longest > 1u) team_assemble(sys[it.sys], it.rank, it.size, it.parts, kTeamIterCycles * longest * limit, &S.err, sp);
+        if (S.err) {
+            if (threadIdx.x == 0) atomicOr(&sp->error, kErrTeamWait);
+            return;
+        }
         team_system<kT, kCsr, kSr>(sys[it.sys], it, limit, S, smem + team_fixed_bytes(kT), w);
         __syncthreads();
         if (S.err) return;  // every CTA's later waits would run out as well

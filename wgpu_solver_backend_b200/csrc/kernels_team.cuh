@@ -58,15 +58,17 @@ static_assert(kTeamLuBytes % 16 == 0 && kTeamColBytes % 16 == 0 && kTeamIdxBytes
 // 7.0, 5.9, 5.8; 164 parts on 82 CTAs -, 8.2, 7.9; 148 CTAs in k_stream -, 13.5,
 // 13.4).
 __host__ __device__ constexpr uint32_t team_copies(uint32_t size) { return size <= 80u ? 1u : 8u; }
+// (And one a CTA for the team to assemble.)
 __host__ __device__ constexpr uint64_t team_red_entries(uint32_t size) {
-    return (uint64_t)kRedEntries * size * team_copies(size);
+    return ((uint64_t)kRedEntries * team_copies(size) + 1u) * size;
 }
 
 // The kernel whose CTAs hold up to `parts` (1 or 2) parts of a system, launched
 // cooperatively, one CTA per SM, with kTeamThreads threads and the arguments
 // (const SysDesc *, StepParams *, const TeamItem *items, const uint32_t
-// *item_off, uint32_t limit): CTA c works through items [item_off[c],
-// item_off[c + 1]), each for up to `limit` iterations. (More warps on an SM
+// *item_off, uint32_t limit, uint32_t longest): CTA c works through items
+// [item_off[c], item_off[c + 1]), `longest` at most, each for up to `limit`
+// iterations. (More warps on an SM
 // have too few registers: two CTAs of 512 threads spilled, and the spills did
 // not fit in what L1 the shared memory leaves: 26 systems of 9^3 nodes 13.5 us
 // an iteration against 10.7; so did one CTA of 24 warp tiles, 4^3 nodes 5.5 us
