@@ -43,3 +43,25 @@ def test_teams_wait_for_a_long_system(own_ctx, layout, wide, then):
         xb, rb = batch.result(i, m.n)
         assert (rb["rc"], rb["iterations"]) == (r["rc"], r["iterations"])
         assert np.array_equal(xb.view(np.uint32), x.view(np.uint32))
+
+
+# Limits from far below an exchange to about as long as one with the load before
+# it: whichever waits run out, a system that ends as converged has its bits.
+@pytest.mark.parametrize("limit", [100, 1000, 3000, 10000, 30000, 100000])
+def test_what_converges_under_a_short_limit_is_right(own_ctx, limit):
+    systems = [ring_system(n, (1, 7), n) for n in (10290, 70, 7000, 3360, 281, 141, 9000, 21000)]
+    kw = dict(max_iter=3000, rel_tol=1e-6)
+    mats = [wsb.Matrix.create(own_ctx, *s[:4]) for s in systems]
+    alone = [m.solve(s[4], **kw) for m, s in zip(mats, systems)]
+    own_ctx.set_wait_limit(limit)
+    batch = wsb.Batch(own_ctx)
+    ids = [batch.add(m, s[4], **kw) for m, s in zip(mats, systems)]
+    try:
+        batch.solve()
+    except wsb.WsbError:
+        pass
+    for i, m, (x, r) in zip(ids, mats, alone):
+        xb, rb = batch.result(i, m.n)
+        assert rb["rc"] in (0, _lib.TIMEOUT)
+        if rb["rc"] == 0:
+            assert rb["iterations"] == r["iterations"] and np.array_equal(xb.view(np.uint32), x.view(np.uint32))

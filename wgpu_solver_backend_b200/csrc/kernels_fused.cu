@@ -1245,6 +1245,7 @@ __device__ __forceinline__ void flush_upd(const SysDesc *__restrict__ sys, StepP
     if (kK == K_INIT) {
         st->bb = sum.x;
         st->rz_old = sum.y;
+        st->fresh = *const_cast<volatile uint32_t *>(&sp->error) != 0;  // (of k_spmv_init)
         uint32_t status = ST_RUNNING;
         if (sum.x == 0.0) status = ST_CONVERGED;
         else if (st->max_iter == 0) status = ST_MAXITER;

@@ -133,7 +133,7 @@ __device__ __forceinline__ void stream_system(const SysDesc &D, uint32_t limit, 
     constexpr uint32_t kUpd = kSr ? kStreamUpdBrowsSr : kStreamUpdBrows, kVecs = kSr ? 4u : 2u;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     SysState *st = D.st;
-    if (!st->active) return;
+    if (!st->active || st->fresh) return;  // (fresh: a wait of the init kernels ran out)
     // This CTA's block rows (an even first one: 16-byte aligned slices).
     const uint32_t nbr = D.n / 6u, half = (nbr + 1u) / 2u;
     const uint32_t b0 = min(nbr, 2u * (uint32_t)((uint64_t)blockIdx.x * half / gridDim.x));
