@@ -1270,6 +1270,7 @@ int Engine::step(uint32_t loop_limit, bool *any_left, uint32_t team_limit) {
         Slot &sl = *slots_[s];
         const SysState &st = h_state_[s];
         body_iters = std::max<uint64_t>(body_iters, st.iter);
+        if (st.failed) continue;  // ends with the step's error
         if (st.active && st.iter >= st.max_iter) {
             // Past its own limit and still active: the device bookkeeping is
             // broken for this system; retire it with an error.

@@ -569,7 +569,10 @@ __device__ __forceinline__ void stream_system(const SysDesc &D, uint32_t limit, 
     }
     __syncthreads();
     if (S.err) {
-        if (tid == 0) atomicOr(&sp->error, kErrTeamWait);
+        if (tid == 0) {
+            atomicOr(&sp->error, kErrTeamWait);
+            st->failed = 1;
+        }
         return;
     }
     if (blockIdx.x == 0 && tid == 0) {

@@ -705,7 +705,11 @@ __device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it,
     }
     __syncthreads();
     if (S.err) {
-        if (tid == 0) atomicOr(&w.sp->error, kErrTeamWait);
+        // (Its teammates may have come to the end: the system has failed.)
+        if (tid == 0) {
+            atomicOr(&w.sp->error, kErrTeamWait);
+            st->failed = 1;
+        }
         return;
     }
 #pragma unroll

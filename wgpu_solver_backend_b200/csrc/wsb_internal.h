@@ -109,6 +109,7 @@ struct alignas(64) SysState {
     uint32_t cnt_c;
     uint32_t fresh;             // persistent kernels: r, z, p and the first scalars are still to be formed
     double gamma_prev;          // single reduction: (r, u) of the previous iteration
+    uint32_t failed, pad;       // persistent kernels: a CTA left without its rows, whatever the others made of it
 };
 
 // A published partial sum: written and read as one 16-byte access, valid once
