@@ -1,10 +1,12 @@
-"""Waits of the persistent kernels (k_team): a CTA that has begun a system waits
-for those of its team that are still in another one, however long that takes."""
+"""Limits of the persistent kernels' waits: a CTA that has come to a system waits
+for those of its team that are still in another one, however long that takes; a
+wait within a system ends with a timeout, and the next solve is right."""
 import numpy as np
 import pytest
 
 import wgpu_solver_backend_b200 as wsb
 from test_gpu_stream import ring_system
+from test_gpu_team_csr import csr_system
 from wgpu_solver_backend_b200 import _lib
 
 pytestmark = pytest.mark.gpu
@@ -65,3 +67,20 @@ def test_what_converges_under_a_short_limit_is_right(own_ctx, limit):
         assert rb["rc"] in (0, _lib.TIMEOUT)
         if rb["rc"] == 0:
             assert rb["iterations"] == r["iterations"] and np.array_equal(xb.view(np.uint32), x.view(np.uint32))
+
+
+# Two workgroups, many, and more than one tree of partials.
+@pytest.mark.parametrize("n", [300, 4001, 70001])
+def test_reference_arithmetic_honours_the_limit(own_ctx, n):
+    rp, ci, v, bs, b = csr_system(n, 1, 6, n)
+    m = wsb.Matrix.create(own_ctx, rp, ci, v, bs, layout=wsb.LAYOUT_CSR)
+    kw = dict(max_iter=500, rel_tol=1e-5, precision=wsb.PREC_REFERENCE_F32, raise_on_error=False)
+    x_ok, r_ok = m.solve(b, **kw)
+    assert r_ok["rc"] == 0
+    own_ctx.set_wait_limit(1)
+    x0 = np.full(n, 3.0, np.float32)
+    x, r = m.solve(b, x0=x0, **kw)
+    assert r["rc"] == _lib.TIMEOUT and np.array_equal(x, x0)
+    own_ctx.set_wait_limit(0)
+    x, r = m.solve(b, **kw)
+    assert r["iterations"] == r_ok["iterations"] and np.array_equal(x.view(np.uint32), x_ok.view(np.uint32))

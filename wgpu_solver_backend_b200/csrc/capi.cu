@@ -214,7 +214,8 @@ static int solve_reference(Context *ctx, const MatA &A, const Precond &M, const 
     std::unique_ptr<CUgraphExec_st, cudaError_t (*)(cudaGraphExec_t)> eguard(nullptr, cudaGraphExecDestroy);
     if (resident) {
         RefPcg R{n, M.nb, (uint32_t)resident - 1u, A.row_ptr, A.col, A.val, M.lu, M.bs, db, dx, dz, dp, dap,
-                 reinterpret_cast<unsigned long long *>(dr), dst, hist_cap ? dhist : nullptr, hist_cap};
+                 reinterpret_cast<unsigned long long *>(dr), dst, hist_cap ? dhist : nullptr, hist_cap,
+                 (long long)(ctx->wait_cycles ? std::min<uint64_t>(ctx->wait_cycles, kTeamWaitCycles) : kTeamWaitCycles)};
         void *args[] = {&R};
         WSB_CUDA_TRY(ctx, cudaLaunchCooperativeKernel(ref_pcg_kernel(), dim3(grid_for(n, 256)), dim3(kRefThreads), args,
                                                       (size_t)ref_pcg_smem(R.width), st));

@@ -275,7 +275,7 @@ __device__ __forceinline__ float tree256_warp(F get) {
 // valid in lane 0: the workgroups' trees, then trees over their results.
 // `release`: the CTA's writes come before the partial.
 __device__ __forceinline__ float ref_all_sum(const float *prod, unsigned long long *parts, uint32_t tag, bool release,
-                                             RefShared &S, RefState *st) {
+                                             RefShared &S, RefState *st, long long lim) {
     const uint32_t lane = threadIdx.x & 31u, wgs = gridDim.x, copies = team_copies(wgs);
     float v = tree256_warp([&](uint32_t i) { return prod[i]; });
     if (wgs == 1) return v;
@@ -303,7 +303,7 @@ __device__ __forceinline__ float ref_all_sum(const float *prod, unsigned long lo
 #pragma unroll
             for (int j = 0; j < 8; ++j) ok = ok && (uint32_t)(q[j] >> 32) == tag;
             if (__all_sync(kFull, ok)) break;
-            if (__any_sync(kFull, clock64() - t0 > kTeamWaitCycles)) {
+            if (__any_sync(kFull, clock64() - t0 > lim) || ((k & 255u) == 0 && __any_sync(kFull, ld_error(st) != 0))) {
                 S.err = 1;
                 atomicExch(&st->error, 1u);
                 return 0.0f;
@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(kRefThreads, 2) k_ref_pcg(const RefPcg D) {
     }
     __syncthreads();
     if (warp < 2) {
-        const float v = ref_all_sum(prod + 256u * warp, warp ? part2 : part1, tag, true, S, D.st);
+        const float v = ref_all_sum(prod + 256u * warp, warp ? part2 : part1, tag, true, S, D.st, D.wait_cycles);
         if (lane == 0) S.v[warp] = v;
     }
     __syncthreads();
@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(kRefThreads, 2) k_ref_pcg(const RefPcg D) {
         if (own) prod[tid] = __fmul_rn(p, ap);
         __syncthreads();
         if (warp == 0) {
-            const float v = ref_all_sum(prod, part0, tag, false, S, D.st);
+            const float v = ref_all_sum(prod, part0, tag, false, S, D.st, D.wait_cycles);
             if (lane == 0) S.v[0] = v;
         }
         __syncthreads();
@@ -540,7 +540,7 @@ __global__ void __launch_bounds__(kRefThreads, 2) k_ref_pcg(const RefPcg D) {
         }
         __syncthreads();
         if (warp < 2) {
-            const float v = ref_all_sum(prod + 256u * warp, warp ? part2 : part1, tag, true, S, D.st);
+            const float v = ref_all_sum(prod + 256u * warp, warp ? part2 : part1, tag, true, S, D.st, D.wait_cycles);
             if (lane == 0) S.v[warp] = v;
         }
         __syncthreads();

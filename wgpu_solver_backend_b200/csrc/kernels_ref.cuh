@@ -53,6 +53,7 @@ struct RefPcg {
     RefState *st;                      // tolerances and limit; the outcome
     double *history;
     uint64_t hist_cap;
+    long long wait_cycles;             // limit of a wait (SM cycles)
 };
 constexpr int kRefThreads = 288;  // a thread a row, and 32 for the rows beside the CTA's
 constexpr uint32_t kRefCols = 1280, kRefHash = 2048;

@@ -8,7 +8,6 @@ namespace wsb {
 namespace {
 
 constexpr uint32_t kFull = 0xffffffffu;
-constexpr long long kTeamWaitCycles = 4000000000ll;  // about 2 s
 
 __device__ __forceinline__ void st_entry(RedEntry *e, double v, uint32_t tag) {
     asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(e),
@@ -42,7 +41,9 @@ __device__ __forceinline__ unsigned long long ld_packet_if(const unsigned long l
                  : "memory");
     return v;
 }
-__device__ __forceinline__ uint32_t ld_error(const StepParams *sp) {
+// The error word of a launch (StepParams, RefState).
+template <class T>
+__device__ __forceinline__ uint32_t ld_error(const T *sp) {
     uint32_t v;
     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&sp->error) : "memory");
     return v;

@@ -112,6 +112,8 @@ struct alignas(64) SysState {
     uint32_t failed, pad;       // persistent kernels: a CTA left without its rows, whatever the others made of it
 };
 
+constexpr long long kTeamWaitCycles = 4000000000ll;  // the most and the default limit of a persistent kernel's wait: about 2 s
+
 // A published partial sum: written and read as one 16-byte access, valid once
 // its tag is the expected one.
 struct alignas(16) RedEntry {
