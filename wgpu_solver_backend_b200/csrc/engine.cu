@@ -1028,7 +1028,7 @@ int Engine::launch_team(const std::vector<uint32_t> &ids, bool csr, uint32_t lim
     // A CTA's wait for one in another system is bounded by the launch's
     // iterations (36 s an item of its list with so many of them).
     if (longest > 1) limit = std::min(limit, 1u << 20);
-    const void *kernel = team_kernel((int)run.parts, csr, algo_ == (uint32_t)WSB_ALG_SINGLE_REDUCTION);
+    const void *kernel = team_kernel((int)run.parts, csr, algo_ == (uint32_t)WSB_ALG_SINGLE_REDUCTION, longest > 1);
     WSB_CUDA_TRY(ctx_, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTeamSmemMax));
     const auto &lists = run.lists;
     const uint32_t grid = (uint32_t)lists.size();

@@ -742,7 +742,9 @@ __device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it,
     }
 }
 
-template <int kT, bool kCsr, bool kSr>
+// kLists: CTAs may have several items. (With one part a CTA the call alone costs
+// every iteration 0.02 to 0.05 us, so there is a variant without it.)
+template <int kT, bool kCsr, bool kSr, bool kLists>
 __global__ void __launch_bounds__(kTeamThreads, 1)
     k_team(const SysDesc *__restrict__ sys, StepParams *sp, const TeamItem *__restrict__ items,
            const uint32_t *__restrict__ item_off, uint32_t limit, uint32_t longest) {
@@ -756,10 +758,12 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
     const uint32_t i1 = item_off[blockIdx.x + 1];
     for (uint32_t i = item_off[blockIdx.x]; i < i1; ++i) {
         const TeamItem it = items[i];
-        if (longest > 1u) team_assemble(sys[it.sys], it.rank, it.size, it.parts, kTeamIterCycles * longest * limit, &S.err, sp);
-        if (S.err) {
-            if (threadIdx.x == 0) atomicOr(&sp->error, kErrTeamWait);
-            return;
+        if (kLists && longest > 1u) {
+            team_assemble(sys[it.sys], it.rank, it.size, it.parts, kTeamIterCycles * longest * limit, &S.err, sp);
+            if (S.err) {
+                if (threadIdx.x == 0) atomicOr(&sp->error, kErrTeamWait);
+                return;
+            }
         }
         team_system<kT, kCsr, kSr>(sys[it.sys], it, limit, S, smem + team_fixed_bytes(kT), w);
         __syncthreads();
@@ -839,13 +843,13 @@ __global__ void __launch_bounds__(kPlanThreads) k_team_plan_csr(SysDesc D, uint3
 }  // namespace
 
 template <bool kSr>
-static const void *team_kernel_of(int parts, bool csr) {
-    return csr          ? (const void *)k_team<1, true, kSr>
-           : parts == 1 ? (const void *)k_team<1, false, kSr>
-                        : (const void *)k_team<2, false, kSr>;
+static const void *team_kernel_of(int parts, bool csr, bool lists) {
+    return parts == 2 ? (const void *)k_team<2, false, kSr, true>
+           : csr      ? (lists ? (const void *)k_team<1, true, kSr, true> : (const void *)k_team<1, true, kSr, false>)
+                      : (lists ? (const void *)k_team<1, false, kSr, true> : (const void *)k_team<1, false, kSr, false>);
 }
-const void *team_kernel(int parts, bool csr, bool single_reduction) {
-    return single_reduction ? team_kernel_of<true>(parts, csr) : team_kernel_of<false>(parts, csr);
+const void *team_kernel(int parts, bool csr, bool single_reduction, bool lists) {
+    return single_reduction ? team_kernel_of<true>(parts, csr, lists) : team_kernel_of<false>(parts, csr, lists);
 }
 
 cudaError_t team_plan_csr(const SysDesc &D, uint32_t *count, uint32_t *most, uint32_t parts, cudaStream_t st) {

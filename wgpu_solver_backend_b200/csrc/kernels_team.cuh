@@ -63,17 +63,16 @@ __host__ __device__ constexpr uint64_t team_red_entries(uint32_t size) {
     return ((uint64_t)kRedEntries * team_copies(size) + 1u) * size;
 }
 
-// The kernel whose CTAs hold up to `parts` (1 or 2) parts of a system, launched
-// cooperatively, one CTA per SM, with kTeamThreads threads and the arguments
-// (const SysDesc *, StepParams *, const TeamItem *items, const uint32_t
-// *item_off, uint32_t limit, uint32_t longest): CTA c works through items
-// [item_off[c], item_off[c + 1]), `longest` at most, each for up to `limit`
-// iterations. (More warps on an SM
-// have too few registers: two CTAs of 512 threads spilled, and the spills did
-// not fit in what L1 the shared memory leaves: 26 systems of 9^3 nodes 13.5 us
-// an iteration against 10.7; so did one CTA of 24 warp tiles, 4^3 nodes 5.5 us
-// against 2.9.)
-const void *team_kernel(int parts, bool csr, bool single_reduction);
+// The kernel whose CTAs hold up to `parts` (1 or 2) parts of a system, one item
+// each or `lists` of them, launched cooperatively, one CTA per SM, with
+// kTeamThreads threads and the arguments (const SysDesc *, StepParams *, const
+// TeamItem *items, const uint32_t *item_off, uint32_t limit, uint32_t longest):
+// CTA c works through items [item_off[c], item_off[c + 1]), `longest` at most,
+// each for up to `limit` iterations. (More warps on an SM have too few registers:
+// two CTAs of 512 threads spilled, and the spills did not fit in what L1 the
+// shared memory leaves: 26 systems of 9^3 nodes 13.5 us an iteration against
+// 10.7; so did one CTA of 24 warp tiles, 4^3 nodes 5.5 us against 2.9.)
+const void *team_kernel(int parts, bool csr, bool single_reduction, bool lists);
 // Fills D.tile_idx, D.ext_cols and D.ext_count (= count) of a CSR system whose
 // tiles are set, `parts` parts of D.team_warps tiles. most[0] becomes the most
 // columns outside a part, most[1] whether that is more than D.ext_cap (nothing
