@@ -1,10 +1,12 @@
 """A server whose requests take different paths: systems of the loop kernels
 that retire while others of theirs go on, beside a refined system of a
-persistent kernel (whose sweeps upload the descriptors again)."""
+persistent kernel (whose sweeps upload the descriptors again); and budgets
+without room for what the persistent kernels need besides."""
 import numpy as np
 import pytest
 
 import wgpu_solver_backend_b200 as wsb
+from wgpu_solver_backend_b200 import _lib
 
 pytestmark = pytest.mark.gpu
 
@@ -54,3 +56,27 @@ def test_retired_loop_systems_beside_a_refined_one(ctx):
     for (x, r), (xa, ra) in zip(served, alone):
         assert r["rc"] == 0 and r["iterations"] == ra["iterations"]
         assert np.array_equal(x.view(np.uint32), xa.view(np.uint32))
+
+
+# A system of the loop kernels, and one that k_team would take.
+@pytest.mark.parametrize("n", [80000, 4000])
+def test_budget_of_the_loop_kernels_memory(ctx, n):
+    """A budget of what a system needs in the loop kernels (matrix, factors,
+    vectors, partials) admits it, whatever the other kernels would need."""
+    rp, ci, v, bs, b = chain_system(n, 1e-2, n)
+    nnz, nb, pad, tiles = len(v), len(bs) - 1, 64, n // 16 + 64
+    matrix = 8 * nnz + 4 * (n + 1) + 8 * pad + 8 * tiles
+    factors = 144 * nb + 4 * (nb + 1) + 16 * tiles + 1024
+    vectors = 24 * (n + pad) + 24 * tiles + 8 * 4096
+    kw = dict(max_iter=5000, rel_tol=1e-6)
+    xa, ra = wsb.Matrix.create(ctx, rp, ci, v, bs).solve(b, **kw)
+    for budget, rc in ((matrix + factors + vectors, 0), (matrix + factors + vectors - 1, _lib.OUT_OF_MEMORY)):
+        srv = wsb.Server(ctx, memory_budget_bytes=budget)
+        try:
+            x, r = srv.wait(srv.submit(rp, ci, v, bs, b, **kw), 60.0)
+        finally:
+            srv.close()
+        assert r["rc"] == rc
+        if rc == 0:  # (FP64 sums may be grouped in another way)
+            assert r["iterations"] == ra["iterations"]
+            assert np.linalg.norm(x.astype(np.float64) - xa) < 1e-6 * np.linalg.norm(xa)

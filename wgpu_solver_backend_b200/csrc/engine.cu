@@ -501,8 +501,10 @@ int Engine::add(const MatA *A, const Precond *M, const SolveCfg &cfg, uint32_t *
     const size_t n = A->n, vf = a256((n + kPadElems) * sizeof(float));
     const uint64_t max_hist = cfg.max_iter > 0 ? cfg.max_iter : 1;
     sl->hist_cap = std::min<uint64_t>(cfg.hist_cap, max_hist);
-    team_plan(sl.get());
-    stream_plan(sl.get());
+    if (!cfg.loop_kernels) {
+        team_plan(sl.get());
+        stream_plan(sl.get());
+    }
     size_t off[19], tot = 0;
     auto take = [&](int k, size_t bytes) {
         off[k] = tot;

@@ -94,6 +94,7 @@ struct SolveCfg {
     uint32_t max_refine = 50;
     uint64_t hist_cap = 0;
     int algorithm = WSB_ALG_CLASSIC;  // the PCG recurrence (wsb_algorithm)
+    bool loop_kernels = false;        // no memory for what the persistent kernels need besides
 };
 
 struct SolveOutcome {

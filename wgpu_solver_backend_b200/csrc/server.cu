@@ -47,6 +47,7 @@ struct Request {
     std::unique_ptr<Precond> M;
     uint32_t slot = 0;
     uint64_t reserved = 0;
+    uint64_t bytes = 0, more_bytes = 0;  // loop_bytes, persistent_bytes
     enum State { QUEUED, UPLOADING, READY, ACTIVE, DONE } state = QUEUED;
     int status = WSB_PENDING;
     std::string error;
@@ -57,29 +58,38 @@ struct Request {
     Clock::time_point t_submit, t_done;
 };
 
-// Device bytes a request holds while resident (matrix, LU, vectors, partials).
-uint64_t estimate_bytes(const Request &r) {
+// Device bytes a request holds while resident (matrix, LU, vectors, partials)
+// when the loop kernels iterate it.
+uint64_t loop_bytes(const Request &r) {
     const uint64_t n = r.n, nnz = r.nnz, nb = r.bs_len ? r.bs_len - 1 : 0;
     uint64_t a = 8 * nnz + 4 * (n + 1) + 8 * kPadElems + 8 * (n / 16 + 64);      // CSR (BSR6 is smaller)
     uint64_t m = 144 * nb + 4 * (nb + 1) + 16 * (n / 16 + 64) + 1024;            // LU, starts, tiles
     uint64_t v = 6 * 4 * (n + kPadElems) + 8 * (n / 16 + 64) + 16 * (n / 16 + 64) + 8 * 4096;
     if (r.cfg.precision == WSB_PREC_MIXED_F64_IR) v += 12 * (n + kPadElems);
     if (r.cfg.algorithm == WSB_ALG_SINGLE_REDUCTION) v += 4 * (n + kPadElems);
+    v += 8 * std::min<uint64_t>(r.cfg.hist_cap, r.cfg.max_iter + 1);
+    return a + m + v;
+}
+
+// What the persistent kernels need besides. Above the rows that k_team takes of
+// a CSR system only BSR6 systems go there: a second p or z packets (8 bytes a row
+// at most) and the partials, in place of CSR arrays of 26 bytes a row and more.
+uint64_t persistent_bytes(const Request &r) {
+    const uint64_t n = r.n;
+    if (n > 32ull * kTeamWarps * 160) return 0;
     // k_team: z packets; k_stream: the other buffer of p; published partials
     // (for teams of one warp tile a CTA at most).
-    v += 8 * (n + kPadElems) + sizeof(RedEntry) * team_red_entries((uint32_t)std::min<uint64_t>(n / (6 * kTeamWarpBrows) + 1, 512));
-    v += 8 * std::min<uint64_t>(r.cfg.hist_cap, r.cfg.max_iter + 1);
+    uint64_t v = 8 * (n + kPadElems) +
+                 sizeof(RedEntry) * team_red_entries((uint32_t)std::min<uint64_t>(n / (6 * kTeamWarpBrows) + 1, 512));
     // k_team, CSR: warp tiles of at least 27 rows, a place of two bytes for each
     // column (padded to the tile's longest row; a third of a CTA's shared memory
     // at most), the columns outside each part.
-    if (n <= 32ull * kTeamWarps * 160) {
-        const uint64_t tiles = n / 27 + 1, parts = std::min<uint64_t>(tiles, 160);
-        uint64_t longest = 0;
-        for (uint64_t i = 0; i < n; ++i) longest = std::max<uint64_t>(longest, r.p_row_ptr[i + 1] - r.p_row_ptr[i]);
-        v += 12 * (tiles + 1) + std::min(64 * tiles * (longest + 3), parts * (kTeamSmemMax / 3)) +
-             4 * parts * std::min<uint64_t>(n, kTeamMaxExt);
-    }
-    return a + m + v;
+    const uint64_t tiles = n / 27 + 1, parts = std::min<uint64_t>(tiles, 160);
+    uint64_t longest = 0;
+    for (uint64_t i = 0; i < n; ++i) longest = std::max<uint64_t>(longest, r.p_row_ptr[i + 1] - r.p_row_ptr[i]);
+    v += 12 * (tiles + 1) + std::min(64 * tiles * (longest + 3), parts * (kTeamSmemMax / 3)) +
+         4 * parts * std::min<uint64_t>(n, kTeamMaxExt);
+    return v;
 }
 
 }  // namespace
@@ -129,6 +139,12 @@ struct wsb_server {
         else ++stats.failed;
     }
 
+    // A request that fits the budget without the persistent kernels' memory only
+    // goes without them.
+    uint64_t need_of(const Request &r) const {
+        return r.bytes + r.more_bytes <= opts.memory_budget_bytes ? r.bytes + r.more_bytes : r.bytes;
+    }
+
     void upload_loop(cudaStream_t upload_stream) {
         cudaSetDevice(ctx->device);
         thread_alloc_pool() = pool;
@@ -139,13 +155,13 @@ struct wsb_server {
                 cv_upload.wait(lk, [&] {
                     if (stopping) return true;
                     if (queued.empty()) return false;
-                    const uint64_t need = estimate_bytes(*queued.front());
+                    const uint64_t need = need_of(*queued.front());
                     return need > opts.memory_budget_bytes || bytes_in_use + need <= opts.memory_budget_bytes;
                 });
                 if (stopping) return;
                 r = queued.front();
                 queued.pop_front();
-                const uint64_t need = estimate_bytes(*r);
+                const uint64_t need = need_of(*r);
                 if (need > opts.memory_budget_bytes) {
                     ++stats.rejected;
                     finish(r, WSB_ERR_OUT_OF_MEMORY, "request needs more device memory than the server budget");
@@ -153,6 +169,7 @@ struct wsb_server {
                     continue;
                 }
                 r->reserved = need;
+                r->cfg.loop_kernels = need < r->bytes + r->more_bytes;
                 bytes_in_use += need;
                 bytes_peak = std::max(bytes_peak, bytes_in_use);
                 r->state = Request::UPLOADING;
@@ -399,6 +416,8 @@ extern "C" int wsb_server_submit(wsb_server *s, uint32_t n, const uint32_t *row_
         r->x64_out = o->x64_out;
     }
     r->cfg = c;
+    r->bytes = loop_bytes(*r);
+    r->more_bytes = persistent_bytes(*r);
     if (c.hist_cap) r->hist.assign(std::min<uint64_t>(c.hist_cap, max_iter + 1), 0.0);
     r->t_submit = Clock::now();
     std::lock_guard<std::mutex> lk(s->mu);
