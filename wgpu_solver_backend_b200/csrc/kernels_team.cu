@@ -705,11 +705,7 @@ __device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it,
     }
     __syncthreads();
     if (S.err) {
-        // (Its teammates may have come to the end: the system has failed.)
-        if (tid == 0) {
-            atomicOr(&w.sp->error, kErrTeamWait);
-            st->failed = 1;
-        }
+        if (tid == 0) atomicOr(&w.sp->error, kErrTeamWait);
         return;
     }
 #pragma unroll
@@ -767,7 +763,11 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
         }
         team_system<kT, kCsr, kSr>(sys[it.sys], it, limit, S, smem + team_fixed_bytes(kT), w);
         __syncthreads();
-        if (S.err) return;  // every CTA's later waits would run out as well
+        if (S.err) {  // every CTA's later waits would run out as well
+            // (Its teammates may have come to the end: the system has failed.)
+            if (threadIdx.x == 0) sys[items[i].sys].st->failed = 1;
+            return;
+        }
     }
 }
 
