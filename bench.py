@@ -41,19 +41,33 @@ def peaks():
         return 6650.0, "fallback"
 
 
-# DRAM bytes per algorithmic byte of the SpMV kernel, from one ncu capture of
-# k_spmv_loop on the 56^3 lattice (BSR6 tiles, 206 MB of matrix > L2; see
-# profiles/k_spmv_loop_bsr6_side56.md): dram__bytes_read.sum 184.378112 MB +
-# dram__bytes_write.sum 4.038656 MB over 188.285444 MB of algorithmic bytes.
-# The kernel streams every byte once, so the traffic scales with the launch's
-# algorithmic bytes.
-SPMV_DRAM_PER_ALGO_BYTE = (184.378112e6 + 4.038656e6) / 188285444.0
+# DRAM bytes per algorithmic byte of a k_stream solve, from one ncu capture of 30
+# iterations on the 56^3 lattice (206 MB of matrix and factors > L2; see
+# profiles/k_team_k_stream.md): dram__bytes_read.sum 6012.8128 MB +
+# dram__bytes_write.sum 178.929152 MB over 30 x 255.721988 MB of algorithmic
+# bytes. Matrix and factors come from memory once an iteration, the vectors stay
+# in the L2.
+STREAM_DRAM_PER_ALGO_BYTE = (6012.8128e6 + 178.929152e6) / (30 * 255721988.0)
 
 
-def spmv_traffic(algo_bytes):
-    return {"traffic": algo_bytes * SPMV_DRAM_PER_ALGO_BYTE,
-            "traffic_note": "dram read+write bytes per launch, scaled from an ncu capture of the same kernel on "
-                            "the 56^3 lattice (ratio %.4f to the algorithmic bytes)" % SPMV_DRAM_PER_ALGO_BYTE}
+def stream_roofline(bytes_per_iteration, iterations, solve_ms, peak, peak_kind):
+    """The roofline block of an 80^3 BSR6 solve: one k_stream launch (and the two
+    kernels that start it, in the time) over all iterations' algorithmic bytes."""
+    algo = bytes_per_iteration * iterations
+    gbs = algo / solve_ms / 1e6
+    return {"bound": "hbm", "kernel": "k_stream: a whole solve of the 3.07M-unknown 80^3 system, BSR6 (the layout the "
+                                      "library picks for it), in one launch",
+            "achieved": gbs, "peak": peak, "unit": "GB/s", "frac": gbs / peak, "peak_kind": peak_kind,
+            "traffic": algo * STREAM_DRAM_PER_ALGO_BYTE,
+            "traffic_note": "dram read+write bytes per launch, scaled from an ncu capture of the same kernel on the "
+                            "56^3 lattice (ratio %.4f to the algorithmic bytes: the vectors stay in the L2)"
+                            % STREAM_DRAM_PER_ALGO_BYTE,
+            "algorithmic_bytes_per_launch": int(algo), "launch_us": solve_ms * 1e3,
+            "algorithmic_bytes_per_iteration": int(bytes_per_iteration), "iterations": iterations}
+
+
+LOOP_KERNELS_NOTE = ("the fallback path's kernels, each timed on its own; BSR6 solves of this size run k_stream and launch "
+                     "none of them")
 
 
 class ClockSampler:
@@ -223,16 +237,10 @@ def run_plain(args, world, rank, local):
     dev_s = e0.elapsed_time(e1) / 1e3
     dev_s = reduce_max(dev_s, world)
     barrier(world)
-    # Per-kernel device times of the solver's own loop kernels (CUDA events
-    # around each launch, outside the graph), on the same matrix.
+    # The loop kernels on the same matrix (CUDA events around each launch): not
+    # part of the timed solves, which run k_stream.
     kt = m.kernel_times(d_b.data_ptr(), iterations=20)
-    spmv_s = kt["spmv_ms"] / 1e3
     peak, peak_kind = peaks()
-    spmv_gbs = info["spmv_bytes"] / spmv_s / 1e9
-    upd_bytes = 28 * n + 144 * info["num_blocks"]
-    kernels = {"spmv": {"ms": kt["spmv_ms"], "bytes": info["spmv_bytes"], "gbs": spmv_gbs},
-               "update": {"ms": kt["update_ms"], "bytes": upd_bytes, "gbs": upd_bytes / kt["update_ms"] / 1e6},
-               "pupdate": {"ms": kt["pupdate_ms"], "bytes": 12 * n, "gbs": 12 * n / kt["pupdate_ms"] / 1e6}}
     iter_gbs = info["iteration_bytes"] * iters / (dev_s / args.steps) / 1e9
     # End to end through the C ABI with host buffers (copies in the timed region).
     x_host = np.zeros(n, np.float32)
@@ -253,11 +261,9 @@ def run_plain(args, world, rank, local):
                    "l2": "inputs larger than L2 (matrix %.0f MB)" % (info["device_bytes"] / 1e6)},
         "e2e": {"value": replica_rate(world, args.steps, e2e_s), "unit": "solves/s", "h2d_bytes_per_step": 8 * n,
                 "d2h_bytes_per_step": 4 * n},
-        "roofline": {"bound": "hbm", "kernel": "spmv (BSR6 tiles)" if info["layout"] == wsb.LAYOUT_BSR6 else "spmv",
-                     "achieved": spmv_gbs, "peak": peak, "unit": "GB/s", "frac": spmv_gbs / peak,
-                     "peak_kind": peak_kind, **spmv_traffic(info["spmv_bytes"]),
-                     "algorithmic_bytes_per_launch": info["spmv_bytes"], "launch_us": spmv_s * 1e6},
-        "iteration_gbs": iter_gbs, "iteration_frac": iter_gbs / peak, "kernels": kernels,
+        "roofline": stream_roofline(info["iteration_bytes"], iters, dev_s / args.steps * 1e3, peak, peak_kind),
+        "iteration_gbs": iter_gbs, "iteration_frac": iter_gbs / peak,
+        "loop_kernels": dict(kernel_block(kt, info, n, peak), note=LOOP_KERNELS_NOTE),
         "gpu_launches": args.steps * int(res["kernel_launches"]),
         "clocks": clk,
     }
@@ -432,8 +438,9 @@ def kernel_block(kt, info, n, peak):
 
 def measure_c2(ctx, stream, peak):
     """The plain 80^3 system (n = 3,072,000, nnz = 127,641,600, tolerance
-    1e-6) in both layouts: per-kernel times of the loop kernels (CUDA events
-    per launch), whole solves (CUDA events, graph loop), per-iteration GB/s."""
+    1e-6) in both layouts: whole solves (CUDA events; BSR6 in k_stream, CSR in the
+    graph of the loop kernels), per-iteration GB/s, and the loop kernels' own
+    times (CUDA events per launch)."""
     import torch
 
     import wgpu_solver_backend_b200 as wsb
@@ -463,13 +470,16 @@ def measure_c2(ctx, stream, peak):
             ms += e0.elapsed_time(e1) / reps
         it = int(r["iterations"])
         ib = info["iteration_bytes"]
-        out[name] = {"kernels": kernel_block(kt, info, n, peak), "solve_ms": ms, "iterations": it,
+        loop_kernels = kernel_block(kt, info, n, peak)
+        if name == "bsr6":
+            loop_kernels["note"] = LOOP_KERNELS_NOTE
+        out[name] = {"loop_kernels": loop_kernels, "solve_ms": ms, "iterations": it,
                      "iteration_us": ms * 1e3 / it, "iteration_bytes": int(ib),
                      "iteration_gbs": ib * it / (ms / 1e3) / 1e9, "iteration_frac": ib * it / (ms / 1e3) / 1e9 / peak,
                      "matrix_bytes": int(info["device_bytes"])}
-        # The opt-in single-reduction recurrence on the same matrix: two
-        # kernels per iteration, SpMV + 68 n bytes (the update kernel also
-        # reads and writes s and forms p = u + beta p).
+        # The opt-in single-reduction recurrence on the same matrix: SpMV + 68 n
+        # bytes an iteration (the update also reads and writes s and forms p = u
+        # + beta p).
         sr = dict(kw, algorithm=wsb.ALG_SINGLE_REDUCTION)
         d_x.zero_()
         m.solve_device(d_b.data_ptr(), d_x.data_ptr(), **sr)  # warm-up
@@ -701,7 +711,7 @@ def run_serve(args, world, rank, local):
     srv2.close()
     fcfs1 = fcfs_latencies(arrivals, plain_lat)
     fcfs2 = fcfs_latencies(arrivals2, plain_lat + plain_lat)
-    # Dominant kernel (SpMV + p.Ap) on the largest system of the set.
+    # The loop kernels on the largest system of the set (not part of its solves).
     big = int(np.argmax([p["n"] for p in pool]))
     d_b = torch.from_numpy(pool[big]["b"]).cuda()
     torch.cuda.synchronize()
@@ -711,7 +721,6 @@ def run_serve(args, world, rank, local):
     serve_largest = kernel_block(kt, info, pool[big]["n"], peak)
     c2 = measure_c2(ctx, stream, peak)
     c4 = measure_c4(ctx, stream, peak)
-    top = c2["bsr6"]["kernels"]["spmv"]
     e2e = replica_rate(world, args.steps * R, e2e_s)
     line = {
         "metric": METRIC, "value": replica_rate(world, args.steps * R, dev_s), "unit": "solves/s", "n_gpus": world,
@@ -744,18 +753,15 @@ def run_serve(args, world, rank, local):
                              (world * R / plain_res_s)},
         "results": {"ok": ok, "of": len(results), "max_final_relres": relres_max,
                     "iterations_min_median_max": [int(min(iters)), int(np.median(iters)), int(max(iters))]},
-        "roofline": {"bound": "hbm", "kernel": "k_spmv_loop (SpMV + p.Ap) on the 3.07M-unknown 80^3 system, BSR6 "
-                               "(the layout the library picks for it); CSR beside it in c2",
-                     "achieved": top["gbs"], "peak": peak, "unit": "GB/s", "frac": top["frac"],
-                     "peak_kind": peak_kind, **spmv_traffic(top["bytes"]),
-                     "algorithmic_bytes_per_launch": top["bytes"], "launch_us": top["us"]},
+        "roofline": stream_roofline(c2["bsr6"]["iteration_bytes"], c2["bsr6"]["iterations"], c2["bsr6"]["solve_ms"], peak,
+                                    peak_kind),
         "resident_pass_hbm": {"algorithmic_bytes": pass_bytes, "gbs": pass_bytes / pass_s / 1e9,
                               "frac": pass_bytes / pass_s / 1e9 / peak,
                               "note": "sum over requests of PCG iterations x bytes per iteration; the FP64 "
                                       "refinement sweeps' residual and update passes are not counted"},
         "c2": c2,
         "c4": c4,
-        "serve_largest_system_kernels": serve_largest,
+        "serve_largest_system_loop_kernels": dict(serve_largest, note=LOOP_KERNELS_NOTE),
         "serve_tolerance_mix": {"targets": "FP64 relres 1e-6 or 1e-10, p = 1/2 each (seeded)",
                                 "solves_per_s": R / mk_mix, "met_target": mix_ok, "of": R,
                                 "p50_ms": float(np.percentile(lat_mix, 50)), "p99_ms": float(np.percentile(lat_mix, 99)),
