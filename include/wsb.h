@@ -282,12 +282,16 @@ int wsb_matrix_create(wsb_context *ctx, uint32_t n, const uint32_t *row_ptr, con
 int wsb_matrix_info_get(const wsb_matrix *m, wsb_matrix_info *out);
 void wsb_matrix_destroy(wsb_matrix *m);
 /* Tile autotuner (no counterpart in the reference, whose kernels have one  */
-/* fixed launch shape): times the solver's SpMV and update kernels on this  */
-/* matrix for a few tile sizes (a short PCG run on b = ones), keeps the     */
-/* fastest of each, and records the choice for matrices of the same shape   */
-/* class (layout, n within a factor of 2, nonzeros per row) created later   */
-/* in this process. Retuned tiles regroup the FP64 partial sums of the dot  */
-/* products: results agree with the untuned ones to FP64 rounding.          */
+/* fixed launch shape): times the SpMV and update kernels of the loop path  */
+/* on this matrix for a few tile sizes (a short PCG run on b = ones), keeps */
+/* the fastest of each, and records the choice for matrices of the same     */
+/* shape class (layout, n within a factor of 2, nonzeros per row) created   */
+/* later in this process. The tiles serve wsb_matrix_spmv_device and solves */
+/* that the loop kernels iterate (large CSR systems, long block rows);      */
+/* there they regroup the FP64 partial sums of the dot products, so results */
+/* agree with the untuned ones to FP64 rounding. Solves of the persistent   */
+/* kernels do not use them, but for the first residual of large BSR6        */
+/* systems.                                                                 */
 typedef struct wsb_tune_result {
     uint32_t spmv_rows;          /* rows per SpMV tile (6 x block rows for BSR6) */
     uint32_t spmv_cap;           /* nonzeros (CSR) or 6x6 blocks (BSR6) per SpMV tile */
@@ -330,8 +334,9 @@ int wsb_matrix_spmv_device(wsb_context *ctx, wsb_matrix *m, const float *d_x, fl
 int wsb_matrix_spmv_check(wsb_context *ctx, wsb_matrix *m);
 
 /* Measurement aid (no counterpart in the reference): runs `iterations` PCG
- * iterations of this matrix with right-hand side d_b (device) outside the
- * CUDA graph, CUDA events around each launch, and writes the mean duration
+ * iterations of this matrix with right-hand side d_b (device) in the loop
+ * kernels, whichever kernel its solves run (most run a persistent one that is
+ * a single launch), CUDA events around each launch, and writes the mean duration
  * in ms of the SpMV+p.Ap kernel, the update+preconditioner kernel and the
  * p-update kernel to ms[0..2]; ms[3] and ms[4] receive the iteration count
  * and status code of the system afterwards (a valid measurement has

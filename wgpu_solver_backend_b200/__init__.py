@@ -384,8 +384,8 @@ class Matrix:
         return Matrix(ctx, h)
 
     def autotune(self, iterations: int = 8) -> dict:
-        """Times candidate tile sizes of the SpMV and update kernels on this
-        matrix, keeps the fastest and records them for matrices of the same
+        """Times candidate tile sizes of the loop path's SpMV and update kernels
+        on this matrix, keeps the fastest and records them for matrices of the same
         shape class created later (wsb_matrix_autotune)."""
         r = _lib.TuneResult()
         _check(_lib_handle().wsb_matrix_autotune(self.ctx.handle, self.handle, int(iterations), C.byref(r)),

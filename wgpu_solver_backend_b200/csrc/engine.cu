@@ -442,11 +442,13 @@ int Engine::finish_team_plans() {
 }
 
 // Whether k_stream iterates a system that k_team does not: BSR6, more block
-// rows than k_team's narrow CTAs hold, every five consecutive ones within a
-// product stage. (It takes the device for one system at a time, which pays
-// where one system fills it: 22^3 nodes 11.5 us an iteration alone, 25 us in
-// the loop kernels, which need 9 us a system-iteration at 20^3 when eight share
-// them.)
+// rows than k_team's CTAs hold with one part each, every five consecutive ones
+// within a product stage. It takes the device for one system at a time, also
+// where several are active, and is still ahead of the loop kernels, which share
+// it (B200, batches to 1e-6, loop kernels and here: two systems of 27^3 nodes
+// 11.6 and 6.7 ms, eight 30.8 and 26.5, sixteen 57.4 and 51.6; eight of 32^3 43
+// and 34, of 40^3 81 and 58; three of 56^3 79 and 63; single reduction, eight of
+// 40^3, 83 and 57).
 // The loop kernels keep what is left: large CSR systems, longer block rows.
 void Engine::stream_plan(Slot *sl) const {
     const MatA &A = *sl->A;

@@ -17,12 +17,13 @@
 //     pass of its own for it.
 // Product phase: a lane owns a row, its 6x6 blocks from the stage, products
 // rounded and added in index order. Update phase: a lane owns a block (block
-// solve in registers), results go back into the stage and out by bulk stores.
+// solve in registers); x and r (kSr: p and s too) go back into the stage and out
+// by bulk stores, z goes straight to memory.
 // Arithmetic is that of kernels_fused.cu operation by operation; only the
 // grouping of the FP64 sums differs (per lane over its tiles, warp, CTA, device).
 //
 // Measured (B200, us an iteration, loop kernels -> here): 32^3 nodes 31.8 ->
-// 13.0, 40^3 41.5 -> 19.0 (single reduction 39.2 -> 19.0), 64^3 87.0 -> 61.3,
+// 12.9, 40^3 41.5 -> 18.5 (single reduction 39.2 -> 18.5), 64^3 87.0 -> 61.3,
 // 80^3 145.9 -> 114.5 (with the gathers behind the wait for the tile's values
 // 15.2, 21, 65, 122). At 80^3 the product runs at the copy rate of HBM; up to
 // 40^3 the two all-reduces (1.5 us each over 148 CTAs, as long alone) and the
@@ -314,11 +315,12 @@ __device__ __forceinline__ void stream_system(const SysDesc &D, uint32_t limit, 
     };
 
     // ---- update phase ------------------------------------------------------
-    // Slices of a stage: x, r (kSr: p, s), which come and go by bulk copies. What the product has just written (A p and p; kSr: w) and
-    // u = z are read and z is written by plain accesses: a bulk load of them
-    // would need a proxy fence behind the product, and a bulk store of z would
-    // have to be waited for before the reduction. (z as {value, tag} packets,
-    // which need no fence, doubled the gathers' bytes: 80^3 125 -> 139 us.)
+    // Slices of a stage: x, r (kSr: p, s), which come and go by bulk copies. What
+    // the product has just written (A p and p; kSr: w) and u = z are read and z is
+    // written by plain accesses: a bulk load of them would need a proxy fence
+    // behind the product, and a bulk store of z would have to be waited for before
+    // the reduction. (z as {value, tag} packets, which need no fence, doubled the
+    // gathers' bytes: 80^3 125 -> 139 us.)
     auto slice = [&](uint32_t s, uint32_t v) {
         return reinterpret_cast<float *>(stage + s * kStreamUpdStage + kUpd * 144u) + v * kUpd * 6u;
     };

@@ -20,10 +20,10 @@
 //     exchanged.
 // Measured (B200, us an iteration, loop kernels -> here): 4^3 nodes 24.4 -> 2.8,
 // 9^3 23.5 -> 4.3, 12^3 24.8 -> 4.6, 17^3 25.7 -> 4.6, 21^3 27.5 -> 5.3; with
-// two parts a CTA 9^3 6.0, 14^3 6.5 (one: 4.6), 20^3 6.8 (5.3), and 22^3 6.7,
-// 24^3 6.7, 26^3 6.8 (in k_stream 10.5 to 11). CSR: 4^3 21.3 -> 3.2, 19^3 28.6
-// -> 5.7. Single reduction: 4^3 24.6 -> 3.2, 16^3 25.8 -> 5.0, 26^3 28.6 -> 7.2.
-// 48 systems of 4^3 to 24^3 nodes at once: 27.6 ms -> 13.7.
+// two parts a CTA 9^3 6.0, 14^3 6.5 (one: 4.6), 20^3 6.8 (5.3), and 22^3 6.5,
+// 24^3 6.6, 26^3 6.6 (in k_stream 10.5 to 11). CSR: 4^3 21.3 -> 3.3, 19^3 28.6
+// -> 5.7. Single reduction: 4^3 24.6 -> 3.2, 16^3 25.8 -> 5.0, 26^3 28.6 -> 6.8.
+// 48 systems of 4^3 to 24^3 nodes at once: 27.6 ms -> 13.2.
 // What is left is latency (7 of 13 warps wait at a barrier at any time, issue
 // slots 28 % used): per iteration two hops through the L2 (800 cycles for
 // 8 CTAs, 1,400 for 31), the FP64 sums (nine cycles an add, 36 with the shuffle
@@ -543,8 +543,8 @@ __device__ __forceinline__ void team_system(const SysDesc &D, const TeamItem it,
         }
     };
     // p = z + beta p of the lane's rows and of their block columns (p = z when
-    // first; kSr: u = z at the columns, p is the update's). All operands come before the first store, which the compiler
-    // could not move a load across.
+    // first; kSr: u = z at the columns, p is the update's). All operands come
+    // before the first store, which the compiler could not move a load across.
     auto advance_bsr = [&](bool first, float bf) {
 #pragma unroll
         for (int t = 0; t < kT; ++t) {
